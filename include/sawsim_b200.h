@@ -246,8 +246,11 @@ int ss_adjoint_gradient(ss_handle *h, int n_f, const double *omega, double V, in
  *  candidate 3 (DMMA 64x64, three real products, C tile staged in shared
  *  memory while the K loop runs), 37 panel-step GEMM tiles per point run as
  *  thin SIMT 128x8 / 8x128 tiles (tasks at most 8 columns wide or 8 rows high,
- *  beside the DMMA tiles; 0 when the autotuner kept them in DMMA tiles).
- *  Slots past 37 read 0.
+ *  beside the DMMA tiles; 0 when the autotuner kept them in DMMA tiles), 38 1 when
+ *  the scaled system is complex symmetric and its fronts took the symmetric path
+ *  (only the upper triangle of every update block is formed; 12 then counts the
+ *  symmetric update).
+ *  Slots past 38 read 0.
  */
 int ss_stats(const ss_handle *h, double *out, int n);
 

@@ -11,6 +11,7 @@
 #include "dev_complex.cuh"
 #include "krylov.cuh"
 #include "tc_gemm.cuh"
+#include "sym_scale.cuh"
 
 #include <algorithm>
 #include <chrono>
@@ -168,6 +169,8 @@ struct FrontArgs {
   T tiny;                            // static pivot perturbation threshold
   int *nperturb;
   const int *active;                 // solves: frequencies still iterating (nullptr = all)
+  const SymFront *sf;                // symmetric path: pivot blocks and the row maps of their
+  const int *imap;                   // sources (nullptr: general path)
 };
 
 template <class T>
@@ -379,6 +382,55 @@ __device__ __forceinline__ void st_el(cplx<T> *p, cplx<T> v) {
   w.x = v.x;
   w.y = v.y;
   *reinterpret_cast<typename VecOf<T>::V *>(p) = w;
+}
+// value of an update-block entry of a symmetric front from its sources:
+// (i, j) are the entry's row and column in source 0 and in source 1, negative where it
+// has none
+template <class T>
+__device__ __forceinline__ cplx<T> sym_gather(const SymFront &s, const cplx<T> *arena, int i0, int j0, int i1, int j1) {
+  cplx<T> v{0, 0};
+  if (i0 >= 0 && j0 >= 0) v = ld_once(arena + s.cb[0] + (int64_t)i0 * s.cld[0] + j0);
+  if (i1 >= 0 && j1 >= 0) v = v + ld_once(arena + s.cb[1] + (int64_t)i1 * s.cld[1] + j1);
+  return v;
+}
+
+// C tile of a symmetric Schur update (rows tk.r0.., columns tk.c0..) copied into shared
+// memory (row stride CS) by cp.async, each entry on or above the diagonal from the one
+// source that has it (zeros elsewhere); ir and ic receive the tile's source rows and
+// columns.  Entries that both sources have need the second one added in the epilogue.
+template <class T, int BM, int BN, int NT, int CS>
+__device__ __forceinline__ void sym_stage(cplx<T> *Cs, const SymFront &s, const cplx<T> *arena,
+                                          const int *__restrict__ imap, const GemmTask &tk, int (&ir)[2][BM],
+                                          int (&ic)[2][BN]) {
+  constexpr uint32_t EB = sizeof(cplx<T>);
+  const int nch = s.nch;
+  for (int q = threadIdx.x; q < BM + BN; q += NT) {
+    const bool row = q < BM;
+    const int p = row ? tk.r0 + q : tk.c0 + q - BM;
+    const bool in = p < (row ? tk.rhi : tk.chi);
+    const int v0 = in ? imap[s.imap[0] + p] : -1, v1 = in && nch > 1 ? imap[s.imap[1] + p] : -1;
+    if (row)
+      ir[0][q] = v0, ir[1][q] = v1;
+    else
+      ic[0][q - BM] = v0, ic[1][q - BM] = v1;
+  }
+  __syncthreads();
+  const int c = threadIdx.x % BN;
+  const int j0 = ic[0][c], j1 = ic[1][c];
+  const int64_t o0 = s.cb[0], o1 = s.cb[1];
+  const int l0 = s.cld[0], l1 = s.cld[1];
+#pragma unroll 4
+  for (int r = threadIdx.x / BN; r < BM; r += NT / BN) {
+    const int i0 = ir[0][r], i1 = ir[1][r];
+    const bool up = tk.r0 + r <= tk.c0 + c, h0 = up && (i0 | j0) >= 0, h1 = up && (i1 | j1) >= 0;
+    const int64_t o = h0 ? o0 + (int64_t)i0 * l0 + j0 : o1 + (int64_t)i1 * l1 + j1;
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&Cs[r * CS + c]), n = h0 || h1 ? EB : 0u;
+    const cplx<T> *src = h0 || h1 ? arena + o : arena;
+    if constexpr (EB == 16)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+    else
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+  }
 }
 // Which assembly kernel: 0 the row-chunk one, 1 the row-owned one in global
 // memory, 2 the row-owned one with each row staged in shared memory.  Defaults:
@@ -940,7 +992,9 @@ static inline int tile_bn(int s) {
 template <class T, int S>
 constexpr int gemm_cst_bytes() { return Tile<S>::BM * (Tile<S>::BN + 1) * (int)sizeof(cplx<T>); }
 // (the thin tiles: four CTAs per SM, so that more tiles hide their load latency)
-template <class T, int S, bool CST = false>
+// SYM: the tile belongs to the upper triangle of a symmetric update block and is
+// written as (its sources' entries) - A B (sym_front.cuh; tasks name pivot blocks).
+template <class T, int S, bool CST = false, bool SYM = false>
 __global__ void __launch_bounds__(256, (S == kThinCol || S == kThinRow) ? 4 : sizeof(T) == 4 ? 2 : 1)
     front_gemm_kernel(FrontArgs<T> a, const GemmTask *__restrict__ tasks) {
   constexpr int BM = Tile<S>::BM, BN = Tile<S>::BN, TM = Tile<S>::TM, TN = Tile<S>::TN, BK = kGemmBK;
@@ -957,11 +1011,18 @@ __global__ void __launch_bounds__(256, (S == kThinCol || S == kThinRow) ? 4 : si
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const GemmTask tk = tasks[blockIdx.x];
   const int fq = blockIdx.y;
-  const int ld = a.ld[tk.f];
-  cplx<T> *F = a.arena + (int64_t)fq * a.stride + a.off[tk.f];
+  const int ld = SYM ? a.sf[tk.f].ld : a.ld[tk.f];
+  cplx<T> *F = a.arena + (int64_t)fq * a.stride + (SYM ? a.sf[tk.f].off : a.off[tk.f]);
   const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
   cplx<T> *Cs = reinterpret_cast<cplx<T> *>(smem_raw);
-  if constexpr (CST) {
+  [[maybe_unused]] __shared__ int s_ir[2][SYM ? BM : 1], s_ic[2][SYM ? BN : 1];
+  if constexpr (SYM) {
+    const SymFront &sy = a.sf[tk.f];
+    if (sy.nch) {
+      sym_stage<T, BM, BN, 256, CS>(Cs, sy, a.arena + (int64_t)fq * a.stride, a.imap, tk, s_ir, s_ic);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  } else if constexpr (CST) {
     constexpr uint32_t EB = sizeof(cplx<T>);
     for (int idx = threadIdx.x; idx < BM * BN; idx += 256) {
       const int r = idx / BN, c = idx % BN;
@@ -1027,7 +1088,7 @@ __global__ void __launch_bounds__(256, (S == kThinCol || S == kThinRow) ? 4 : si
     }
     __syncthreads();
   }
-  if constexpr (CST) {
+  if constexpr (CST || SYM) {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
   }
@@ -1041,7 +1102,14 @@ __global__ void __launch_bounds__(256, (S == kThinCol || S == kThinRow) ? 4 : si
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
       const int c = tk.c0 + tx + TX * j;
-      if constexpr (CST)
+      if constexpr (SYM) {
+        const SymFront &sy = a.sf[tk.f];
+        const int rl = ty + TY * i, cl = tx + TX * j;
+        cv[j] = cplx<T>{0, 0};
+        if (sy.nch > 1 && rok && c >= r && c < tk.chi && (s_ir[0][rl] | s_ic[0][cl] | s_ir[1][rl] | s_ic[1][cl]) >= 0)
+          cv[j] = ld_once(a.arena + (int64_t)fq * a.stride + sy.cb[1] + (int64_t)s_ir[1][rl] * sy.cld[1] + s_ic[1][cl]);
+        if (sy.nch) cv[j] = cv[j] + Cs[rl * CS + cl];
+      } else if constexpr (CST)
         cv[j] = Cs[(ty + TY * i) * CS + tx + TX * j];
       else
         cv[j] = (rok && c < tk.chi) ? Fr[c] : cplx<T>{0, 0};
@@ -1049,7 +1117,7 @@ __global__ void __launch_bounds__(256, (S == kThinCol || S == kThinRow) ? 4 : si
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
       const int c = tk.c0 + tx + TX * j;
-      if (rok && c < tk.chi) Fr[c] = cv[j] - acc[i][j];
+      if (rok && c < tk.chi && (!SYM || c >= r)) Fr[c] = cv[j] - acc[i][j];
     }
   }
 }
@@ -1318,6 +1386,8 @@ __global__ void __launch_bounds__(128, 2) front_dmma3_kernel(FrontArgs<double> a
 
 }  // namespace ss
 
+#include "sym_front.cuh"
+
 namespace ss {
 
 // Triangular solves stage each 32x32 diagonal block in shared memory (row stride
@@ -1363,7 +1433,7 @@ __global__ void __launch_bounds__(256) front_fwd_kernel(FrontArgs<T> a, const cd
     for (int i = threadIdx.x; i < nn; i += blockDim.x) v[rel[i]] = v[rel[i]] + wc[i];
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
+  if (!a.sf && threadIdx.x == 0) {
     for (int j = 0; j < k; ++j) {
       const int p = sp[j];
       if (p != j) {
@@ -1376,10 +1446,21 @@ __global__ void __launch_bounds__(256) front_fwd_kernel(FrontArgs<T> a, const cd
   __syncthreads();
   // blocked unit-lower solve: warp 0 solves each 32x32 diagonal block with
   // shuffles, then one thread per row below it subtracts the block (each thread's
-  // entries are one contiguous run of its row, all of them in flight at once)
+  // entries are one contiguous run of its row, all of them in flight at once).  On the
+  // symmetric path the pivots come in blocks with an interchange of their own (sp[b0 + j]
+  // = the block's row that its pivot j came from), gathered when the block is reached.
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int jb = 0; jb < k; jb += 32) {
-    const int je = min(k, jb + 32), bw = je - jb;
+  const int bs = a.sf ? sym_block(k) : k;
+  for (int b0 = 0; b0 < k; b0 += bs) {
+  const int b1 = min(k, b0 + bs);
+  if (a.sf) {
+    for (int i = threadIdx.x; i < b1 - b0; i += blockDim.x) D[i] = v[b0 + i];
+    __syncthreads();
+    for (int i = threadIdx.x; i < b1 - b0; i += blockDim.x) v[b0 + i] = D[sp[b0 + i]];
+    __syncthreads();
+  }
+  for (int jb = b0; jb < b1; jb += 32) {
+    const int je = min(b1, jb + 32), bw = je - jb;
     stage_diag(D, F, ld, jb, bw);
     __syncthreads();
     if (wid == 0) {
@@ -1401,6 +1482,7 @@ __global__ void __launch_bounds__(256) front_fwd_kernel(FrontArgs<T> a, const cd
       v[r] = acc;
     }
     __syncthreads();
+  }
   }
   // update rows keep the children's sums; front_fwd_l21_kernel subtracts L21 y
   for (int r = k + threadIdx.x; r < m; r += blockDim.x) w[a.relpos_ptr[f] + r - k] = v[r];
@@ -1681,9 +1763,14 @@ __global__ void __launch_bounds__(256) front_tbwd_kernel(FrontArgs<T> a, cd *__r
   int *sp = reinterpret_cast<int *>(z + k);   // this front's pivots, loaded in parallel
   for (int j = threadIdx.x; j < k; j += blockDim.x) sp[j] = a.piv[(int64_t)fq * a.n + p0 + j];
   __syncthreads();
+  // (symmetric path: pivot blocks from the last one up; inside a block the pivot order,
+  // and its interchange undone before the block is subtracted from the earlier ones)
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int je = k; je > 0; je -= 32) {
-    const int jb = max(0, je - 32), bw = je - jb;
+  const int bs = a.sf ? sym_block(k) : k;
+  for (int b0 = (k - 1) / bs * bs; b0 >= 0; b0 -= bs) {
+  const int b1 = min(k, b0 + bs);
+  for (int je = b1; je > b0; je -= 32) {
+    const int jb = max(b0, je - 32), bw = je - jb;
     stage_diag(D, F, ld, jb, bw);
     __syncthreads();
     if (wid == 0) {
@@ -1697,14 +1784,28 @@ __global__ void __launch_bounds__(256) front_tbwd_kernel(FrontArgs<T> a, cd *__r
       if (lane < bw) z[jb + lane] = xv;
     }
     __syncthreads();
-    for (int r = threadIdx.x; r < jb; r += blockDim.x) {
+    for (int r = b0 + threadIdx.x; r < jb; r += blockDim.x) {
       cplx<T> acc = z[r];
       for (int t = 0; t < bw; ++t) acc = cfms(acc, F[(int64_t)(jb + t) * ld + r], z[jb + t]);
       z[r] = acc;
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
+  if (a.sf) {
+    for (int i = threadIdx.x; i < b1 - b0; i += blockDim.x) D[i] = z[b0 + i];
+    __syncthreads();
+    for (int i = threadIdx.x; i < b1 - b0; i += blockDim.x) z[b0 + sp[b0 + i]] = D[i];
+    __syncthreads();
+    for (int r = threadIdx.x; r < b0; r += blockDim.x) {
+      cplx<T> acc = z[r];
+#pragma unroll 4
+      for (int t = b0; t < b1; ++t) acc = cfms(acc, F[(int64_t)t * ld + r], z[t]);
+      z[r] = acc;
+    }
+    __syncthreads();
+  }
+  }
+  if (!a.sf && threadIdx.x == 0) {
     for (int j = k - 1; j >= 0; --j) {
       const int p = sp[j];
       if (p != j) {
@@ -1803,7 +1904,7 @@ struct Plan {
   struct Graph {
     int kind;                              // 0 factorisation, 1 solve, 2 transposed solve
     int nb;
-    const void *key[8];
+    const void *key[10];
     cudaGraphExec_t exec = nullptr;
     int launches = 0, schur_launches = 0;
   };
@@ -1841,6 +1942,20 @@ struct Plan {
   int64_t stage_rows = 0;                  // packed rows of the widest level, per frequency
   bool tma_ok = false;                     // staging buffer and tensor map ready for this sweep
   DBuf d_pk, d_pitems, d_tt[2];
+  // symmetric path (sym_front.cuh): the pivot blocks of every front, level by level and
+  // block by block: slot level_slot[l] + i holds block i of the level's fronts (their
+  // pivot, panel and Schur tasks; pk_ptr, pi_ptr and tt_ptr run over slots too), with the
+  // arrowhead entries of each task and the sources' row maps
+  bool sym = false;
+  std::vector<int> level_slot;
+  std::vector<int> slot_maxk;
+  std::vector<int64_t> npiv_ptr, npan_ptr;
+  std::vector<NarrowTask> npiv, npan;
+  std::vector<uint16_t> apos;
+  std::vector<int> aslot, imap;
+  std::vector<SymFront> sf;
+  int sym_nev = 0;                         // timed Schur updates of one factorisation
+  DBuf d_npiv, d_npan, d_apos, d_aslot, d_imap, d_sf, d_soff, d_sld, d_sk, d_sm;
   CUtensorMap tmap{};                      // 2D map over the staging buffer (128-byte rows)
   ~Plan() {
     for (auto &g : graphs)
@@ -1890,6 +2005,186 @@ static bool panel_col_narrow(int k, int j0) {
   return (j0 == b0 ? b1 : std::min(k, j0 + kPanel)) - j0 <= kThinMax;
 }
 static bool panel_row_narrow(int k, int j0) { return std::min(k, j0 + kPanel) - j0 <= kThinMax; }
+
+// tiles of the entries on and above the diagonal of rows [k, rhi) and columns [k, m) of
+// pivot block f
+static void add_upper_tiles(std::vector<GemmTask> &v, int bm, int bn, int f, int k, int rhi, int m) {
+  for (int r = k; r < rhi; r += bm)
+    for (int c = k; c < m; c += bn)
+      if (c + bn > r) v.push_back(GemmTask{f, r, c, rhi, m, 0, k});
+}
+
+// Pivot blocks are grouped kGroup pivots at a time: a block updates only the rows of its
+// group (the next blocks need them), the rest of the front gets the whole group at once.
+// The trailing block is then read and written once per group instead of once per block,
+// with a four times longer K loop behind each tile's epilogue.
+constexpr int kGroup = 256;
+
+// Launch plan of the symmetric path.
+Plan *build_sym_plan(Handle &h, bool tensor_schur) {
+  const Symbolic &S = h.sym;
+  Plan *P = new Plan();
+  P->sym = true;
+  P->tuned = !tensor_schur;
+  for (int i = 0; i < S.max_m; ++i) P->imap.push_back(i);   // the identity map, at 0
+  P->level_slot.assign(1, 0);
+  for (auto *v : {&P->npiv_ptr, &P->npan_ptr, &P->schur_ptr, &P->pk_ptr, &P->pi_ptr, &P->tt_ptr[0],
+                  &P->tt_ptr[1]})
+    v->assign(1, 0);
+  std::vector<int> key;
+  std::vector<int64_t> cnt;
+  std::vector<std::vector<NarrowTask>> piv, pan;
+  // Schur updates of a step: pivot block (or group), last row and last column
+  struct Update {
+    int id, rhi, m, k;
+  };
+  std::vector<std::vector<Update>> upd;
+  for (int l = 0; l < S.nlevel; ++l) {
+    int lk = 0, lu = 0, steps = 0;
+    piv.assign(0, {});
+    pan.assign(0, {});
+    upd.assign(0, {});
+    for (int64_t q = S.level_ptr[l]; q < S.level_ptr[l + 1]; ++q) {
+      const int f = S.level_fronts[q], k = S.k[f], m = S.m[f], ld = S.ld[f];
+      lk = std::max(lk, k);
+      lu = std::max(lu, m - k);
+      const int bs = sym_block(k), nblk = (k + bs - 1) / bs;
+      steps = std::max(steps, nblk);
+      if ((int)piv.size() < nblk) piv.resize(nblk), pan.resize(nblk), upd.resize(nblk);
+      const int ng = std::max(1, kGroup / bs);      // blocks per group
+      int group0 = 0;                               // first block of the group, as an index into P->sf
+      // arrowhead entries on and above the diagonal, by block and 64-column chunk
+      std::vector<int> chunk0(nblk + 1, 0);      // first bucket of each block (F11, then its chunks)
+      for (int i = 0; i < nblk; ++i) {
+        const int b1 = std::min(k, bs * (i + 1));
+        chunk0[i + 1] = chunk0[i] + 1 + (m - b1 + 63) / 64;
+      }
+      const int64_t e0 = S.arrow_ptr[f], e1 = S.arrow_ptr[f + 1];
+      key.assign((size_t)(e1 - e0), -1);
+      cnt.assign((size_t)chunk0[nblk] + 1, 0);
+      for (int64_t e = e0; e < e1; ++e) {
+        const int r = S.arrow_pos[e] / ld, c = S.arrow_pos[e] % ld;
+        if (r > c) continue;
+        const int i = r / bs, b1 = std::min(k, bs * (i + 1));
+        key[e - e0] = chunk0[i] + (c < b1 ? 0 : 1 + (c - b1) / 64);
+        ++cnt[key[e - e0] + 1];
+      }
+      for (size_t i = 0; i + 1 < cnt.size(); ++i) cnt[i + 1] += cnt[i];
+      const int64_t a0 = (int64_t)P->apos.size();
+      P->apos.resize(a0 + cnt.back());
+      P->aslot.resize(a0 + cnt.back());
+      std::vector<int64_t> fill(cnt.begin(), cnt.end());
+      for (int64_t e = e0; e < e1; ++e) {
+        if (key[e - e0] < 0) continue;
+        const int r = S.arrow_pos[e] / ld, c = S.arrow_pos[e] % ld;
+        const int i = r / bs, b0 = bs * i, b1 = std::min(k, b0 + bs);
+        const int64_t at = a0 + fill[key[e - e0]]++;
+        P->apos[at] = (uint16_t)((r - b0) * 64 + (c < b1 ? c - b0 : (c - b1) % 64));
+        P->aslot[at] = (int)S.arrow_slot[e];
+      }
+      for (int i = 0; i < nblk; ++i) {
+        const int b0 = bs * i, b1 = std::min(k, b0 + bs), id = (int)P->sf.size();
+        SymFront s{};
+        s.off = S.off[f] + (int64_t)b0 * (ld + 1);
+        s.p0 = S.p0[f] + b0;
+        s.k = b1 - b0;
+        s.m = m - b0;
+        s.ld = ld;
+        if (i == 0) {
+          s.nch = (int)(S.child_ptr[f + 1] - S.child_ptr[f]);
+          for (int c = 0; c < s.nch; ++c) {
+            const int ch = S.child[S.child_ptr[f] + c];
+            s.cb[c] = S.off[ch] + (int64_t)S.k[ch] * S.ld[ch] + S.k[ch];
+            s.cld[c] = S.ld[ch];
+            s.imap[c] = (int64_t)P->imap.size();
+            P->imap.resize(P->imap.size() + m, -1);
+            const int *rel = &S.relpos[S.relpos_ptr[ch]];
+            for (int j = 0; j < S.m[ch] - S.k[ch]; ++j) P->imap[s.imap[c] + rel[j]] = j;
+          }
+        } else {      // in place, through the identity map
+          s.nch = 1;
+          s.cb[0] = s.off;
+          s.cld[0] = ld;
+          s.imap[0] = 0;
+        }
+        P->sf.push_back(s);
+        const int64_t *cp = &cnt[chunk0[i]];
+        piv[i].push_back(NarrowTask{id, -1, (int)(a0 + cp[0]), (int)(a0 + cp[1])});
+        for (int c = 0; c < (s.m - s.k + 63) / 64; ++c)
+          pan[i].push_back(NarrowTask{id, 64 * c, (int)(a0 + cp[1 + c]), (int)(a0 + cp[2 + c])});
+        if (i % ng == 0) group0 = id;
+        const bool last = i + 1 == nblk || (i + 1) % ng == 0;
+        const int g0 = i / ng * ng * bs, g1 = std::min(k, g0 + ng * bs);     // the group's pivots
+        if (!last) {
+          upd[i].push_back(Update{id, g1 - b0, s.m, s.k});
+        } else if (m > g1) {
+          // the whole group: a pivot block entry of its own when it has several blocks
+          int gid = id;
+          if (group0 != id) {
+            SymFront g = P->sf[group0];
+            g.k = g1 - g0;
+            gid = (int)P->sf.size();
+            P->sf.push_back(g);
+          }
+          upd[i].push_back(Update{gid, P->sf[gid].m, P->sf[gid].m, g1 - g0});
+        }
+        P->schur_flops += 4.0 * s.k * (double)(s.m - s.k) * (s.m - s.k + 1);
+      }
+    }
+    P->lvl_maxk.push_back(lk);
+    P->lvl_maxu.push_back(lu);
+    for (int i = 0; i < steps; ++i) {
+      P->npiv.insert(P->npiv.end(), piv[i].begin(), piv[i].end());
+      P->npan.insert(P->npan.end(), pan[i].begin(), pan[i].end());
+      P->npiv_ptr.push_back((int64_t)P->npiv.size());
+      P->npan_ptr.push_back((int64_t)P->npan.size());
+      int mk = 0;
+      for (const NarrowTask &t : piv[i]) mk = std::max(mk, P->sf[t.f].k);
+      double work = 0, padded = 0;
+      for (const Update &t : upd[i]) {
+        if (tensor_schur)
+          add_upper_tiles(P->tasks, tile_bm(kSquare), tile_bn(kSquare), t.id, t.k, t.rhi, t.m);
+        else
+          add_upper_tiles(P->tasks, 64, 64, t.id, t.k, t.rhi, t.m);
+        const int ur = t.rhi - t.k, uc = t.m - t.k;
+        const double ar = (ur + tc::PADC - 1) / tc::PADC * tc::PADC, ac = (uc + tc::PADC - 1) / tc::PADC * tc::PADC;
+        work += (double)ur * uc * t.k;
+        padded += ar * ac * ((t.k + tc::KCH - 1) / tc::KCH * tc::KCH);
+      }
+      P->slot_maxk.push_back(mk);
+      P->schur_ptr.push_back((int64_t)P->tasks.size());
+      P->pick.push_back(tensor_schur ? 2 : 3);
+      if (!tensor_schur) continue;
+      // packed operands and the TMA kernels' tiles; slots that are mostly padding in
+      // 128-row tiles stay on the SIMT kernel
+      int64_t rows = 0;
+      for (const Update &t : upd[i]) {
+        if (padded > 2.5 * work) break;
+        const int kc = (t.k + tc::KCH - 1) / tc::KCH, au = (t.rhi - t.k + tc::PADC - 1) / tc::PADC * tc::PADC,
+                  bu = (t.m - t.k + tc::PADC - 1) / tc::PADC * tc::PADC;
+        const int pf = (int)P->pk.size();
+        P->pk.push_back(tc::PackFront{rows, t.id, kc, au, bu});
+        for (int c = 0; c < kc; ++c) P->pitems.push_back(make_int2(pf, c));
+        for (int v = 0; v < 2; ++v) {
+          const int bnc = v == 0 ? 128 : 64;
+          for (int r0 = t.k; r0 < t.rhi; r0 += tc::BM)
+            for (int c0 = t.k; c0 < t.m; c0 += bnc)
+              if (c0 + bnc > r0)
+                P->tt[v].push_back(
+                    tc::TmaTask{rows, t.id, r0, c0, t.rhi, t.m, kc, au, bu, r0 - t.k, 2 * (c0 - t.k)});
+        }
+        rows += tc::pack_rows(kc, au, bu);
+      }
+      P->stage_rows = std::max(P->stage_rows, rows);
+      P->pk_ptr.push_back((int64_t)P->pk.size());
+      P->pi_ptr.push_back((int64_t)P->pitems.size());
+      P->tt_ptr[0].push_back((int64_t)P->tt[0].size());
+      P->tt_ptr[1].push_back((int64_t)P->tt[1].size());
+    }
+    P->level_slot.push_back(P->level_slot.back() + steps);
+  }
+  return P;
+}
 
 Plan *build_plan(Handle &h, int small_m, bool tensor_schur) {
   Symbolic &S = h.sym;
@@ -2204,6 +2499,82 @@ static int encode_stage_map(Handle &h, CUtensorMap &map, void *base, int64_t row
   return SS_OK;
 }
 
+// scaled copies of the condensed values with the current row and column scales
+static int scale_values(Handle &h) {
+  const int64_t n = h.sym.n;
+  const unsigned nb = (unsigned)((n + 255) / 256);
+  const size_t cb = (size_t)h.c_nnz * sizeof(cd);
+  SS_CK(dalloc(h.dKs, cb));
+  SS_CK(dalloc(h.dMs, cb));
+  if (h.have_D) SS_CK(dalloc(h.dDs, cb));
+  auto scale = [&](const DBuf &in, DBuf &out) {
+    scale_csr_kernel<<<nb, 256, 0, h.stream>>>(n, h.dc_ptr.as<int64_t>(), h.dc_idx.as<int64_t>(),
+                                               h.drow_scale.as<double>(), h.dcol_scale.as<double>(), in.as<cd>(),
+                                               out.as<cd>());
+  };
+  scale(h.dKc, h.dKs);
+  scale(h.dMc, h.dMs);
+  if (h.have_D) scale(h.dDc, h.dDs);
+  SS_CK(cudaGetLastError());
+  return SS_OK;
+}
+
+// Symmetric equilibration at angular frequency w (sym_scale.cuh); `ok` tells whether
+// the scaled system is symmetric to kSymTol (entries are at most about 1).
+constexpr double kSymTol = 1e-13;
+static int equilibrate_sym(Handle &h, double w, bool &ok) {
+  const int64_t n = h.sym.n;
+  const unsigned nb = (unsigned)((n + 255) / 256), wb = (unsigned)((n + 7) / 8);
+  constexpr int kParts = 592;
+  SS_CK(dalloc(h.drow_scale, n * sizeof(double)));
+  SS_CK(dalloc(h.dcol_scale, n * sizeof(double)));
+  DBuf phi, part, t, d, flag;
+  SS_CK(dalloc(phi, n));
+  SS_CK(dalloc(part, 2 * kParts * sizeof(double)));
+  SS_CK(dalloc(t, n * sizeof(double)));
+  SS_CK(dalloc(d, n * sizeof(double)));
+  SS_CK(dalloc(flag, sizeof(int)));
+  const int64_t *rp = h.dc_ptr.as<int64_t>(), *ci = h.dc_idx.as<int64_t>();
+  const cd *D = h.have_D && h.beta ? h.dDc.as<cd>() : nullptr;
+  sym_phi_kernel<<<nb, 256, 0, h.stream>>>(n, rp, ci, h.dMc.as<cd>(), phi.as<unsigned char>());
+  sym_ratio_kernel<<<kParts, 256, 0, h.stream>>>(n, rp, ci, h.dKc.as<cd>(), phi.as<unsigned char>(), part.as<double>());
+  sym_factor_kernel<<<std::min(nb, 148u), 256, 0, h.stream>>>(n, kParts, part.as<double>(), phi.as<unsigned char>(),
+                                                              t.as<double>(), d.as<double>());
+  // three Ruiz steps, from d to drow_scale and back (the third ends in drow_scale)
+  double *from = d.as<double>(), *to = h.drow_scale.as<double>();
+  for (int it = 0; it < 3; ++it) {
+    sym_ruiz_kernel<<<wb, 256, 0, h.stream>>>(n, rp, ci, h.dKc.as<cd>(), h.dMc.as<cd>(), D, w * w, w * h.beta,
+                                              t.as<double>(), from, to);
+    std::swap(from, to);
+  }
+  sym_cols_kernel<<<nb, 256, 0, h.stream>>>(n, t.as<double>(), h.drow_scale.as<double>(), h.dcol_scale.as<double>());
+  int rc = scale_values(h);
+  if (rc) return rc;
+  SS_CK(cudaMemsetAsync(flag.p, 0, sizeof(int), h.stream));
+  sym_check_kernel<<<wb, 256, 0, h.stream>>>(n, rp, ci, h.dKs.as<cd>(), h.dMs.as<cd>(),
+                                             D ? h.dDs.as<cd>() : nullptr, w * w, w * h.beta, kSymTol, flag.as<int>());
+  int bad = 0;
+  SS_CK(cudaMemcpyAsync(&bad, flag.p, sizeof(int), cudaMemcpyDeviceToHost, h.stream));
+  SS_CK(cudaStreamSynchronize(h.stream));
+  ok = bad == 0;
+  if (ok) h.scale_w = w;
+  return SS_OK;
+}
+
+// Whether the symmetric path can take this handle's fronts at all: at most two
+// children per front (its kernels' gathers), 32-bit entry slots, and no forced general
+// tile (SS_SCHUR_TILE, SS_SCHUR_TILE_C64: measurement and test overrides of the
+// general path; SS_SYMMETRIC=0 switches the symmetric path off).
+static bool sym_possible(const Handle &h) {
+  if (getenv("SS_SCHUR_TILE") || getenv("SS_SCHUR_TILE_C64")) return false;
+  if (const char *e = getenv("SS_SYMMETRIC"))
+    if (!atoi(e)) return false;
+  const Symbolic &S = h.sym;
+  for (int f = 0; f < S.nfront; ++f)
+    if (S.child_ptr[f + 1] - S.child_ptr[f] > 2) return false;
+  return h.c_nnz < ((int64_t)1 << 31);
+}
+
 // equilibration at angular frequency w (Ruiz, 3 sweeps)
 static int equilibrate(Handle &h, double w) {
   const int64_t n = h.sym.n;
@@ -2230,22 +2601,10 @@ static int equilibrate(Handle &h, double w) {
     scale_update_kernel<<<nb, 256, 0, h.stream>>>(n, h.dcol_scale.as<double>(), nullptr,
                                                   cmax.as<unsigned long long>());
   }
-  const size_t cb = (size_t)h.c_nnz * sizeof(cd);
-  SS_CK(dalloc(h.dKs, cb));
-  SS_CK(dalloc(h.dMs, cb));
-  scale_csr_kernel<<<nb, 256, 0, h.stream>>>(n, h.dc_ptr.as<int64_t>(), h.dc_idx.as<int64_t>(),
-                                             h.drow_scale.as<double>(), h.dcol_scale.as<double>(), h.dKc.as<cd>(),
-                                             h.dKs.as<cd>());
-  scale_csr_kernel<<<nb, 256, 0, h.stream>>>(n, h.dc_ptr.as<int64_t>(), h.dc_idx.as<int64_t>(),
-                                             h.drow_scale.as<double>(), h.dcol_scale.as<double>(), h.dMc.as<cd>(),
-                                             h.dMs.as<cd>());
-  if (h.have_D) {
-    SS_CK(dalloc(h.dDs, cb));
-    scale_csr_kernel<<<nb, 256, 0, h.stream>>>(n, h.dc_ptr.as<int64_t>(), h.dc_idx.as<int64_t>(),
-                                               h.drow_scale.as<double>(), h.dcol_scale.as<double>(),
-                                               h.dDc.as<cd>(), h.dDs.as<cd>());
+  {
+    const int rc = scale_values(h);
+    if (rc) return rc;
   }
-  SS_CK(cudaGetLastError());
   h.scale_w = w;
   return SS_OK;
 }
@@ -2263,6 +2622,7 @@ struct Sweeper {
   }
   FrontArgs<T> a{};
   int64_t wstride = 0;
+  int chunk = 0;                             // frequencies the chunk buffers hold
   int launches = 0, schur_launches = 0;
   int *tc_err = nullptr;                     // device flag: a tensor-core tile timed out
   std::vector<cudaEvent_t> &ev;              // Schur GEMM timing (the plan's events)
@@ -2273,7 +2633,7 @@ struct Sweeper {
   explicit Sweeper(Handle &hh, Plan &pp) : h(hh), P(pp), ev(pp.ev) {
     pivb = ((size_t)std::max(1, h.sym.max_k) * sizeof(int) + 15) / 16 * 16;
     if (ev.empty()) {
-      ev.resize(2 * std::max(1, h.sym.nlevel));
+      ev.resize(2 * std::max(1, P.sym ? P.level_slot.back() : h.sym.nlevel));
       // recorded once outside any capture: the graphs' event-record nodes then
       // re-record them at every replay and their elapsed times can be read
       for (auto &e : ev) {
@@ -2287,13 +2647,13 @@ struct Sweeper {
   // (kind, nb, key pointers): captured on first use, replayed afterwards.
   template <class Body>
   int graphed(int kind, int nb, std::initializer_list<const void *> key, Body body) {
-    const void *k[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    const void *k[10] = {};
     int i = 0;
     for (const void *p : key) k[i++] = p;
     for (auto &g : P.graphs) {
       if (g.kind != kind || g.nb != nb) continue;
       bool same = true;
-      for (int j = 0; j < 8; ++j) same = same && g.key[j] == k[j];
+      for (int j = 0; j < 10; ++j) same = same && g.key[j] == k[j];
       if (!same) continue;
       SS_CK(cudaGraphLaunch(g.exec, h.stream));
       launches += g.launches;
@@ -2313,7 +2673,7 @@ struct Sweeper {
     Plan::Graph g;
     g.kind = kind;
     g.nb = nb;
-    for (int j = 0; j < 8; ++j) g.key[j] = k[j];
+    for (int j = 0; j < 10; ++j) g.key[j] = k[j];
     const cudaError_t ie = cudaGraphInstantiate(&g.exec, graph, 0);
     cudaGraphDestroy(graph);
     SS_CK(ie);
@@ -2323,8 +2683,113 @@ struct Sweeper {
     SS_CK(cudaGraphLaunch(g.exec, h.stream));
     return SS_OK;
   }
+  // Schur update of slot q on the symmetric path with candidate c (complex64: 0 / 1 TMA
+  // tiles of 128 / 64 columns, 2 SIMT; complex128: one kernel)
+  void sym_schur(int q, int c, int nb) {
+    const int64_t t0 = P.schur_ptr[q], t1 = P.schur_ptr[q + 1];
+    const GemmTask *tasks = P.d_tasks.template as<GemmTask>();
+    const dim3 grid((unsigned)(t1 - t0), nb);
+    if constexpr (sizeof(T) == 8) {
+      sym_schur_kernel<<<grid, 128, sym_schur_smem(), h.stream>>>(a, tasks + t0);
+    } else {
+      if (c == 2 || !P.tma_ok || P.pk_ptr[q + 1] == P.pk_ptr[q]) {
+        front_gemm_kernel<T, kSquare, false, true>
+            <<<grid, 256, gemm_cst_bytes<T, kSquare>(), h.stream>>>(a, tasks + t0);
+        return;
+      }
+      const int64_t i0 = P.pi_ptr[q], i1 = P.pi_ptr[q + 1], q0 = P.tt_ptr[c][q], q1 = P.tt_ptr[c][q + 1];
+      const int64_t *off = P.d_soff.template as<int64_t>();
+      const int *ld = P.d_sld.template as<int>();
+      cf *ar = reinterpret_cast<cf *>(a.arena);
+      tc::pack_kernel<<<dim3((unsigned)(i1 - i0), nb), tc::PACK_THREADS, 0, h.stream>>>(
+          ar, a.stride, off, ld, P.d_sk.template as<int>(), P.d_sm.template as<int>(),
+          P.d_pk.template as<tc::PackFront>(), P.d_pitems.template as<int2>() + i0, h.tc_stage.template as<float>(),
+          P.stage_rows);
+      const unsigned ctas = (unsigned)std::min<int64_t>((q1 - q0) * nb, h.num_sms);
+      auto tma = [&](auto kernel, int threads, int smem) {
+        kernel<<<ctas, threads, smem, h.stream>>>(P.tmap, ar, a.stride, off, ld,
+                                                  P.d_tt[c].template as<tc::TmaTask>() + q0, (int)(q1 - q0), nb,
+                                                  P.stage_rows, tc_err, a.sf, a.imap);
+      };
+      if (c == 0)
+        tma(tc::tma_gemm_kernel<128, 2, true>, tc::TmaCfg<128, 2>::THREADS, tc::TmaCfg<128, 2>::SMEM);
+      else
+        tma(tc::tma_gemm_kernel<64, 3, true>, tc::TmaCfg<64, 3>::THREADS, tc::TmaCfg<64, 3>::SMEM);
+    }
+  }
+  // complex64: the fastest Schur candidate of each slot
+  int sym_tune(int nb) {
+    if (P.tuned) return SS_OK;
+    const int ns = P.level_slot.back();
+    std::vector<cudaEvent_t> e(2 * 3 * ns);
+    for (auto &x : e) SS_CK(cudaEventCreate(&x));
+    P.tune_ms.assign(3 * (size_t)ns, 0.f);
+    auto has = [&](int q, int c) {
+      return P.schur_ptr[q + 1] > P.schur_ptr[q] && (c == 2 || (P.tma_ok && P.pk_ptr[q + 1] > P.pk_ptr[q]));
+    };
+    for (int c = 0; c < 3; ++c)
+      for (int q = 0; q < ns; ++q) {
+        if (!has(q, c)) continue;
+        cudaEventRecord(e[2 * (c * ns + q)], h.stream);
+        sym_schur(q, c, nb);
+        cudaEventRecord(e[2 * (c * ns + q) + 1], h.stream);
+      }
+    SS_CK(cudaGetLastError());
+    SS_CK(cudaStreamSynchronize(h.stream));
+    for (int q = 0; q < ns; ++q)
+      for (int c = 2; c >= 0; --c) {
+        if (!has(q, c)) continue;
+        cudaEventElapsedTime(&P.tune_ms[c * ns + q], e[2 * (c * ns + q)], e[2 * (c * ns + q) + 1]);
+        if (P.tune_ms[c * ns + q] < P.tune_ms[P.pick[q] * ns + q]) P.pick[q] = (char)c;
+      }
+    for (auto &x : e) cudaEventDestroy(x);
+    if (getenv("SS_DEBUG_TUNE"))
+      for (int q = 0; q < ns; ++q)
+        fprintf(stderr, "slot %d tasks %lld tma %.3f %.3f simt %.3f\n", q, (long long)(P.schur_ptr[q + 1] - P.schur_ptr[q]),
+                P.tune_ms[q], P.tune_ms[ns + q], P.tune_ms[2 * ns + q]);
+    P.tuned = true;
+    return SS_OK;
+  }
+  // the symmetric factorisation's launch sequence
+  int sym_factor(int nb) {
+    const uint16_t *ap = P.d_apos.template as<uint16_t>();
+    const int *as = P.d_aslot.template as<int>();
+    nev = 0;
+    for (int l = 0; l < h.sym.nlevel; ++l)
+      for (int q = P.level_slot[l]; q < P.level_slot[l + 1]; ++q) {
+        const int64_t v0 = P.npiv_ptr[q], v1 = P.npiv_ptr[q + 1], p0 = P.npan_ptr[q], p1 = P.npan_ptr[q + 1];
+        const int mk = P.slot_maxk[q];
+        sym_pivot_kernel<T><<<(unsigned)((v1 - v0) * nb), kPivotThreads, pivot_smem<T>(mk), h.stream>>>(
+            a, P.d_npiv.template as<NarrowTask>() + v0, nb, ap, as);
+        ++launches;
+        if (p1 == p0) continue;      // no columns right of any block
+        sym_panel_kernel<T><<<(unsigned)((p1 - p0) * nb), kPanelColThreads, panel_smem<T>(mk), h.stream>>>(
+            a, P.d_npan.template as<NarrowTask>() + p0, nb, ap, as);
+        ++launches;
+        if (P.schur_ptr[q + 1] == P.schur_ptr[q]) continue;
+        SS_CK(cudaEventRecordWithFlags(ev[2 * nev], h.stream, cudaEventRecordExternal));
+        sym_schur(q, P.pick[q], nb);
+        SS_CK(cudaEventRecordWithFlags(ev[2 * nev + 1], h.stream, cudaEventRecordExternal));
+        ++nev;
+        ++launches;
+        ++schur_launches;
+      }
+    P.sym_nev = nev;
+    SS_CK(cudaGetLastError());
+    return SS_OK;
+  }
   // factorisation of a chunk as one graph replay
   int factor_graphed(int nb) {
+    if (P.sym) {
+      int rc = sym_tune(nb);
+      if (rc) return rc;
+      // (the tensor map baked into the graph depends on the staging buffer and its rows)
+      rc = graphed(100, nb, {a.arena, a.piv, a.omega, a.Kc, a.Mc, a.Dc, a.nperturb, tc_err, h.tc_stage.p,
+                             reinterpret_cast<const void *>((uintptr_t)chunk)},
+                   [&] { return sym_factor(nb); });
+      nev = P.sym_nev;
+      return rc;
+    }
     {
       const int rc = tune(nb);
       if (rc) return rc;
@@ -2810,9 +3275,26 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
                       int *iters, double *disp, const SweepExtra *ex, const SweepOpts &opt) {
   Symbolic &S = h.sym;
   const int64_t n = S.n;
-  const int pi = sizeof(T) == 8 ? 0 : 1;
+  double wmax = 0;
+  for (int i = 0; i < n_f; ++i) wmax = std::max(wmax, std::fabs(omega[i]));
+  const bool try_sym = sym_possible(h);
+  if (h.scale_w != wmax || h.scale_tried != try_sym) {
+    bool sym = false;
+    if (try_sym) {
+      const int rc = equilibrate_sym(h, wmax, sym);
+      if (rc) return rc;
+    }
+    if (!sym) {
+      const int rc = equilibrate(h, wmax);
+      if (rc) return rc;
+    }
+    h.scale_sym = sym;
+    h.scale_tried = try_sym;
+  }
+  // plans by precision and by symmetry of the scaled system
+  const int pi = (sizeof(T) == 8 ? 0 : 1) + (h.scale_sym ? 2 : 0);
   if (!h.plan[pi]) {
-    Plan *P = build_plan(h, small_limit<T>(), sizeof(T) == 4);
+    Plan *P = h.scale_sym ? build_sym_plan(h, sizeof(T) == 4) : build_plan(h, small_limit<T>(), sizeof(T) == 4);
     h.plan[pi] = P;
     SS_CK(dupload(P->d_small, P->fronts_small));
     SS_CK(dupload(P->d_large, P->fronts_large));
@@ -2843,6 +3325,33 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
                                tc::TmaCfg<128, 2>::SMEM));
     SS_CK(cudaFuncSetAttribute(tc::tma_gemm_kernel<64, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                tc::TmaCfg<64, 3>::SMEM));
+    if (P->sym) {
+      std::vector<int64_t> off;
+      std::vector<int> ld, sk, sm;
+      for (const SymFront &s : P->sf) off.push_back(s.off), ld.push_back(s.ld), sk.push_back(s.k), sm.push_back(s.m);
+      SS_CK(dupload(P->d_soff, off));
+      SS_CK(dupload(P->d_sld, ld));
+      SS_CK(dupload(P->d_sk, sk));
+      SS_CK(dupload(P->d_sm, sm));
+      SS_CK(dupload(P->d_sf, P->sf));
+      SS_CK(dupload(P->d_imap, P->imap));
+      SS_CK(dupload(P->d_npiv, P->npiv));
+      SS_CK(dupload(P->d_npan, P->npan));
+      SS_CK(dupload(P->d_apos, P->apos));
+      SS_CK(dupload(P->d_aslot, P->aslot));
+      SS_CK(cudaFuncSetAttribute(sym_pivot_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)pivot_smem<T>(kNarrowK)));
+      SS_CK(cudaFuncSetAttribute(sym_panel_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)panel_smem<T>(kNarrowK)));
+      if constexpr (sizeof(T) == 4)
+        SS_CK(cudaFuncSetAttribute(front_gemm_kernel<T, kSquare, false, true>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_cst_bytes<T, kSquare>()));
+      SS_CK(cudaFuncSetAttribute(sym_schur_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sym_schur_smem()));
+      SS_CK(cudaFuncSetAttribute(tc::tma_gemm_kernel<128, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 tc::TmaCfg<128, 2>::SMEM));
+      SS_CK(cudaFuncSetAttribute(tc::tma_gemm_kernel<64, 3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 tc::TmaCfg<64, 3>::SMEM));
+    }
     if (sizeof(T) == 4) {
       SS_CK(dupload(P->d_pk, P->pk));
       SS_CK(dupload(P->d_pitems, P->pitems));
@@ -2871,12 +3380,6 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
     }
   }
   Plan &P = *static_cast<Plan *>(h.plan[pi]);
-  double wmax = 0;
-  for (int i = 0; i < n_f; ++i) wmax = std::max(wmax, std::fabs(omega[i]));
-  if (h.scale_w != wmax) {
-    int rc = equilibrate(h, wmax);
-    if (rc) return rc;
-  }
   const int64_t W = S.relpos_ptr[S.nfront];
   const int krylov_m = opt.krylov_m;
   const int krylov_restarts = opt.restarts;
@@ -2992,6 +3495,9 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
   a.tiny = sizeof(T) == 8 ? (T)h.opt.tiny_c128 : (T)h.opt.tiny_c64;
   a.nperturb = npert.as<int>();
   a.active = h.dmask.as<int>();
+  a.sf = P.sym ? P.d_sf.as<SymFront>() : nullptr;
+  a.imap = P.sym ? P.d_imap.as<int>() : nullptr;
+  sw.chunk = B;
   sw.wstride = W;
   const int maxit = sizeof(T) == 8 ? 1 : 40;   // FP64: one refinement step
   const double tol = sizeof(T) == 8 ? 1e-15 : 1e-12;
@@ -3197,6 +3703,7 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
   h.st[20] = h.st[21] = h.st[22] = h.st[36] = 0;
   h.st[23] = P.panel_cst ? 4 : P.panel_dmma;
   h.st[37] = P.panel_thin ? (double)P.thin_tasks : 0.0;
+  h.st[38] = P.sym ? 1.0 : 0.0;
   h.st[24] = P.panel_ms[0];
   h.st[25] = std::min(std::min(P.panel_ms[1], P.panel_ms[2]), P.panel_ms[3]);
   h.st[26] = (double)P.fronts_small.size();
@@ -3475,7 +3982,7 @@ int measure_ceiling(Handle &h, int kernel, int m, int k, int nb, int reps, doubl
 namespace ss {
 void free_plans(Handle &h) {
   h.auto_prec = -1;
-  for (int i = 0; i < 2; ++i) {
+  for (int i = 0; i < 4; ++i) {
     delete static_cast<Plan *>(h.plan[i]);
     h.plan[i] = nullptr;
   }

@@ -138,7 +138,9 @@ struct Handle {
   DBuf wk[16];                           // sweep work buffers, kept across calls
   DBuf dct_ptr, dct_idx, dct_src;        // transposed condensed pattern (new order) and value slots
   size_t arena_chunk = 0;
-  void *plan[2] = {nullptr, nullptr};   // factorisation plans per precision
+  // factorisation plans: complex128 and complex64 of the general path, then of the
+  // symmetric path
+  void *plan[4] = {nullptr, nullptr, nullptr, nullptr};
   KrylovWork kw;                         // FGMRES workspace of the mixed sweeps
   // SS_PREC_AUTO's decision for the last probed band (its two end frequencies);
   // dropped with the plans whenever the system changes
@@ -148,6 +150,8 @@ struct Handle {
   DBuf tc_stage;                         // packed tensor-core Schur operands (mixed sweeps)
   DBuf dmask;                            // per chunk frequency: still iterating in a Krylov loop
   double scale_w = -1;                   // frequency the scaling was computed at
+  bool scale_sym = false;                // the scaled system is symmetric (the symmetric scaling was kept)
+  bool scale_tried = false;              // the symmetric scaling was tried
   // solver options (ss_set_option); kept until changed
   struct Options {
     int krylov_m = 30;                   // FGMRES restart length of the mixed sweep
@@ -159,7 +163,7 @@ struct Handle {
     int auto_probe_m = 12;               // Krylov steps of SS_PREC_AUTO's probe
   } opt;
   // stats
-  static constexpr int kStats = 38;
+  static constexpr int kStats = 39;
   double st[kStats] = {0};
 };
 

@@ -49,6 +49,26 @@ struct GemmTask {
   int f, r0, c0, rhi, chi, kk0, kk1;
 };
 
+// One pivot block of a front on the symmetric path (sym_front.cuh) as its kernels read
+// it: the rows and columns of the front from the block's first pivot on, k of them the
+// block's pivots, m in all, at element `off` of a frequency's arena (row stride ld);
+// p0 its first pivot in elimination order.  Its entries come from nch <= 2 sources: an
+// update block at element cb (row stride cld) through the inverse row map at imap (row ->
+// source row, -1 when the source does not have it).
+struct SymFront {
+  int64_t off, p0, cb[2], imap[2];
+  int cld[2];
+  int k, m, ld, nch;
+};
+constexpr int kNarrowK = 64;      // most pivots of a block
+// pivots per block of a front with k pivots (the last block may be smaller): balanced,
+// in whole nodes of four degrees of freedom where that fits
+__host__ __device__ inline int sym_block(int k) {
+  const int nb = k > kNarrowK ? (k + kNarrowK - 1) / kNarrowK : 1;
+  const int b = ((k + nb - 1) / nb + 3) / 4 * 4;
+  return b < kNarrowK ? b : kNarrowK;
+}
+
 namespace tc {
 
 constexpr int BM = 128;              // complex rows per tile (MMA M)
@@ -269,11 +289,15 @@ struct TmaCfg {
   static_assert(SMEM <= 227 * 1024, "shared memory");
 };
 
-template <int BNC, int STG>
+// SYM: the tasks cover the upper triangle of symmetric update blocks, and the epilogue
+// writes (children's entries) - L21 U12 at the entries on and above the diagonal, the
+// children gathered through their inverse row maps, instead of updating C in place.
+template <int BNC, int STG, bool SYM = false>
 __global__ void __launch_bounds__(TmaCfg<BNC, STG>::THREADS, 1)
     tma_gemm_kernel(const __grid_constant__ CUtensorMap tmap, cf *__restrict__ arena, int64_t stride,
                     const int64_t *__restrict__ off, const int *__restrict__ ldv, const TmaTask *__restrict__ tasks,
-                    int ntasks, int nb, int64_t stage_rows, int *__restrict__ err) {
+                    int ntasks, int nb, int64_t stage_rows, int *__restrict__ err, const SymFront *__restrict__ sf = nullptr,
+                    const int *__restrict__ imap = nullptr) {
   using Cfg = TmaCfg<BNC, STG>;
   constexpr int NR = Cfg::NR;
   extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
@@ -415,14 +439,87 @@ __global__ void __launch_bounds__(TmaCfg<BNC, STG>::THREADS, 1)
       const int ld = ldv[tk.f];
       float *F = reinterpret_cast<float *>(arena + (int64_t)fq * stride + off[tk.f]);
       const int a = (int)(ac & 1);
+      const int rbase = tk.r0 + 32 * q;
+      const int nrow = min(32, tk.rhi - rbase);                // rows of this quarter inside the tile
+      if constexpr (SYM) {
+        // column blocks h, h + 2, ...: the children's entries of a block are loaded one
+        // block ahead (the first before the accumulator is waited for), so that their
+        // latency overlaps the MMAs and the previous block's stores
+        constexpr int NBLK = NR / 64;
+        const SymFront &sy = sf[tk.f];
+        const float *Ar = reinterpret_cast<const float *>(arena + (int64_t)fq * stride);
+        const int nch = sy.nch;
+        int ir0 = -1, ir1 = -1;                                // this lane's row in the children
+        if (lane < nrow) {
+          if (nch > 0) ir0 = imap[sy.imap[0] + rbase + lane];
+          if (nch > 1) ir1 = imap[sy.imap[1] + rbase + lane];
+        }
+        int j0[NBLK], j1[NBLK];
+#pragma unroll
+        for (int i = 0; i < NBLK; ++i) {
+          const int c = tk.c0 + 16 * (h + 2 * i) + (lane >> 1);
+          j0[i] = nch > 0 && c < tk.chi ? imap[sy.imap[0] + c] : -1;
+          j1[i] = nch > 1 && c < tk.chi ? imap[sy.imap[1] + c] : -1;
+        }
+        const float *b0 = Ar + (lane & 1);
+        const int64_t o0 = sy.cb[0], o1 = sy.cb[1];
+        const int l0 = sy.cld[0], l1 = sy.cld[1];
+        // each entry from the one source that has it; entries that both have take the
+        // second one in a pass of their own
+        auto gather = [&](int i, float (&cur)[32]) {
+          const int c = tk.c0 + 16 * (h + 2 * i) + (lane >> 1);
+          uint32_t both = 0;
+#pragma unroll
+          for (int rr = 0; rr < 32; ++rr) {
+            const int i0 = __shfl_sync(0xffffffffu, ir0, rr), i1 = __shfl_sync(0xffffffffu, ir1, rr);
+            const bool up = rbase + rr <= c, h0 = up && (i0 | j0[i]) >= 0, h1 = up && (i1 | j1[i]) >= 0;
+            const int64_t o = h0 ? o0 + (int64_t)i0 * l0 + j0[i] : o1 + (int64_t)i1 * l1 + j1[i];
+            cur[rr] = h0 || h1 ? __ldcs(b0 + 2 * o) : 0.f;
+            both |= (uint32_t)(h0 && h1) << rr;
+          }
+          if (__any_sync(0xffffffffu, both != 0)) {
+#pragma unroll
+            for (int rr = 0; rr < 32; ++rr) {
+              const int i1 = __shfl_sync(0xffffffffu, ir1, rr);
+              if (both >> rr & 1) cur[rr] += __ldcs(b0 + 2 * (o1 + (int64_t)i1 * l1 + j1[i]));
+            }
+          }
+        };
+        auto live = [&](int i) { return nrow > 0 && rbase <= tk.c0 + 16 * (h + 2 * i) + 15; };   // warp-uniform
+        float cur[2][32];
+        if (live(0)) gather(0, cur[0]);
+        const bool ok = mbar_wait(smem_u32(&acc_full[a]), (uint32_t)((ac / 2) & 1));
+        if (__any_sync(0xffffffffu, !ok)) {
+          abort_s = 1;
+          break;
+        }
+        tc_fence_after();
+#pragma unroll
+        for (int i = 0; i < NBLK; ++i) {
+          const int blk = h + 2 * i;
+          if (i + 1 < NBLK && live(i + 1)) gather(i + 1, cur[(i + 1) & 1]);
+          float v[32];
+          tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(a * NR + 32 * blk), v);
+#pragma unroll
+          for (int e = 0; e < 32; ++e) stg[lane * 33 + e] = v[e];
+          __syncwarp();
+          const int c = tk.c0 + 16 * blk + (lane >> 1);
+          if (live(i) && c < tk.chi) {
+            float *p0 = F + 2 * ((int64_t)rbase * ld + tk.c0 + 16 * blk) + lane;
+            const int64_t rs = 2 * (int64_t)ld;
+#pragma unroll
+            for (int rr = 0; rr < 32; ++rr)
+              if (rr < nrow && rbase + rr <= c) p0[rr * rs] = cur[i & 1][rr] - stg[rr * 33 + lane];
+          }
+          __syncwarp();
+        }
+      } else {
       const bool ok = mbar_wait(smem_u32(&acc_full[a]), (uint32_t)((ac / 2) & 1));
       if (__any_sync(0xffffffffu, !ok)) {
         abort_s = 1;
         break;
       }
       tc_fence_after();
-      const int rbase = tk.r0 + 32 * q;
-      const int nrow = min(32, tk.rhi - rbase);                // rows of this quarter inside the tile
 #pragma unroll 1
       for (int blk = h; blk < NR / 32; blk += 2) {
         float v[32];
@@ -444,6 +541,7 @@ __global__ void __launch_bounds__(TmaCfg<BNC, STG>::THREADS, 1)
             if (rr < nrow) p0[rr * rs] = cur[rr] - stg[rr * 33 + lane];
         }
         __syncwarp();
+      }
       }
       tc_fence_before();
       mbar_arrive(smem_u32(&acc_empty[a]));
