@@ -383,17 +383,47 @@ __device__ __forceinline__ void st_el(cplx<T> *p, cplx<T> v) {
   w.y = v.y;
   *reinterpret_cast<typename VecOf<T>::V *>(p) = w;
 }
-// value of an update-block entry of a symmetric front from its sources:
-// (i, j) are the entry's row and column in source 0 and in source 1, negative where it
-// has none
-template <class T>
-__device__ __forceinline__ cplx<T> sym_gather(const SymFront &s, const cplx<T> *arena, int i0, int j0, int i1, int j1) {
-  cplx<T> v{0, 0};
-  if (i0 >= 0 && j0 >= 0) v = ld_once(arena + s.cb[0] + (int64_t)i0 * s.cld[0] + j0);
-  if (i1 >= 0 && j1 >= 0) v = v + ld_once(arena + s.cb[1] + (int64_t)i1 * s.cld[1] + j1);
-  return v;
+// Entry of a pivot block from its sources: (i0, j0) are its row and column in source 0
+// and (i1, j1) in source 1, negative where a source does not have it.  `at` receives the
+// element offset of the first source that has it (the return value tells whether one
+// does) and `both` whether the second one has it too.  The offset is selected, not the
+// loaded value, so a batch of entries costs one round trip to memory.
+__device__ __forceinline__ bool sym_pick(const SymFront &s, int i0, int j0, int i1, int j1, int64_t &at, bool &both) {
+  const bool h0 = (i0 | j0) >= 0, h1 = (i1 | j1) >= 0;
+  at = h0 ? s.cb[0] + (int64_t)i0 * s.cld[0] + j0 : s.cb[1] + (int64_t)i1 * s.cld[1] + j1;
+  both = h0 && h1;
+  return h0 || h1;
 }
-
+// Arrowhead entries [a0, a1) of a tile added at add(position, value): four per thread and
+// round, the positions and slots, then the values, then the sums.
+template <class T, class Add>
+__device__ __forceinline__ void add_arrows(const FrontArgs<T> &a, int a0, int a1, const uint16_t *__restrict__ apos,
+                                           const int *__restrict__ aslot, double om, Add add) {
+  constexpr int U = 4;
+  const double w2 = om * om;
+  for (int q0 = a0 + threadIdx.x; q0 < a1; q0 += U * blockDim.x) {
+    int pos[U], slot[U];
+    cd kv[U], mv[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int q = q0 + u * blockDim.x;
+      pos[u] = q < a1 ? apos[q] : -1;
+      slot[u] = q < a1 ? aslot[q] : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      kv[u] = ld_el(a.Kc + slot[u]);
+      mv[u] = ld_el(a.Mc + slot[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (pos[u] < 0) continue;
+      cd v = kv[u] - mv[u] * w2;
+      if (a.Dc) v = v + cmul(cd{0.0, om * a.beta}, a.Dc[slot[u]]);
+      add(pos[u], to_t<T>(v));
+    }
+  }
+}
 // C tile of a symmetric Schur update (rows tk.r0.., columns tk.c0..) copied into shared
 // memory (row stride CS) by cp.async, each entry on or above the diagonal from the one
 // source that has it (zeros elsewhere); ir and ic receive the tile's source rows and
@@ -1387,6 +1417,7 @@ __global__ void __launch_bounds__(128, 2) front_dmma3_kernel(FrontArgs<double> a
 }  // namespace ss
 
 #include "sym_front.cuh"
+#include "sym_solve.cuh"
 
 namespace ss {
 
@@ -1433,7 +1464,7 @@ __global__ void __launch_bounds__(256) front_fwd_kernel(FrontArgs<T> a, const cd
     for (int i = threadIdx.x; i < nn; i += blockDim.x) v[rel[i]] = v[rel[i]] + wc[i];
     __syncthreads();
   }
-  if (!a.sf && threadIdx.x == 0) {
+  if (threadIdx.x == 0) {
     for (int j = 0; j < k; ++j) {
       const int p = sp[j];
       if (p != j) {
@@ -1446,21 +1477,10 @@ __global__ void __launch_bounds__(256) front_fwd_kernel(FrontArgs<T> a, const cd
   __syncthreads();
   // blocked unit-lower solve: warp 0 solves each 32x32 diagonal block with
   // shuffles, then one thread per row below it subtracts the block (each thread's
-  // entries are one contiguous run of its row, all of them in flight at once).  On the
-  // symmetric path the pivots come in blocks with an interchange of their own (sp[b0 + j]
-  // = the block's row that its pivot j came from), gathered when the block is reached.
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int bs = a.sf ? sym_block(k) : k;
-  for (int b0 = 0; b0 < k; b0 += bs) {
-  const int b1 = min(k, b0 + bs);
-  if (a.sf) {
-    for (int i = threadIdx.x; i < b1 - b0; i += blockDim.x) D[i] = v[b0 + i];
-    __syncthreads();
-    for (int i = threadIdx.x; i < b1 - b0; i += blockDim.x) v[b0 + i] = D[sp[b0 + i]];
-    __syncthreads();
-  }
-  for (int jb = b0; jb < b1; jb += 32) {
-    const int je = min(b1, jb + 32), bw = je - jb;
+  // entries are one contiguous run of its row, all of them in flight at once)
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  for (int jb = 0; jb < k; jb += 32) {
+    const int je = min(k, jb + 32), bw = je - jb;
     stage_diag(D, F, ld, jb, bw);
     __syncthreads();
     if (wid == 0) {
@@ -1482,7 +1502,6 @@ __global__ void __launch_bounds__(256) front_fwd_kernel(FrontArgs<T> a, const cd
       v[r] = acc;
     }
     __syncthreads();
-  }
   }
   // update rows keep the children's sums; front_fwd_l21_kernel subtracts L21 y
   for (int r = k + threadIdx.x; r < m; r += blockDim.x) w[a.relpos_ptr[f] + r - k] = v[r];
@@ -1569,7 +1588,7 @@ __global__ void __launch_bounds__(256) front_bwd_kernel(FrontArgs<T> a, cd *__re
   cd *xf = x + (int64_t)fq * a.n;
   for (int i = threadIdx.x; i < k; i += blockDim.x) z[i] = to_t<T>(xf[p0 + i]);   // y - U12 x_U
   __syncthreads();
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   // blocked upper solve from the bottom: warp 0 solves each diagonal block,
   // then one thread per row above it subtracts the block (contiguous runs of the
   // rows, all of a thread's loads in flight at once)
@@ -1763,14 +1782,9 @@ __global__ void __launch_bounds__(256) front_tbwd_kernel(FrontArgs<T> a, cd *__r
   int *sp = reinterpret_cast<int *>(z + k);   // this front's pivots, loaded in parallel
   for (int j = threadIdx.x; j < k; j += blockDim.x) sp[j] = a.piv[(int64_t)fq * a.n + p0 + j];
   __syncthreads();
-  // (symmetric path: pivot blocks from the last one up; inside a block the pivot order,
-  // and its interchange undone before the block is subtracted from the earlier ones)
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int bs = a.sf ? sym_block(k) : k;
-  for (int b0 = (k - 1) / bs * bs; b0 >= 0; b0 -= bs) {
-  const int b1 = min(k, b0 + bs);
-  for (int je = b1; je > b0; je -= 32) {
-    const int jb = max(b0, je - 32), bw = je - jb;
+  for (int je = k; je > 0; je -= 32) {
+    const int jb = max(0, je - 32), bw = je - jb;
     stage_diag(D, F, ld, jb, bw);
     __syncthreads();
     if (wid == 0) {
@@ -1784,28 +1798,14 @@ __global__ void __launch_bounds__(256) front_tbwd_kernel(FrontArgs<T> a, cd *__r
       if (lane < bw) z[jb + lane] = xv;
     }
     __syncthreads();
-    for (int r = b0 + threadIdx.x; r < jb; r += blockDim.x) {
+    for (int r = threadIdx.x; r < jb; r += blockDim.x) {
       cplx<T> acc = z[r];
       for (int t = 0; t < bw; ++t) acc = cfms(acc, F[(int64_t)(jb + t) * ld + r], z[jb + t]);
       z[r] = acc;
     }
     __syncthreads();
   }
-  if (a.sf) {
-    for (int i = threadIdx.x; i < b1 - b0; i += blockDim.x) D[i] = z[b0 + i];
-    __syncthreads();
-    for (int i = threadIdx.x; i < b1 - b0; i += blockDim.x) z[b0 + sp[b0 + i]] = D[i];
-    __syncthreads();
-    for (int r = threadIdx.x; r < b0; r += blockDim.x) {
-      cplx<T> acc = z[r];
-#pragma unroll 4
-      for (int t = b0; t < b1; ++t) acc = cfms(acc, F[(int64_t)t * ld + r], z[t]);
-      z[r] = acc;
-    }
-    __syncthreads();
-  }
-  }
-  if (!a.sf && threadIdx.x == 0) {
+  if (threadIdx.x == 0) {
     for (int j = k - 1; j >= 0; --j) {
       const int p = sp[j];
       if (p != j) {
@@ -1948,14 +1948,15 @@ struct Plan {
   // arrowhead entries of each task and the sources' row maps
   bool sym = false;
   std::vector<int> level_slot;
-  std::vector<int> slot_maxk;
-  std::vector<int64_t> npiv_ptr, npan_ptr;
-  std::vector<NarrowTask> npiv, npan;
+  std::vector<int> slot_maxk[4], slot_pank[2];   // most pivots: by pivot class, by chunk width
+  std::vector<int64_t> npiv_ptr[4], npan_ptr[2];
+  std::vector<NarrowTask> npiv[4], npan[2];
   std::vector<uint16_t> apos;
   std::vector<int> aslot, imap;
   std::vector<SymFront> sf;
+  std::vector<int> wide, wide_ptr;         // fronts of more than one pivot block, by level
   int sym_nev = 0;                         // timed Schur updates of one factorisation
-  DBuf d_npiv, d_npan, d_apos, d_aslot, d_imap, d_sf, d_soff, d_sld, d_sk, d_sm;
+  DBuf d_npiv[4], d_npan[2], d_apos, d_aslot, d_imap, d_sf, d_wide, d_soff, d_sld, d_sk, d_sm;
   CUtensorMap tmap{};                      // 2D map over the staging buffer (128-byte rows)
   ~Plan() {
     for (auto &g : graphs)
@@ -2028,12 +2029,14 @@ Plan *build_sym_plan(Handle &h, bool tensor_schur) {
   P->tuned = !tensor_schur;
   for (int i = 0; i < S.max_m; ++i) P->imap.push_back(i);   // the identity map, at 0
   P->level_slot.assign(1, 0);
-  for (auto *v : {&P->npiv_ptr, &P->npan_ptr, &P->schur_ptr, &P->pk_ptr, &P->pi_ptr, &P->tt_ptr[0],
+  P->wide_ptr.assign(1, 0);
+  for (auto *v : {&P->npiv_ptr[0], &P->npiv_ptr[1], &P->npiv_ptr[2], &P->npiv_ptr[3], &P->npan_ptr[0], &P->npan_ptr[1], &P->schur_ptr, &P->pk_ptr, &P->pi_ptr, &P->tt_ptr[0],
                   &P->tt_ptr[1]})
     v->assign(1, 0);
   std::vector<int> key;
   std::vector<int64_t> cnt;
-  std::vector<std::vector<NarrowTask>> piv, pan;
+  std::vector<std::vector<NarrowTask>> piv;
+  std::vector<std::vector<std::pair<NarrowTask, int>>> pan;      // with the chunk width
   // Schur updates of a step: pivot block (or group), last row and last column
   struct Update {
     int id, rhi, m, k;
@@ -2049,7 +2052,9 @@ Plan *build_sym_plan(Handle &h, bool tensor_schur) {
       lk = std::max(lk, k);
       lu = std::max(lu, m - k);
       const int bs = sym_block(k), nblk = (k + bs - 1) / bs;
+      const int cw = tensor_schur ? panel_cols<float>(bs) : panel_cols<double>(bs);   // chunk width
       steps = std::max(steps, nblk);
+      if (nblk > 1) P->wide.push_back(f);
       if ((int)piv.size() < nblk) piv.resize(nblk), pan.resize(nblk), upd.resize(nblk);
       const int ng = std::max(1, kGroup / bs);      // blocks per group
       int group0 = 0;                               // first block of the group, as an index into P->sf
@@ -2057,7 +2062,7 @@ Plan *build_sym_plan(Handle &h, bool tensor_schur) {
       std::vector<int> chunk0(nblk + 1, 0);      // first bucket of each block (F11, then its chunks)
       for (int i = 0; i < nblk; ++i) {
         const int b1 = std::min(k, bs * (i + 1));
-        chunk0[i + 1] = chunk0[i] + 1 + (m - b1 + 63) / 64;
+        chunk0[i + 1] = chunk0[i] + 1 + (m - b1 + cw - 1) / cw;
       }
       const int64_t e0 = S.arrow_ptr[f], e1 = S.arrow_ptr[f + 1];
       key.assign((size_t)(e1 - e0), -1);
@@ -2066,7 +2071,7 @@ Plan *build_sym_plan(Handle &h, bool tensor_schur) {
         const int r = S.arrow_pos[e] / ld, c = S.arrow_pos[e] % ld;
         if (r > c) continue;
         const int i = r / bs, b1 = std::min(k, bs * (i + 1));
-        key[e - e0] = chunk0[i] + (c < b1 ? 0 : 1 + (c - b1) / 64);
+        key[e - e0] = chunk0[i] + (c < b1 ? 0 : 1 + (c - b1) / cw);
         ++cnt[key[e - e0] + 1];
       }
       for (size_t i = 0; i + 1 < cnt.size(); ++i) cnt[i + 1] += cnt[i];
@@ -2079,7 +2084,7 @@ Plan *build_sym_plan(Handle &h, bool tensor_schur) {
         const int r = S.arrow_pos[e] / ld, c = S.arrow_pos[e] % ld;
         const int i = r / bs, b0 = bs * i, b1 = std::min(k, b0 + bs);
         const int64_t at = a0 + fill[key[e - e0]]++;
-        P->apos[at] = (uint16_t)((r - b0) * 64 + (c < b1 ? c - b0 : (c - b1) % 64));
+        P->apos[at] = (uint16_t)((r - b0) * 64 + (c < b1 ? c - b0 : (c - b1) % cw));
         P->aslot[at] = (int)S.arrow_slot[e];
       }
       for (int i = 0; i < nblk; ++i) {
@@ -2110,8 +2115,8 @@ Plan *build_sym_plan(Handle &h, bool tensor_schur) {
         P->sf.push_back(s);
         const int64_t *cp = &cnt[chunk0[i]];
         piv[i].push_back(NarrowTask{id, -1, (int)(a0 + cp[0]), (int)(a0 + cp[1])});
-        for (int c = 0; c < (s.m - s.k + 63) / 64; ++c)
-          pan[i].push_back(NarrowTask{id, 64 * c, (int)(a0 + cp[1 + c]), (int)(a0 + cp[2 + c])});
+        for (int c = 0; c < (s.m - s.k + cw - 1) / cw; ++c)
+          pan[i].push_back({NarrowTask{id, cw * c, (int)(a0 + cp[1 + c]), (int)(a0 + cp[2 + c])}, cw});
         if (i % ng == 0) group0 = id;
         const bool last = i + 1 == nblk || (i + 1) % ng == 0;
         const int g0 = i / ng * ng * bs, g1 = std::min(k, g0 + ng * bs);     // the group's pivots
@@ -2131,27 +2136,35 @@ Plan *build_sym_plan(Handle &h, bool tensor_schur) {
         P->schur_flops += 4.0 * s.k * (double)(s.m - s.k) * (s.m - s.k + 1);
       }
     }
+    P->wide_ptr.push_back((int)P->wide.size());
     P->lvl_maxk.push_back(lk);
     P->lvl_maxu.push_back(lu);
     for (int i = 0; i < steps; ++i) {
-      P->npiv.insert(P->npiv.end(), piv[i].begin(), piv[i].end());
-      P->npan.insert(P->npan.end(), pan[i].begin(), pan[i].end());
-      P->npiv_ptr.push_back((int64_t)P->npiv.size());
-      P->npan_ptr.push_back((int64_t)P->npan.size());
-      int mk = 0;
-      for (const NarrowTask &t : piv[i]) mk = std::max(mk, P->sf[t.f].k);
+      for (int c = 0; c < 4; ++c) {
+        int mk = 0;
+        for (const NarrowTask &t : piv[i])
+          if (pivot_class(P->sf[t.f].k) == 16 * (c + 1)) P->npiv[c].push_back(t), mk = std::max(mk, P->sf[t.f].k);
+        P->npiv_ptr[c].push_back((int64_t)P->npiv[c].size());
+        P->slot_maxk[c].push_back(mk);
+      }
+      for (int c = 0; c < 2; ++c) {      // 64- and 32-column chunks
+        int mk = 0;
+        for (const auto &t : pan[i])
+          if (t.second == (c ? 32 : 64)) P->npan[c].push_back(t.first), mk = std::max(mk, P->sf[t.first.f].k);
+        P->npan_ptr[c].push_back((int64_t)P->npan[c].size());
+        P->slot_pank[c].push_back(mk);
+      }
       double work = 0, padded = 0;
       for (const Update &t : upd[i]) {
         if (tensor_schur)
           add_upper_tiles(P->tasks, tile_bm(kSquare), tile_bn(kSquare), t.id, t.k, t.rhi, t.m);
         else
-          add_upper_tiles(P->tasks, 64, 64, t.id, t.k, t.rhi, t.m);
+          add_upper_tiles(P->tasks, 32, 64, t.id, t.k, t.rhi, t.m);
         const int ur = t.rhi - t.k, uc = t.m - t.k;
         const double ar = (ur + tc::PADC - 1) / tc::PADC * tc::PADC, ac = (uc + tc::PADC - 1) / tc::PADC * tc::PADC;
         work += (double)ur * uc * t.k;
         padded += ar * ac * ((t.k + tc::KCH - 1) / tc::KCH * tc::KCH);
       }
-      P->slot_maxk.push_back(mk);
       P->schur_ptr.push_back((int64_t)P->tasks.size());
       P->pick.push_back(tensor_schur ? 2 : 3);
       if (!tensor_schur) continue;
@@ -2690,7 +2703,7 @@ struct Sweeper {
     const GemmTask *tasks = P.d_tasks.template as<GemmTask>();
     const dim3 grid((unsigned)(t1 - t0), nb);
     if constexpr (sizeof(T) == 8) {
-      sym_schur_kernel<<<grid, 128, sym_schur_smem(), h.stream>>>(a, tasks + t0);
+      sym_schur_kernel<<<grid, 128, kSymSchurSmem, h.stream>>>(a, tasks + t0);
     } else {
       if (c == 2 || !P.tma_ok || P.pk_ptr[q + 1] == P.pk_ptr[q]) {
         front_gemm_kernel<T, kSquare, false, true>
@@ -2750,22 +2763,37 @@ struct Sweeper {
     P.tuned = true;
     return SS_OK;
   }
+  template <int KMAX>
+  void pivot_launch(int q, int nb) {
+    constexpr int c = KMAX / 16 - 1;
+    const int64_t t0 = P.npiv_ptr[c][q], t1 = P.npiv_ptr[c][q + 1];
+    if (t1 == t0) return;
+    sym_pivot_kernel<T, KMAX><<<(unsigned)((t1 - t0) * nb), 2 * KMAX, pivot_smem<T>(P.slot_maxk[c][q]), h.stream>>>(
+        a, P.d_npiv[c].template as<NarrowTask>() + t0, nb, P.d_apos.template as<uint16_t>(), P.d_aslot.template as<int>());
+    ++launches;
+  }
+  template <int CW>
+  void panel_launch(int q, int nb) {
+    constexpr int c = CW == 64 ? 0 : 1;
+    const int64_t t0 = P.npan_ptr[c][q], t1 = P.npan_ptr[c][q + 1];
+    if (t1 == t0) return;
+    sym_panel_kernel<T, CW>
+        <<<(unsigned)((t1 - t0) * nb), kPanelColThreads, panel_smem<T>(P.slot_pank[c][q], CW), h.stream>>>(
+            a, P.d_npan[c].template as<NarrowTask>() + t0, nb, P.d_apos.template as<uint16_t>(),
+            P.d_aslot.template as<int>());
+    ++launches;
+  }
   // the symmetric factorisation's launch sequence
   int sym_factor(int nb) {
-    const uint16_t *ap = P.d_apos.template as<uint16_t>();
-    const int *as = P.d_aslot.template as<int>();
     nev = 0;
     for (int l = 0; l < h.sym.nlevel; ++l)
       for (int q = P.level_slot[l]; q < P.level_slot[l + 1]; ++q) {
-        const int64_t v0 = P.npiv_ptr[q], v1 = P.npiv_ptr[q + 1], p0 = P.npan_ptr[q], p1 = P.npan_ptr[q + 1];
-        const int mk = P.slot_maxk[q];
-        sym_pivot_kernel<T><<<(unsigned)((v1 - v0) * nb), kPivotThreads, pivot_smem<T>(mk), h.stream>>>(
-            a, P.d_npiv.template as<NarrowTask>() + v0, nb, ap, as);
-        ++launches;
-        if (p1 == p0) continue;      // no columns right of any block
-        sym_panel_kernel<T><<<(unsigned)((p1 - p0) * nb), kPanelColThreads, panel_smem<T>(mk), h.stream>>>(
-            a, P.d_npan.template as<NarrowTask>() + p0, nb, ap, as);
-        ++launches;
+        pivot_launch<16>(q, nb);
+        pivot_launch<32>(q, nb);
+        pivot_launch<48>(q, nb);
+        pivot_launch<64>(q, nb);
+        panel_launch<64>(q, nb);
+        if constexpr (sizeof(T) == 8) panel_launch<32>(q, nb);
         if (P.schur_ptr[q + 1] == P.schur_ptr[q]) continue;
         SS_CK(cudaEventRecordWithFlags(ev[2 * nev], h.stream, cudaEventRecordExternal));
         sym_schur(q, P.pick[q], nb);
@@ -2810,6 +2838,7 @@ struct Sweeper {
   int solve_graphed(int kind, int nb, const cd *b, cd *x) {
     const int64_t n = h.sym.n;
     SS_CK(cudaMemcpyAsync(stage_b, b, (size_t)nb * n * sizeof(cd), cudaMemcpyDeviceToDevice, h.stream));
+    if (P.sym) kind = 1;       // one system, one graph
     int rc = graphed(kind, nb, {a.arena, a.piv, stage_b, stage_x, stage_wv, a.Kc, a.active},
                      [&] { return kind == 1 ? solve(nb, stage_b, stage_x, stage_wv) : solve_t(nb, stage_b, stage_x, stage_wv); });
     if (rc) return rc;
@@ -3176,8 +3205,46 @@ struct Sweeper {
     return SS_OK;
   }
 
+  // the symmetric path's solve of A' x = b, which is also A'^T x = b
+  int sym_solve(int nb, const cd *b, cd *x, cplx<T> *wv) {
+    const Symbolic &S = h.sym;
+    const int *lf = h.d_level_fronts.as<int>(), *wide = P.d_wide.template as<int>();
+    for (int pass = 0; pass < 2; ++pass)
+      for (int i = 0; i < S.nlevel; ++i) {
+        const int l = pass == 0 ? i : S.nlevel - 1 - i;
+        const int mk = P.lvl_maxk[l], mu = P.lvl_maxu[l];
+        const int nf = (int)(S.level_ptr[l + 1] - S.level_ptr[l]), nw = P.wide_ptr[l + 1] - P.wide_ptr[l];
+        // the widest block of the level (sym_block is not monotone in k)
+        const int maxb = mk <= kNarrowK ? sym_block(mk) : kNarrowK;
+        const int bs = mk + mu <= 192 ? 128 : 256;
+        const size_t sm = ((size_t)maxb * (maxb + 1) + mk + mu) * sizeof(cplx<T>);
+        FrontArgs<T> c = a, cw = a;
+        c.fronts = lf + S.level_ptr[l];
+        cw.fronts = wide + P.wide_ptr[l];
+        if (pass == 0) {
+          sym_fwd_kernel<T><<<dim3(nf, nb), bs, sm, h.stream>>>(c, b, x, wv, wstride, maxb);
+          if (nw && mu > 0) {
+            const unsigned z = (unsigned)((mu + kSolveRows - 1) / kSolveRows);
+            front_fwd_l21_kernel<T><<<dim3(nw, nb, z), 256, mk * sizeof(cplx<T>), h.stream>>>(cw, x, wv, wstride);
+            ++launches;
+          }
+        } else {
+          if (nw && mu > 0) {
+            const unsigned z = (unsigned)((mk + kSolveRows - 1) / kSolveRows);
+            front_bwd_u12_kernel<T><<<dim3(nw, nb, z), 256, (size_t)mu * sizeof(cplx<T>), h.stream>>>(cw, x);
+            ++launches;
+          }
+          sym_bwd_kernel<T><<<dim3(nf, nb), bs, sm, h.stream>>>(c, x, maxb);
+        }
+        ++launches;
+      }
+    SS_CK(cudaGetLastError());
+    return SS_OK;
+  }
+
   // x <- A'^-1 b for nb frequencies (x may alias nothing; wv workspace)
   int solve(int nb, const cd *b, cd *x, cplx<T> *wv) {
+    if (P.sym) return sym_solve(nb, b, x, wv);
     const Symbolic &S = h.sym;
     const size_t sm = (size_t)S.max_m * sizeof(cplx<T>);
     const size_t smk = (size_t)std::max(1, S.max_k) * sizeof(cplx<T>);
@@ -3212,6 +3279,7 @@ struct Sweeper {
   }
   // mu <- A'^-T c for nb frequencies (same factors; wv workspace)
   int solve_t(int nb, const cd *cvec, cd *mu, cplx<T> *wv) {
+    if (P.sym) return sym_solve(nb, cvec, mu, wv);
     const Symbolic &S = h.sym;
     const size_t sm = (size_t)S.max_m * sizeof(cplx<T>);
     const size_t smk = (size_t)std::max(1, S.max_k) * sizeof(cplx<T>);
@@ -3334,19 +3402,23 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
       SS_CK(dupload(P->d_sk, sk));
       SS_CK(dupload(P->d_sm, sm));
       SS_CK(dupload(P->d_sf, P->sf));
+      SS_CK(dupload(P->d_wide, P->wide));
       SS_CK(dupload(P->d_imap, P->imap));
-      SS_CK(dupload(P->d_npiv, P->npiv));
-      SS_CK(dupload(P->d_npan, P->npan));
+      for (int c = 0; c < 4; ++c) SS_CK(dupload(P->d_npiv[c], P->npiv[c]));
+      for (int c = 0; c < 2; ++c) SS_CK(dupload(P->d_npan[c], P->npan[c]));
       SS_CK(dupload(P->d_apos, P->apos));
       SS_CK(dupload(P->d_aslot, P->aslot));
-      SS_CK(cudaFuncSetAttribute(sym_pivot_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)pivot_smem<T>(kNarrowK)));
-      SS_CK(cudaFuncSetAttribute(sym_panel_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)panel_smem<T>(kNarrowK)));
+      SS_CK(cudaFuncSetAttribute(sym_pivot_kernel<T, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)pivot_smem<T>(64)));
+      SS_CK(cudaFuncSetAttribute(sym_panel_kernel<T, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)panel_smem<T>(sizeof(T) == 8 ? 40 : 64, 64)));
+      if constexpr (sizeof(T) == 8)
+        SS_CK(cudaFuncSetAttribute(sym_panel_kernel<T, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)panel_smem<T>(64, 32)));
       if constexpr (sizeof(T) == 4)
         SS_CK(cudaFuncSetAttribute(front_gemm_kernel<T, kSquare, false, true>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_cst_bytes<T, kSquare>()));
-      SS_CK(cudaFuncSetAttribute(sym_schur_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sym_schur_smem()));
+      SS_CK(cudaFuncSetAttribute(sym_schur_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSymSchurSmem));
       SS_CK(cudaFuncSetAttribute(tc::tma_gemm_kernel<128, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  tc::TmaCfg<128, 2>::SMEM));
       SS_CK(cudaFuncSetAttribute(tc::tma_gemm_kernel<64, 3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -3363,6 +3435,11 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
     const int vec = (int)std::min<int64_t>(227 * 1024, (int64_t)S.max_m * (int64_t)sizeof(cplx<T>));
     const int vecd = (int)std::min<int64_t>(227 * 1024, vec + (int64_t)kDiagElems * sizeof(cplx<T>) +
                                                            ((int64_t)std::max(1, S.max_k) * 4 + 15) / 16 * 16);
+    if (P->sym) {
+      const int sm = (int)std::min<int64_t>(227 * 1024, (int64_t)(kNarrowK * (kNarrowK + 1) + S.max_k + S.max_m) * (int64_t)sizeof(cplx<T>));
+      SS_CK(cudaFuncSetAttribute(sym_fwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+      SS_CK(cudaFuncSetAttribute(sym_bwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+    }
     if (vecd > 48 * 1024) {
       SS_CK(cudaFuncSetAttribute(front_fwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, vecd));
       SS_CK(cudaFuncSetAttribute(front_tfwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, vecd));

@@ -21,28 +21,33 @@
 // applied to the L21 rows of an earlier one, the solves apply each block's interchange
 // when they reach it.
 #pragma once
+#include <type_traits>
 
 namespace ss {
 
-// Upper triangle of F22 = (children) - L21 U12 in 64 x 64 tiles on the FP64 tensor
-// cores: the K loop of front_dmma3_kernel<2, 2> (three real products per complex
-// block); the children's entries are copied into the staged C tile by cp.async when
-// the CTA starts (each entry from the one child that has it), so their latency
-// overlaps the K loop; entries that both children have take the second one in the
-// epilogue.  Tiles below the diagonal are not launched; a diagonal tile skips the
-// entries below it.
+// Upper triangle of an update block = (its sources) - L21 U12 on the FP64 tensor cores,
+// in tiles of 32 x 64 by four warps of 16 x 32 each (three real products per complex
+// 8x8x4 block, operands staged as in front_dmma3_kernel).  The sources' entries are
+// copied into the staged C tile by cp.async when the CTA starts, so their latency overlaps
+// the K loop; entries that both sources have take the second one in the epilogue.  Tiles
+// below the diagonal are not launched; in the others a warp skips its 8x8 blocks below it,
+// and the K loop its last half chunk when that is empty.
+//   32 x 64: 96 accumulator registers, three CTAs per SM.  64 x 64 tiles (two CTAs) wait
+// for C more and leave more of a diagonal tile unused: 40.2 against 33.7 ms for the updates
+// of the 64x256 ME1 cell at 11 points, 10.5 against 8.6 ms for the 8x2x26 Hex27 slab at 33.
 constexpr int kSymCS = 65;
-constexpr int sym_schur_smem() { return 64 * kSymCS * (int)sizeof(cd); }
-__global__ void __launch_bounds__(128, 2) sym_schur_kernel(FrontArgs<double> a, const GemmTask *__restrict__ tasks) {
-  constexpr int BS = 64 + 2;
-  __shared__ __align__(16) cd As[2][64 * kDmmaAS];
+constexpr int kSymSchurSmem = 32 * kSymCS * (int)sizeof(cd);
+__global__ void __launch_bounds__(128, 3)
+    sym_schur_kernel(FrontArgs<double> a, const GemmTask *__restrict__ tasks) {
+  constexpr int MB = 2, BM = 16 * MB, WR = 8 * MB, BS = 64 + 2;
+  __shared__ __align__(16) cd As[2][BM * kDmmaAS];
   __shared__ __align__(16) cd Bs[2][kDmmaBK * BS];
-  __shared__ int ir[2][64], ic[2][64];
+  __shared__ int ir[2][BM], ic[2][64];
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cd *Cs = reinterpret_cast<cd *>(smem_raw);
   const GemmTask tk = tasks[blockIdx.x];
-  const SymFront s = a.sf[tk.f];
-  const int ld = s.ld;
+  const SymFront &s = a.sf[tk.f];
+  const int ld = s.ld, nch = s.nch;
   cd *arena = a.arena + (int64_t)blockIdx.y * a.stride;
   cd *F = arena + s.off;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -50,7 +55,7 @@ __global__ void __launch_bounds__(128, 2) sym_schur_kernel(FrontArgs<double> a, 
   const int g = lane >> 2, t = lane & 3;
   auto issue = [&](int buf, int kb) {
 #pragma unroll
-    for (int q = 0; q < 64 * kDmmaBK / 128; ++q) {
+    for (int q = 0; q < BM * kDmmaBK / 128; ++q) {
       const int idx = threadIdx.x + 128 * q;
       const int r = idx / kDmmaBK, k = idx % kDmmaBK;
       const int gr = tk.r0 + r, gk = kb + k;
@@ -70,17 +75,23 @@ __global__ void __launch_bounds__(128, 2) sym_schur_kernel(FrontArgs<double> a, 
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   const int nk = (tk.kk1 - tk.kk0 + kDmmaBK - 1) / kDmmaBK;
-  if (s.nch) {
-    sym_stage<double, 64, 64, 128, kSymCS>(Cs, s, arena, a.imap, tk, ir, ic);
+  if (nch) {
+    sym_stage<double, BM, 64, 128, kSymCS>(Cs, s, arena, a.imap, tk, ir, ic);
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
-  double p1[4][4][2], p2[4][4][2], p3[4][4][2];
+  // first column block of the warp with an entry on or above the diagonal, per row block:
+  // row block i needs column blocks j with 8 j + 7 >= 8 i + dr
+  const int dr = tk.r0 + wm * WR - (tk.c0 + wn * 32);
+  auto j0 = [&](int i) { return (8 * i + dr - 7 + 7) >> 3; };    // ceil((8 i + dr - 7) / 8)
+  const int rows = min(tk.rhi, tk.r0 + BM) - (tk.r0 + wm * WR);  // the warp's rows inside the tile
+  double p1[MB][4][2], p2[MB][4][2], p3[MB][4][2];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < MB; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int e = 0; e < 2; ++e) p1[i][j][e] = p2[i][j][e] = p3[i][j][e] = 0.0;
+  const bool whole = j0(MB - 1) <= 0 && rows >= WR, some = rows > 0 && j0(0) < 4;
   issue(0, tk.kk0);
   for (int kc = 0; kc < nk; ++kc) {
     const int buf = kc & 1;
@@ -91,37 +102,47 @@ __global__ void __launch_bounds__(128, 2) sym_schur_kernel(FrontArgs<double> a, 
       asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
     __syncthreads();
+    auto half = [&](int kk, auto whole_c) {
+      constexpr bool WHOLE = decltype(whole_c)::value;
+      cd av[MB];
+      double as[MB];
 #pragma unroll
-    for (int kk = 0; kk < kDmmaBK; kk += 4) {
-      cd av[4];
-      double as[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int ar = wm * 32 + i * 8 + g;
+      for (int i = 0; i < MB; ++i) {
+        const int ar = wm * WR + i * 8 + g;
         av[i] = As[buf][ar * kDmmaAS + dmma_acol(ar, kk + t)];
         as[i] = av[i].x + av[i].y;
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
+        if (!WHOLE && j < j0(0)) continue;
         const cd bv = Bs[buf][(kk + t) * BS + wn * 32 + j * 8 + g];
         const double bs = bv.x + bv.y;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < MB; ++i) {
+          if (!WHOLE && (j < j0(i) || 8 * i >= rows)) continue;
           dmma(p1[i][j][0], p1[i][j][1], av[i].x, bv.x);
           dmma(p2[i][j][0], p2[i][j][1], av[i].y, bv.y);
           dmma(p3[i][j][0], p3[i][j][1], as[i], bs);
         }
       }
+    };
+    const bool second = tk.kk0 + kc * kDmmaBK + 4 < tk.kk1;
+    if (whole) {
+      half(0, std::true_type{});
+      if (second) half(4, std::true_type{});
+    } else if (some) {
+      half(0, std::false_type{});
+      if (second) half(4, std::false_type{});
     }
     __syncthreads();
   }
-  const bool two = s.nch > 1;
+  const bool two = nch > 1;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int rl = wm * 32 + i * 8 + g, r = tk.r0 + rl;
+  for (int i = 0; i < MB; ++i) {
+    const int rl = wm * WR + i * 8 + g, r = tk.r0 + rl;
     if (r >= tk.rhi) continue;
     cd *Fr = F + (int64_t)r * ld;
-    const int i0 = s.nch ? ir[0][rl] : -1, i1 = two ? ir[1][rl] : -1;
+    const int i0 = nch ? ir[0][rl] : -1, i1 = two ? ir[1][rl] : -1;
     cd cv[4][2];
 #pragma unroll
     for (int j = 0; j < 4; ++j)
@@ -138,7 +159,7 @@ __global__ void __launch_bounds__(128, 2) sym_schur_kernel(FrontArgs<double> a, 
       for (int e = 0; e < 2; ++e) {
         const int cl = wn * 32 + j * 8 + 2 * t + e, c = tk.c0 + cl;
         if (c < r || c >= tk.chi) continue;
-        if (s.nch) cv[j][e] = Cs[rl * kSymCS + cl] + cv[j][e];
+        if (nch) cv[j][e] = Cs[rl * kSymCS + cl] + cv[j][e];
         const double re = p1[i][j][e] - p2[i][j][e];
         const double im = p3[i][j][e] - p1[i][j][e] - p2[i][j][e];
         st_el(Fr + c, cv[j][e] - cd{re, im});
@@ -149,235 +170,427 @@ __global__ void __launch_bounds__(128, 2) sym_schur_kernel(FrontArgs<double> a, 
 // ------------------------------------------------------------------ pivot blocks
 // A pivot block takes two kernels (and the Schur update) instead of the assembly, panel
 // LU, row-swap, L21, U12 and panel-GEMM launches of every 32-pivot step:
-//  * sym_pivot_kernel assembles F11 in shared memory, factors it and writes it in pivot
-//    order;
-//  * sym_panel_kernel takes one 64-column chunk of F12: it assembles the chunk in shared
-//    memory, and one thread per column solves L11 y = P f (a column of U12) while
-//    another takes the same f as a row of F21 = F12^T and solves z U11 = f^T (a row of
-//    L21), 16 unknowns at a time in registers, the factors read as shared-memory
-//    broadcasts.
+//  * sym_pivot_kernel assembles F11 in shared memory, factors it with a row in two
+//    threads' registers and writes it in pivot order, its 16 x 16 diagonal blocks as
+//    inverses (of the unit lower and of the upper triangle, in their places): the panel
+//    kernel and the solves multiply by them instead of substituting;
+//  * sym_panel_kernel takes one chunk of columns of F12: it assembles the chunk in shared
+//    memory and solves it as rows of F21 = F12^T (z U11 = f^T: L21) and as columns of F12
+//    (L11 y = P f: U12), 16 unknowns at a time: a product with the rows or columns
+//    already solved, then one with the inverted diagonal block.
+// With the block's LU in shared memory, one thread per panel column and a 16-step
+// substitution in the solves, a pass over the 32x128 ME1 cell at 51 points took 89 ms and
+// one over 16x64 at 101 points 21 ms; so, 61 and 15 ms.
 // Row interchanges are implicit (a mask of eliminated rows); `piv` receives, for each
-// pivot position, the front row it came from (the solve kernels gather).
-constexpr int kPivotThreads = 128;
-constexpr int kPanelColThreads = 128;
-constexpr int kNarrowCS = 65;     // row stride of the chunk tile
+// pivot position, the block's row it came from (the solve kernels gather).
+constexpr int kDiagB = 16;        // inverted diagonal blocks
 
-// F11 of one pivot block with its arrowhead entries [a0, a1), or (c0 >= 0) the chunk of F12
-// that starts at update column c0 with its entries
+// F11 of one pivot block with its arrowhead entries [a0, a1), or (c0 >= 0) the chunk of
+// F12 that starts at update column c0 with its entries
 struct NarrowTask {
   int f, c0, a0, a1;
 };
+__host__ __device__ constexpr int pivot_class(int k) { return k <= 16 ? 16 : k <= 32 ? 32 : k <= 48 ? 48 : 64; }
 template <class T>
 __host__ __device__ constexpr size_t pivot_smem(int k) {
-  return ((size_t)k * (k + 1) + k) * sizeof(cplx<T>) + (size_t)3 * k * sizeof(int);
-}
-template <class T>
-__host__ __device__ constexpr size_t panel_smem(int k) {
-  return ((size_t)k * (k + 1) + (size_t)k * kNarrowCS + k) * sizeof(cplx<T>) + (size_t)k * sizeof(int);
+  return (size_t)k * (k + 1) * sizeof(cplx<T>) + (size_t)2 * k * sizeof(int);
 }
 
-// LU of the k x k matrix W (row stride ks, shared memory) with implicit row
-// interchanges, one barrier per pivot: each warp owns the rows wid, wid + NW, ... and
-// keeps the largest next-column entry of its open rows (four rows in flight).
-// perm[j] = row of pivot j.  Returns the number of perturbed pivots.
-template <class T, int NW>
-__device__ __forceinline__ int narrow_lu(cplx<T> *W, int ks, int k, T tiny, int *perm) {
-  __shared__ T s_v[2][NW];
-  __shared__ int s_i[2][NW];
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  {
-    T best = (T)-1;
-    int bi = 0;
-    for (int r = wid + NW * lane; r < k; r += 32 * NW) {
-      const T v = cabs1(W[r * ks]);
-      if (v > best) best = v, bi = r;
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      const T ov = __shfl_down_sync(0xffffffffu, best, o);
-      const int oi = __shfl_down_sync(0xffffffffu, bi, o);
-      if (ov > best || (ov == best && oi < bi)) best = ov, bi = oi;
-    }
-    if (lane == 0) s_v[1][wid] = best, s_i[1][wid] = bi;
-    __syncthreads();
+// 1 / z without overflow or underflow in the squares
+template <class T>
+__device__ __forceinline__ cplx<T> crecip(cplx<T> z) {
+  const T r = (T)1 / fmax(fabs(z.x), fabs(z.y));
+  const T x = z.x * r, y = z.y * r, g = r / (x * x + y * y);
+  return {x * g, -y * g};
+}
+// magnitude of a pivot candidate as an ordered integer, its low 7 bits replaced by the
+// row (the lowest row wins among magnitudes equal to about 2^-13)
+__device__ __forceinline__ unsigned pivot_key(double v, int r) {
+  return ((unsigned)__double2hiint(v) & ~127u) | (unsigned)(127 - r);
+}
+__device__ __forceinline__ unsigned pivot_key(float v, int r) {
+  return (__float_as_uint(v) & ~127u) | (unsigned)(127 - r);
+}
+
+// LU of the k x k matrix W (row stride ks, shared memory; k <= KMAX) in place with
+// implicit row interchanges, by 2 KMAX threads: thread (r, h) holds the entries of row r
+// in columns 2 i + h, i counted from the current column pair (the registers shift down
+// once per pair), in registers.  Per pivot: the warps' candidate keys (one integer
+// reduction each) give the row; its two threads write it to W (it is final) with the
+// pivot's reciprocal; every open row takes its multiplier and updates its registers, so
+// shared memory carries one row per pivot instead of the whole trailing matrix.  The
+// register loop shrinks in four steps.  On return W holds the multipliers and U rows in
+// the original row order, perm[j] the row of pivot j and dinv[j] the reciprocal pivots.
+// (One CTA, k = 64, complex128: 153 us with the trailing matrix in shared memory.)
+template <class T, int KMAX>
+__device__ __forceinline__ int block_lu(cplx<T> *W, int ks, int k, T tiny, int *perm, cplx<T> *dinv) {
+  constexpr int W2 = KMAX / 2, NW = KMAX / 16;
+  __shared__ unsigned s_key[2][NW];
+  const int tid = threadIdx.x, r = tid >> 1, h = tid & 1, lane = tid & 31, wid = tid >> 5;
+  cplx<T> v[W2];
+#pragma unroll
+  for (int i = 0; i < W2; ++i) {
+    const int c = 2 * i + h;
+    v[i] = r < k && c < k ? W[r * ks + c] : cplx<T>{0, 0};
   }
-  unsigned long long done = 0;
-  bool pert_prev = false;
-  int p_prev = 0, npert = 0;
-  for (int j = 0; j < k; ++j) {
-    const int par = (j & 1) ^ 1;
-    T bv = s_v[par][0];
-    int p = s_i[par][0];
+  bool open = r < k;
+  int npert = 0;
+  auto candidate = [&](int par, int hown) {
+    unsigned key = open && h == hown ? pivot_key(cabs1(v[0]), r) : 0u;
+    key = __reduce_max_sync(0xffffffffu, key);
+    if (lane == 0) s_key[par][wid] = key;
+  };
+  candidate(0, 0);
+  // one pivot step: HOWN = parity of column j; WC registers may be nonzero
+  auto step = [&](int j, auto hown_c, auto wc_c) {
+    constexpr int HOWN = decltype(hown_c)::value, WC = decltype(wc_c)::value;
+    __syncthreads();
+    unsigned key = s_key[HOWN][0];
 #pragma unroll
-    for (int q = 1; q < NW; ++q) {
-      const T ov = s_v[par][q];
-      const int oi = s_i[par][q];
-      if (ov > bv || (ov == bv && oi < p)) bv = ov, p = oi;
-    }
-    if (p >= k || (done >> p & 1)) p = __ffsll((long long)~done) - 1;   // no comparable entry (NaN): any open row
-    // the previous pivot's perturbed diagonal is read by no one any more
-    if (pert_prev && tid == 0) W[p_prev * ks + j - 1] = cplx<T>{tiny, (T)0};
-    const int c0 = j + 1 + lane, c1 = c0 + 32;
-    cplx<T> pv = W[p * ks + j];
-    const cplx<T> q0 = c0 < k ? W[p * ks + c0] : cplx<T>{0, 0}, q1 = c1 < k ? W[p * ks + c1] : cplx<T>{0, 0};
-    const bool pert = cabs1(pv) < tiny;
-    if (pert) pv = cplx<T>{tiny, (T)0};
-    const cplx<T> inv = cdiv(cplx<T>{1, 0}, pv);
-    if (tid == 0) perm[j] = p;
-    npert += pert;
-    pert_prev = pert;
-    p_prev = p;
-    done |= 1ull << p;
-    T best = (T)-1;
-    int bi = k;
-    for (int rb = wid; rb < k; rb += 4 * NW) {
-      cplx<T> l[4], v0[4], v1[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int r = min(rb + NW * i, k - 1);
-        const cplx<T> *row = W + r * ks;
-        l[i] = row[j];
-        v0[i] = c0 < k ? row[c0] : cplx<T>{0, 0};
-        v1[i] = c1 < k ? row[c1] : cplx<T>{0, 0};
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        l[i] = cmul(l[i], inv);
-        v0[i] = cfms(v0[i], l[i], q0);
-        v1[i] = cfms(v1[i], l[i], q1);
-      }
-      __syncwarp();      // every lane has read its row's multiplier
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int r = rb + NW * i;
-        if (r >= k || (done >> r & 1)) continue;
-        cplx<T> *row = W + r * ks;
-        if (c0 < k) row[c0] = v0[i];
-        if (c1 < k) row[c1] = v1[i];
-        if (lane == 0) {
-          row[j] = l[i];
-          const T av = cabs1(v0[i]);
-          if (av > best) best = av, bi = r;
+    for (int q = 1; q < NW; ++q) key = max(key, s_key[HOWN][q]);
+    const int p = 127 - (int)(key & 127u);
+    cplx<T> *Wp = W + p * ks;
+    if (r == p) {
+      if (h == HOWN) {
+        cplx<T> pv = v[0];
+        if (cabs1(pv) < tiny) {
+          pv = cplx<T>{tiny, (T)0};
+          npert = npert + 1;
         }
+        Wp[j] = pv;
+        dinv[j] = crecip(pv);
+        perm[j] = p;
       }
+#pragma unroll
+      for (int i = 0; i < WC; ++i) {
+        const int c = j - HOWN + 2 * i + h;
+        if (c > j && c < k) Wp[c] = v[i];
+      }
+      open = false;
     }
-    if (lane == 0) s_v[j & 1][wid] = best, s_i[j & 1][wid] = bi;
     __syncthreads();
-  }
-  if (pert_prev && tid == 0) W[p_prev * ks + k - 1] = cplx<T>{tiny, (T)0};
+    const T ox = __shfl_xor_sync(0xffffffffu, v[0].x, 1), oy = __shfl_xor_sync(0xffffffffu, v[0].y, 1);
+    const cplx<T> vj = h == HOWN ? v[0] : cplx<T>{ox, oy};
+    cplx<T> l = cmul(vj, dinv[j]);
+    if (!open) l = cplx<T>{0, 0};
+    if (open && h == 0) W[r * ks + j] = l;
+#pragma unroll
+    for (int i = 0; i < WC; ++i) {
+      const int c = j - HOWN + 2 * i + h;
+      const cplx<T> q = c > j && c < k ? Wp[c] : cplx<T>{0, 0};
+      const cplx<T> x = cfms(v[i], l, q);
+      if (HOWN == 0)
+        v[i] = x;
+      else if (i > 0)
+        v[i - 1] = x;      // the column pair is done: shift
+    }
+    if (HOWN == 1) v[WC - 1] = cplx<T>{0, 0};
+    candidate(HOWN ^ 1, HOWN ^ 1);
+  };
+  using std::integral_constant;
+  auto pair = [&](int j, auto wc) {
+    step(j, integral_constant<int, 0>{}, wc);
+    if (j + 1 < k) step(j + 1, integral_constant<int, 1>{}, wc);
+  };
+  int j = 0;
+  for (; j < k && k - j > 2 * (3 * W2 / 4); j += 2) pair(j, integral_constant<int, W2>{});
+  for (; j < k && k - j > 2 * (W2 / 2); j += 2) pair(j, integral_constant<int, 3 * W2 / 4>{});
+  for (; j < k && k - j > 2 * (W2 / 4); j += 2) pair(j, integral_constant<int, W2 / 2>{});
+  for (; j < k; j += 2) pair(j, integral_constant<int, W2 / 4>{});
   __syncthreads();
   return npert;
 }
 
-template <class T>
-__global__ void __launch_bounds__(kPivotThreads)
+template <class T, int KMAX>
+__global__ void __launch_bounds__(2 * KMAX)
     sym_pivot_kernel(FrontArgs<T> a, const NarrowTask *__restrict__ tasks, int nb, const uint16_t *__restrict__ apos,
                      const int *__restrict__ aslot) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int NW = kPivotThreads / 32;
+  __shared__ cplx<T> dinv[KMAX];
+  __shared__ int perm[KMAX];
+  constexpr int NT = 2 * KMAX, NW = NT / 32;
   const NarrowTask tk = tasks[blockIdx.x / nb];
   const int fq = blockIdx.x % nb;
   const SymFront &s = a.sf[tk.f];
   const int k = s.k, ks = k + 1;
   cplx<T> *W = reinterpret_cast<cplx<T> *>(smem_raw);
-  int *perm = reinterpret_cast<int *>(W + k * ks + k), *ir = perm + k;
+  int *ir = reinterpret_cast<int *>(W + k * ks);
   cplx<T> *arena = a.arena + (int64_t)fq * a.stride;
   const double om = a.omega[fq];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int nch = s.nch;
   if (nch) {
-    for (int i = tid; i < k; i += kPivotThreads) {
+    for (int i = tid; i < k; i += NT) {
       ir[i] = a.imap[s.imap[0] + i];
       ir[k + i] = nch > 1 ? a.imap[s.imap[1] + i] : -1;
     }
     __syncthreads();
-    // the children's upper entries, mirrored
-    for (int r = wid; r < k; r += NW)
-      for (int c = r + lane; c < k; c += 32) {
-        const cplx<T> v = sym_gather(s, arena, ir[r], ir[c], ir[k + r], ir[k + c]);
-        W[r * ks + c] = v;
-        W[c * ks + r] = v;
+    // the sources' upper entries, mirrored: four rows of 32 columns in flight per warp
+    constexpr int U = 4;
+    for (int cb = 0; cb < k; cb += 32)
+      for (int rb = wid; rb < min(k, cb + 32); rb += U * NW) {
+        const int c = cb + lane;
+        cplx<T> v[U];
+        bool both[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int r = rb + u * NW;
+          const bool in = r < k && c < k && c >= r;
+          int64_t at;
+          const bool has = in && sym_pick(s, ir[min(r, k - 1)], ir[min(c, k - 1)], ir[k + min(r, k - 1)],
+                                          ir[k + min(c, k - 1)], at, both[u]);
+          v[u] = has ? ld_once(arena + at) : cplx<T>{0, 0};
+          both[u] = has && both[u];
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int r = rb + u * NW;
+          if (both[u]) v[u] = v[u] + ld_once(arena + s.cb[1] + (int64_t)ir[k + r] * s.cld[1] + ir[k + c]);
+          if (r < k && c < k && c >= r) {
+            W[r * ks + c] = v[u];
+            W[c * ks + r] = v[u];
+          }
+        }
       }
   } else {
-    for (int t = tid; t < k * ks; t += kPivotThreads) W[t] = cplx<T>{0, 0};
+    for (int t = tid; t < k * ks; t += NT) W[t] = cplx<T>{0, 0};
   }
   __syncthreads();
-#pragma unroll 4
-  for (int q = tk.a0 + tid; q < tk.a1; q += kPivotThreads) {
-    const int r = apos[q] >> 6, c = apos[q] & 63;
-    const cplx<T> v = W[r * ks + c] + to_t<T>(a_entry(a.Kc, a.Mc, a.Dc, aslot[q], om, a.beta));
+  add_arrows(a, tk.a0, tk.a1, apos, aslot, om, [&](int p, cplx<T> e) {
+    const int r = p >> 6, c = p & 63;
+    const cplx<T> v = W[r * ks + c] + e;
     W[r * ks + c] = v;
     W[c * ks + r] = v;
-  }
+  });
   __syncthreads();
-  const int np = narrow_lu<T, NW>(W, ks, k, a.tiny, perm);
-  if (np && tid == 0) atomicAdd(a.nperturb + fq, np);
+  const int np = block_lu<T, KMAX>(W, ks, k, a.tiny, perm, dinv);
+  if (np) atomicAdd(a.nperturb + fq, np);
   cplx<T> *F = arena + s.off;
   const int ld = s.ld;
-  for (int r = wid; r < k; r += NW)
-    for (int c = lane; c < k; c += 32) st_el(F + (int64_t)r * ld + c, W[perm[r] * ks + c]);
-  for (int i = tid; i < k; i += kPivotThreads) a.piv[(int64_t)fq * a.n + s.p0 + i] = perm[i];
+  for (int r = wid; r < k; r += NW) {
+    const cplx<T> *row = W + perm[r] * ks;
+    for (int c = lane; c < k; c += 32)
+      if ((c ^ r) >= kDiagB) st_el(F + (int64_t)r * ld + c, row[c]);
+  }
+  for (int i = tid; i < k; i += NT) a.piv[(int64_t)fq * a.n + s.p0 + i] = perm[i];
+  // inverses of the diagonal blocks, one block per warp: lanes 0-15 a column of the
+  // inverted unit lower triangle each, lanes 16-31 of the inverted upper triangle
+  const int h0 = kDiagB * wid, hw = min(kDiagB, k - h0);
+  if (hw <= 0) return;
+  const int col = lane & 15;
+  cplx<T> x[kDiagB];
+  if (lane < 16) {
+#pragma unroll
+    for (int i = 0; i < kDiagB; ++i) {
+      cplx<T> t{i == col ? (T)1 : (T)0, (T)0};
+      const cplx<T> *row = W + perm[h0 + min(i, hw - 1)] * ks + h0;
+#pragma unroll
+      for (int q = 0; q < i; ++q) t = cfms(t, row[q], x[q]);
+      x[i] = t;
+      if (i > col && i < hw && col < hw) st_el(F + (int64_t)(h0 + i) * ld + h0 + col, t);
+    }
+  } else {
+#pragma unroll
+    for (int i = kDiagB - 1; i >= 0; --i) {
+      cplx<T> t{i == col ? (T)1 : (T)0, (T)0};
+      if (i < hw) {
+        const cplx<T> *row = W + perm[h0 + i] * ks + h0;
+#pragma unroll
+        for (int q = i + 1; q < kDiagB; ++q)
+          if (q < hw) t = cfms(t, row[q], x[q]);
+        t = cmul(t, dinv[h0 + i]);
+        if (i <= col && col < hw) st_el(F + (int64_t)(h0 + i) * ld + h0 + col, t);
+      }
+      x[i] = t;
+    }
+  }
 }
 
-// H unknowns h0 .. h0 + hw of one triangular solve, v_i = (b_i - sum_{t < h0 + i} x_t
-// C(t, i)) d_i.  LOWER: C = L[h0 + i][t], unit diagonal; else C = U[t][h0 + i] and d the
-// reciprocal diagonal.  x points at the solved unknowns (stride xs).
-template <class T, int H, bool LOWER>
-__device__ __forceinline__ void narrow_block(cplx<T> (&v)[H], const cplx<T> *A, int ks, const cplx<T> *x, int64_t xs,
-                                             int h0, int hw, const cplx<T> *dinv) {
+// ------------------------------------------------------------------ panel columns
+// Coefficient (i, t) of an inverted diagonal block at A (row stride ks): LOWER the unit
+// lower triangle's inverse, else the transposed inverse of the upper triangle (both are
+// lower triangular in (i, t)).
+template <class T, bool LOWER>
+__device__ __forceinline__ cplx<T> diag_coef(const cplx<T> *A, int ks, int i, int t) {
+  if (t > i) return cplx<T>{0, 0};
+  if (LOWER && t == i) return cplx<T>{1, 0};
+  return LOWER ? A[i * ks + t] : A[t * ks + i];
+}
+
+// complex128: 8 NJ columns of the chunk tile Y (row stride CS, rows padded to a multiple
+// of 8) solved in place by one warp on the FP64 tensor cores: for 16 rows at a time, the
+// product with the rows already solved (three real products per complex block, fragments
+// as in front_dmma3_kernel), then with the inverted diagonal block.  Bound by the FP64
+// pipe: one thread per column with broadcast coefficients moved 4 x 16 bytes of shared
+// memory per complex multiply-add and took 27 us per 64-pivot, 64-column chunk.
+template <bool LOWER, int NJ>
+__device__ __forceinline__ void panel_dmma(const cd *A, int ks, cd *Y, int CS, int k) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  for (int h0 = 0; h0 < k; h0 += kDiagB) {
+    const int ni = k - h0 > 8 ? 2 : 1;
+    double p1[2][NJ][2], p2[2][NJ][2], p3[2][NJ][2];
+    auto clear = [&] {
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) p1[i][j][e] = p2[i][j][e] = p3[i][j][e] = 0.0;
+    };
+    auto mma = [&](const cd (&av)[2], int row) {
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        const cd bv = Y[row * CS + j * 8 + g];
+        const double bs = bv.x + bv.y;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          if (i >= ni) break;
+          dmma(p1[i][j][0], p1[i][j][1], av[i].x, bv.x);
+          dmma(p2[i][j][0], p2[i][j][1], av[i].y, bv.y);
+          dmma(p3[i][j][0], p3[i][j][1], av[i].x + av[i].y, bs);
+        }
+      }
+    };
+    if (h0) {
+      clear();
+#pragma unroll 2
+      for (int kk = 0; kk < h0; kk += 4) {
+        cd av[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int row = h0 + (i < ni ? i * 8 : 0) + g;
+          av[i] = LOWER ? A[row * ks + kk + t] : A[(kk + t) * ks + row];
+        }
+        mma(av, kk + t);
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            if (i >= ni) continue;
+            cd *y = Y + (h0 + i * 8 + g) * CS + j * 8 + 2 * t + e;
+            *y = cd{y->x - (p1[i][j][e] - p2[i][j][e]), y->y - (p3[i][j][e] - p1[i][j][e] - p2[i][j][e])};
+          }
+      __syncwarp();
+    }
+    clear();
+#pragma unroll
+    for (int kk = 0; kk < kDiagB; kk += 4) {
+      if (kk >= 8 * ni) break;
+      cd av[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        av[i] = diag_coef<double, LOWER>(A + h0 * ks + h0, ks, (i < ni ? i * 8 : 0) + g, kk + t);
+      mma(av, h0 + kk + t);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          if (i < ni)
+            Y[(h0 + i * 8 + g) * CS + j * 8 + 2 * t + e] =
+                cd{p1[i][j][e] - p2[i][j][e], p3[i][j][e] - p1[i][j][e] - p2[i][j][e]};
+    __syncwarp();
+  }
+}
+
+// complex64: 16 columns of the tile solved in place by one warp, 16 rows at a time: a
+// lane holds 4 rows x 2 columns, so each coefficient and each solved entry it loads takes
+// part in two and four multiply-adds (one column per thread is bound by the broadcast
+// loads).
+template <bool LOWER>
+__device__ __forceinline__ void panel_simt(const cf *A, int ks, cf *Y, int CS, int k) {
+  const int lane = threadIdx.x & 31, c = 2 * (lane & 7), r = 4 * (lane >> 3);
+  for (int h0 = 0; h0 < k; h0 += kDiagB) {
+    cf x[4][2];
+    auto load = [&](cf (&y)[2], int row) {
+      const float4 q = *reinterpret_cast<const float4 *>(Y + row * CS + c);
+      y[0] = cf{q.x, q.y};
+      y[1] = cf{q.z, q.w};
+    };
+    auto store = [&](int row, const cf (&y)[2]) {
+      *reinterpret_cast<float4 *>(Y + row * CS + c) = make_float4(y[0].x, y[0].y, y[1].x, y[1].y);
+    };
+    if (h0) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) load(x[i], h0 + r + i);
 #pragma unroll 4
-  for (int t = 0; t < h0; ++t) {
-    const cplx<T> xt = x[t * xs];
+      for (int t = 0; t < h0; ++t) {
+        cf y[2];
+        load(y, t);
 #pragma unroll
-    for (int i = 0; i < H; ++i)
-      if (i < hw) v[i] = cfms(v[i], LOWER ? A[(h0 + i) * ks + t] : A[t * ks + h0 + i], xt);
+        for (int i = 0; i < 4; ++i) {
+          const cf q = LOWER ? A[(h0 + r + i) * ks + t] : A[t * ks + h0 + r + i];
+          x[i][0] = cfms(x[i][0], q, y[0]);
+          x[i][1] = cfms(x[i][1], q, y[1]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) store(h0 + r + i, x[i]);
+      __syncwarp();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[i][0] = x[i][1] = cf{0.f, 0.f};
+#pragma unroll 4
+    for (int t = 0; t < kDiagB; ++t) {
+      cf y[2];
+      load(y, h0 + t);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const cf q = diag_coef<float, LOWER>(A + h0 * ks + h0, ks, r + i, t);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          x[i][e].x = fmaf(q.x, y[e].x, fmaf(-q.y, y[e].y, x[i][e].x));
+          x[i][e].y = fmaf(q.x, y[e].y, fmaf(q.y, y[e].x, x[i][e].y));
+        }
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) store(h0 + r + i, x[i]);
+    __syncwarp();
   }
-#pragma unroll
-  for (int i = 0; i < H; ++i) {
-    if (i >= hw) break;
-#pragma unroll
-    for (int t = 0; t < i; ++t)
-      v[i] = cfms(v[i], LOWER ? A[(h0 + i) * ks + h0 + t] : A[(h0 + t) * ks + h0 + i], v[t]);
-    if (!LOWER) v[i] = cmul(v[i], dinv[h0 + i]);
-  }
-}
-// one column of U12 in place at y (row stride ld, global memory)
-template <class T, int H>
-__device__ __forceinline__ void narrow_upper(const cplx<T> *A, int ks, cplx<T> *y, int64_t ld, int h0, int hw) {
-  cplx<T> v[H];
-#pragma unroll
-  for (int i = 0; i < H; ++i) v[i] = i < hw ? ld_el(y + (h0 + i) * ld) : cplx<T>{0, 0};
-  narrow_block<T, H, true>(v, A, ks, y, ld, h0, hw, nullptr);
-#pragma unroll
-  for (int i = 0; i < H; ++i)
-    if (i < hw) st_el(y + (h0 + i) * ld, v[i]);
-}
-// one row of L21 in place in its column of the chunk tile
-template <class T, int H>
-__device__ __forceinline__ void narrow_lower(const cplx<T> *A, int ks, cplx<T> *z, const cplx<T> *dinv, int h0, int hw) {
-  cplx<T> v[H];
-#pragma unroll
-  for (int i = 0; i < H; ++i) v[i] = i < hw ? z[(h0 + i) * kNarrowCS] : cplx<T>{0, 0};
-  narrow_block<T, H, false>(v, A, ks, z, kNarrowCS, h0, hw, dinv);
-#pragma unroll
-  for (int i = 0; i < H; ++i)
-    if (i < hw) z[(h0 + i) * kNarrowCS] = v[i];
 }
 
+constexpr int kPanelColThreads = 128;
+// chunk width and padded sizes: the tile and F11 of one chunk leave room for at least two
+// CTAs per SM (complex128, 64 pivots: 104 KB at 32 columns; 64 would take 137)
 template <class T>
-__global__ void __launch_bounds__(kPanelColThreads, 3)
+__host__ __device__ constexpr int panel_cols(int k) {
+  return sizeof(T) == 8 && k > 40 ? 32 : 64;
+}
+template <class T>
+__host__ __device__ constexpr int panel_rows(int k) {
+  return sizeof(T) == 8 ? (k + 7) / 8 * 8 : (k + 15) / 16 * 16;
+}
+template <class T>
+__host__ __device__ constexpr int panel_ks(int k) {
+  return panel_rows<T>(k) + (sizeof(T) == 8 ? 4 : 1);
+}
+template <class T>
+__host__ __device__ constexpr size_t panel_smem(int k, int cw) {
+  return ((size_t)panel_rows<T>(k) * (panel_ks<T>(k) + cw + 2)) * sizeof(cplx<T>) + (size_t)panel_rows<T>(k) * sizeof(int);
+}
+
+template <class T, int CW>
+__global__ void __launch_bounds__(kPanelColThreads, sizeof(T) == 8 ? 3 : 4)
     sym_panel_kernel(FrontArgs<T> a, const NarrowTask *__restrict__ tasks, int nb, const uint16_t *__restrict__ apos,
                      const int *__restrict__ aslot) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int NW = kPanelColThreads / 32;
+  constexpr int NW = kPanelColThreads / 32, CS = CW + 2, NH = CW / 32;
   const NarrowTask tk = tasks[blockIdx.x / nb];
   const int fq = blockIdx.x % nb;
   const SymFront &s = a.sf[tk.f];
-  const int k = s.k, ks = k + 1, nc = min(64, s.m - k - tk.c0);
+  const int k = s.k, kp = panel_rows<T>(k), ks = panel_ks<T>(k), nc = min(CW, s.m - k - tk.c0);
   const int64_t ld = s.ld;
-  cplx<T> *A = reinterpret_cast<cplx<T> *>(smem_raw);   // F11 in pivot order: L and U
-  cplx<T> *ft = A + k * ks;                             // the chunk of F12, then of L21^T
-  cplx<T> *dinv = ft + k * kNarrowCS;
-  int *perm = reinterpret_cast<int *>(dinv + k);
+  cplx<T> *A = reinterpret_cast<cplx<T> *>(smem_raw);   // F11 in pivot order, zero past k
+  cplx<T> *Y = A + kp * ks;                             // the chunk
+  int *perm = reinterpret_cast<int *>(Y + kp * CS);
   cplx<T> *arena = a.arena + (int64_t)fq * a.stride;
   cplx<T> *F = arena + s.off;
   const double om = a.omega[fq];
@@ -385,65 +598,91 @@ __global__ void __launch_bounds__(kPanelColThreads, 3)
   const int nch = s.nch;
   {
     const int64_t m0 = s.imap[0], m1 = s.imap[1];
-    int j0[2], j1[2];
+    int j0[NH], j1[NH];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < NH; ++h) {
       const int c = lane + 32 * h;
       j0[h] = nch > 0 && c < nc ? a.imap[m0 + k + tk.c0 + c] : -1;
       j1[h] = nch > 1 && c < nc ? a.imap[m1 + k + tk.c0 + c] : -1;
     }
-#pragma unroll 2
-    for (int r = wid; r < k; r += NW) {
-      const int i0 = nch > 0 ? a.imap[m0 + r] : -1, i1 = nch > 1 ? a.imap[m1 + r] : -1;
-      const cplx<T> x0 = sym_gather(s, arena, i0, j0[0], i1, j1[0]), x1 = sym_gather(s, arena, i0, j0[1], i1, j1[1]);
-      ft[r * kNarrowCS + lane] = x0;
-      ft[r * kNarrowCS + lane + 32] = x1;
+    constexpr int U = 4;
+    for (int rb = wid; rb < kp; rb += U * NW) {
+      cplx<T> v[U][NH], d[U][2];
+      bool both[U][NH];
+      int i1[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int r = rb + u * NW;
+        const int i0 = nch > 0 && r < k ? a.imap[m0 + r] : -1;
+        i1[u] = nch > 1 && r < k ? a.imap[m1 + r] : -1;
+#pragma unroll
+        for (int h = 0; h < NH; ++h) {
+          int64_t at;
+          const bool has = sym_pick(s, i0, j0[h], i1[u], j1[h], at, both[u][h]);
+          v[u][h] = has ? ld_once(arena + at) : cplx<T>{0, 0};
+        }
+        // F11 (at most 64 columns; the padding is zero)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int c = lane + 32 * h;
+          d[u][h] = r < k && c < k ? ld_el(F + r * ld + c) : cplx<T>{0, 0};
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int r = rb + u * NW;
+        if (r >= kp) break;
+#pragma unroll
+        for (int h = 0; h < NH; ++h) {
+          if (both[u][h]) v[u][h] = v[u][h] + ld_once(arena + s.cb[1] + (int64_t)i1[u] * s.cld[1] + j1[h]);
+          Y[r * CS + lane + 32 * h] = v[u][h];
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          if (lane + 32 * h < ks) A[r * ks + lane + 32 * h] = d[u][h];
+        if (lane + 64 < ks) A[r * ks + lane + 64] = cplx<T>{0, 0};
+      }
     }
-    for (int r = wid; r < k; r += NW)
-      for (int c = lane; c < k; c += 32) A[r * ks + c] = ld_el(F + r * ld + c);
     for (int i = tid; i < k; i += kPanelColThreads) perm[i] = a.piv[(int64_t)fq * a.n + s.p0 + i];
   }
   __syncthreads();
-#pragma unroll 4
-  for (int q = tk.a0 + tid; q < tk.a1; q += kPanelColThreads) {
-    cplx<T> *d = ft + (apos[q] >> 6) * kNarrowCS + (apos[q] & 63);
-    *d = *d + to_t<T>(a_entry(a.Kc, a.Mc, a.Dc, aslot[q], om, a.beta));
-  }
-  for (int i = tid; i < k; i += kPanelColThreads) dinv[i] = cdiv(cplx<T>{1, 0}, A[i * ks + i]);
+  add_arrows(a, tk.a0, tk.a1, apos, aslot, om, [&](int p, cplx<T> e) {
+    cplx<T> *d = Y + (p >> 6) * CS + (p & 63);
+    *d = *d + e;
+  });
   __syncthreads();
-  // P F12 to the U12 rows (L21 is solved in place in the tile, U12 in global memory)
-  cplx<T> *Y = F + k + tk.c0;
-  for (int r = 16 + wid; r < k; r += NW)
+  // P F12 to the U12 rows; the tile is first solved as rows of L21
+  cplx<T> *U = F + k + tk.c0;
+  for (int r = wid; r < k; r += NW)
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < NH; ++h) {
       const int c = lane + 32 * h;
-      if (c < nc) st_el(Y + r * ld + c, ft[perm[r] * kNarrowCS + c]);
+      if (c < nc) st_el(U + r * ld + c, Y[perm[r] * CS + c]);
     }
-  const int c = tid & 63;
-  cplx<T> first[16];      // the first unknowns' right-hand sides, read before L21 overwrites the tile
-  if (tid < 64) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) first[i] = i < k ? ft[perm[i] * kNarrowCS + c] : cplx<T>{0, 0};
-  }
   __syncthreads();
-  if (tid < 64 && c < nc) {
-    narrow_block<T, 16, true>(first, A, ks, nullptr, 0, 0, min(16, k), nullptr);
-#pragma unroll
-    for (int i = 0; i < 16; ++i)
-      if (i < k) st_el(Y + i * ld + c, first[i]);
-    int h = 16;
-    for (; h + 16 <= k; h += 16) narrow_upper<T, 16>(A, ks, Y + c, ld, h, 16);
-    if (h + 8 <= k) narrow_upper<T, 8>(A, ks, Y + c, ld, h, 8), h += 8;
-    for (; h < k; h += 4) narrow_upper<T, 4>(A, ks, Y + c, ld, h, min(4, k - h));
-  } else if (tid >= 64 && c < nc) {
-    int h = 0;
-    for (; h + 16 <= k; h += 16) narrow_lower<T, 16>(A, ks, ft + c, dinv, h, 16);
-    if (h + 8 <= k) narrow_lower<T, 8>(A, ks, ft + c, dinv, h, 8), h += 8;
-    for (; h < k; h += 4) narrow_lower<T, 4>(A, ks, ft + c, dinv, h, min(4, k - h));
-  }
-  __syncthreads();
-  for (int q = wid; q < nc; q += NW)
-    for (int r = lane; r < k; r += 32) st_el(F + (k + tk.c0 + q) * ld + r, ft[r * kNarrowCS + q]);
+  // each warp on its own columns from here on
+  constexpr int WC = CW / NW;
+  const int cb = wid * WC;
+  auto solve = [&](auto lower) {
+    constexpr bool LOWER = decltype(lower)::value;
+    if constexpr (sizeof(T) == 8)
+      panel_dmma<LOWER, WC / 8>(A, ks, Y + cb, CS, k);
+    else
+      panel_simt<LOWER>(A, ks, Y + cb, CS, k);
+  };
+  solve(std::false_type{});
+  for (int q = 0; q < WC; ++q)
+    if (cb + q < nc)
+      for (int r = lane; r < k; r += 32) st_el(F + (k + tk.c0 + cb + q) * ld + r, Y[r * CS + cb + q]);
+  __syncwarp();
+  const int c = lane % WC;
+#pragma unroll 4
+  for (int r = lane / WC; r < kp; r += 32 / WC)
+    Y[r * CS + cb + c] = r < k && cb + c < nc ? ld_el(U + r * ld + cb + c) : cplx<T>{0, 0};
+  __syncwarp();
+  solve(std::true_type{});
+  for (int r = lane / WC; r < k; r += 32 / WC)
+    if (cb + c < nc) st_el(U + r * ld + cb + c, Y[r * CS + cb + c]);
 }
 
 }  // namespace ss
