@@ -84,61 +84,15 @@ __global__ void rhs_kernel(int64_t n, int nb, const double *__restrict__ omega, 
   b[(int64_t)f * n + R] = v * (-V * rs[R]);
 }
 
-// Q[f] = sum_R kq[R] cs[R] x[f][R] + V Qz, one block per frequency, fixed-order tree
-__global__ void charge_kernel(int64_t n, const cd *__restrict__ kq, const double *__restrict__ cs,
-                              const cd *__restrict__ x, const cd *__restrict__ Qz, double V, cd *__restrict__ Q) {
-  __shared__ cd red[256];
-  const int f = blockIdx.x;
+// Q[f] = sum_R kq[R] cs[R] x[f][R] + V Qz;  grid (8, nb)
+__global__ void __cluster_dims__(kRedCtas, 1, 1) __launch_bounds__(kRedThreads)
+    charge_kernel(int64_t n, const cd *__restrict__ kq, const double *__restrict__ cs, const cd *__restrict__ x,
+                  const cd *__restrict__ Qz, double V, cd *__restrict__ Q) {
+  const int f = blockIdx.y;
   cd acc{0.0, 0.0};
-  for (int64_t R = threadIdx.x; R < n; R += blockDim.x)
-    acc = acc + cmul(kq[R] * cs[R], x[(int64_t)f * n + R]);
-  red[threadIdx.x] = acc;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] = red[threadIdx.x] + red[threadIdx.x + s];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) Q[f] = red[0] + Qz[0] * V;
-}
-
-// r[f] = b[f] - A'(w_f) x[f]   (scaled system, FP64); a thread owns a row for a
-// block of kSpmvFreqs frequencies (the row's matrix data read once per block; each
-// frequency's sum in the order of a one-frequency product).
-// (vp: value slot of each pattern entry, for the transposed operator; nullptr = own slot)
-__global__ void residual_kernel(int64_t n, int nb, const int64_t *__restrict__ rp, const int64_t *__restrict__ ci,
-                                const int64_t *__restrict__ vp, const cd *__restrict__ K, const cd *__restrict__ M,
-                                const cd *__restrict__ D, const double *__restrict__ omega, double beta,
-                                const cd *__restrict__ b, const cd *__restrict__ x, cd *__restrict__ r) {
-  const int64_t R = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int f0 = blockIdx.y * kSpmvFreqs;
-  if (R >= n || f0 >= nb) return;
-  const int nf = min(kSpmvFreqs, nb - f0);
-  double w2[kSpmvFreqs], wb[kSpmvFreqs];
-  cd acc[kSpmvFreqs];
-#pragma unroll
-  for (int q = 0; q < kSpmvFreqs; ++q) {
-    const double w = q < nf ? omega[f0 + q] : 0.0;
-    w2[q] = w * w;
-    wb[q] = w * beta;
-    acc[q] = q < nf ? b[(int64_t)(f0 + q) * n + R] : cd{0.0, 0.0};
-  }
-  const cd *xb = x + (int64_t)f0 * n;
-  for (int64_t t = rp[R]; t < rp[R + 1]; ++t) {
-    const int64_t s = vp ? vp[t] : t;
-    const int64_t j = ci[t];
-    const cd Ks = K[s], Ms = M[s];
-    const cd Ds = D ? D[s] : cd{0.0, 0.0};
-#pragma unroll
-    for (int q = 0; q < kSpmvFreqs; ++q)
-      if (q < nf) {
-        cd a = Ks - Ms * w2[q];
-        if (D) a = a + cmul(cd{0.0, wb[q]}, Ds);
-        acc[q] = acc[q] - cmul(a, xb[(int64_t)q * n + j]);
-      }
-  }
-#pragma unroll
-  for (int q = 0; q < kSpmvFreqs; ++q)
-    if (q < nf) r[(int64_t)(f0 + q) * n + R] = acc[q];
+  SS_RED_LOOP(R, n) acc = acc + cmul(kq[R] * cs[R], x[(int64_t)f * n + R]);
+  acc = cluster_reduce(acc, SumOp{});
+  if (threadIdx.x == 0 && blockIdx.x == 0) Q[f] = acc + Qz[0] * V;
 }
 
 }  // namespace ss
@@ -1819,19 +1773,14 @@ __global__ void __launch_bounds__(256) front_tbwd_kernel(FrontArgs<T> a, cd *__r
   for (int i = threadIdx.x; i < k; i += blockDim.x) xf[p0 + i] = cd{(double)z[i].x, (double)z[i].y};
 }
 
-// out[f] = sum_R u[f][R] * v[f][R] (bilinear, no conjugate), fixed-order tree
-__global__ void dotu_kernel(int64_t n, const cd *__restrict__ u, const cd *__restrict__ v, cd *__restrict__ out) {
-  __shared__ cd red[256];
-  const int f = blockIdx.x;
+// out[f] = sum_R u[f][R] * v[f][R] (bilinear, no conjugate);  grid (8, nb)
+__global__ void __cluster_dims__(kRedCtas, 1, 1) __launch_bounds__(kRedThreads)
+    dotu_kernel(int64_t n, const cd *__restrict__ u, const cd *__restrict__ v, cd *__restrict__ out) {
+  const int f = blockIdx.y;
   cd acc{0.0, 0.0};
-  for (int64_t R = threadIdx.x; R < n; R += blockDim.x) acc = acc + cmul(u[(int64_t)f * n + R], v[(int64_t)f * n + R]);
-  red[threadIdx.x] = acc;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] = red[threadIdx.x] + red[threadIdx.x + s];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[f] = red[0];
+  SS_RED_LOOP(R, n) acc = acc + cmul(u[(int64_t)f * n + R], v[(int64_t)f * n + R]);
+  acc = cluster_reduce(acc, SumOp{});
+  if (threadIdx.x == 0 && blockIdx.x == 0) out[f] = acc;
 }
 
 // c[f][R] = kq[R] * cs[R] for every frequency of the chunk (the charge row in the
@@ -1844,33 +1793,20 @@ __global__ void charge_row_kernel(int64_t n, int nb, const cd *__restrict__ kq, 
   c[(int64_t)f * n + R] = kq[R] * cs[R];
 }
 
-// x += dx and per-frequency max |dx|, max |x| (for the refinement stopping test)
-__global__ void axpy_norm_kernel(int64_t n, cd *__restrict__ x, const cd *__restrict__ dx,
-                                 double *__restrict__ nrm) {
-  __shared__ double s_dx[256], s_x[256];
-  const int f = blockIdx.x;
-  double mdx = 0.0, mx = 0.0;
-  for (int64_t R = threadIdx.x; R < n; R += blockDim.x) {
+// x += dx and per-frequency max |dx|, max |x| (for the refinement stopping test); grid (8, nb)
+__global__ void __cluster_dims__(kRedCtas, 1, 1) __launch_bounds__(kRedThreads)
+    axpy_norm_kernel(int64_t n, cd *__restrict__ x, const cd *__restrict__ dx, double *__restrict__ nrm) {
+  const int f = blockIdx.y;
+  cd mx{0.0, 0.0};
+  SS_RED_LOOP(R, n) {
     const int64_t t = (int64_t)f * n + R;
-    const cd v = x[t] + dx[t];
+    const cd d = dx[t], v = x[t] + d;
     x[t] = v;
-    mdx = fmax(mdx, sqrt(cabs2(dx[t])));
-    mx = fmax(mx, sqrt(cabs2(v)));
+    mx.x = fmax(mx.x, sqrt(cabs2(d)));
+    mx.y = fmax(mx.y, sqrt(cabs2(v)));
   }
-  s_dx[threadIdx.x] = mdx;
-  s_x[threadIdx.x] = mx;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) {
-      s_dx[threadIdx.x] = fmax(s_dx[threadIdx.x], s_dx[threadIdx.x + s]);
-      s_x[threadIdx.x] = fmax(s_x[threadIdx.x], s_x[threadIdx.x + s]);
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    nrm[2 * f] = s_dx[0];
-    nrm[2 * f + 1] = s_x[0];
-  }
+  mx = cluster_reduce(mx, MaxOp{});
+  if (threadIdx.x == 0 && blockIdx.x == 0) nrm[2 * f] = mx.x, nrm[2 * f + 1] = mx.y;
 }
 
 }  // namespace ss
@@ -3631,11 +3567,11 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
     }
     if (getenv("SS_DEBUG_IR")) {
       // backward error of the direct solve: |b - A x| / |b|, and the solution size
-      residual_kernel<<<dim3(vb, spmv_blocks(nb)), 256, 0, h.stream>>>(n, nb, h.dc_ptr.as<int64_t>(), h.dc_idx.as<int64_t>(), nullptr,
-                                                          a.Kc, a.Mc, a.Dc, dom.as<double>(), h.beta, b.as<cd>(),
+      spmv_kernel<<<dim3(spmv_rows(n), spmv_blocks(nb)), 256, 0, h.stream>>>(
+          n, nb, h.dc_ptr.as<int64_t>(), h.dc_idx.as<int64_t>(), nullptr, a.Kc, a.Mc, a.Dc, dom.as<double>(), h.beta, b.as<cd>(),
                                                           x.as<cd>(), r.as<cd>());
-      norm2_kernel<<<nb, 256, 0, h.stream>>>(n, r.as<cd>(), nrm.as<double>());
-      norm2_kernel<<<nb, 256, 0, h.stream>>>(n, b.as<cd>(), nrm.as<double>() + nb);
+      norm2_kernel<<<dim3(kRedCtas, nb), kRedThreads, 0, h.stream>>>(n, r.as<cd>(), nrm.as<double>());
+      norm2_kernel<<<dim3(kRedCtas, nb), kRedThreads, 0, h.stream>>>(n, b.as<cd>(), nrm.as<double>() + nb);
       std::vector<double> q(2 * nb);
       cudaMemcpyAsync(q.data(), nrm.p, 2 * nb * sizeof(double), cudaMemcpyDeviceToHost, h.stream);
       cudaStreamSynchronize(h.stream);
@@ -3643,12 +3579,12 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
               q[0] / q[nb], q[nb - 1] / q[2 * nb - 1]);
     }
     for (int it = 0; it < (use_krylov ? 0 : maxit); ++it) {
-      residual_kernel<<<dim3(vb, spmv_blocks(nb)), 256, 0, h.stream>>>(n, nb, h.dc_ptr.as<int64_t>(), h.dc_idx.as<int64_t>(), nullptr,
-                                                          a.Kc, a.Mc, a.Dc, dom.as<double>(), h.beta, b.as<cd>(),
+      spmv_kernel<<<dim3(spmv_rows(n), spmv_blocks(nb)), 256, 0, h.stream>>>(
+          n, nb, h.dc_ptr.as<int64_t>(), h.dc_idx.as<int64_t>(), nullptr, a.Kc, a.Mc, a.Dc, dom.as<double>(), h.beta, b.as<cd>(),
                                                           x.as<cd>(), r.as<cd>());
       rc = sw.solve_graphed(1, nb, r.as<cd>(), dx.as<cd>());
       if (rc) return rc;
-      axpy_norm_kernel<<<nb, 256, 0, h.stream>>>(n, x.as<cd>(), dx.as<cd>(), nrm.as<double>());
+      axpy_norm_kernel<<<dim3(kRedCtas, nb), kRedThreads, 0, h.stream>>>(n, x.as<cd>(), dx.as<cd>(), nrm.as<double>());
       SS_CK(cudaMemcpyAsync(hn.data(), nrm.p, 2 * nb * sizeof(double), cudaMemcpyDeviceToHost, h.stream));
       SS_CK(cudaStreamSynchronize(h.stream));
       bool all = true;
@@ -3686,20 +3622,20 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
         for (int f = 0; f < nb; ++f) hit[f] += kits[f], aconv[f] = kconv[f], steps_a += kits[f];
       } else {
         // one FP64 refinement step, as for the primal solution
-        residual_kernel<<<dim3(vb, spmv_blocks(nb)), 256, 0, h.stream>>>(n, nb, opT.rp, opT.ci, opT.vp, a.Kc, a.Mc, a.Dc,
+        spmv_kernel<<<dim3(spmv_rows(n), spmv_blocks(nb)), 256, 0, h.stream>>>(n, nb, opT.rp, opT.ci, opT.vp, a.Kc, a.Mc, a.Dc,
                                                             dom.as<double>(), h.beta, cvec.as<cd>(), mu.as<cd>(),
                                                             r.as<cd>());
         rc = sw.solve_graphed(2, nb, r.as<cd>(), dx.as<cd>());
         if (rc) return rc;
-        axpy_norm_kernel<<<nb, 256, 0, h.stream>>>(n, mu.as<cd>(), dx.as<cd>(), nrm.as<double>());
+        axpy_norm_kernel<<<dim3(kRedCtas, nb), kRedThreads, 0, h.stream>>>(n, mu.as<cd>(), dx.as<cd>(), nrm.as<double>());
       }
       if (correct) {
         // dual-weighted correction: Q = c^T x + mu^T (b - A' x) is exact up to
         // (mu_exact - mu)^T (b - A' x), the product of the two solves' errors
-        residual_kernel<<<dim3(vb, spmv_blocks(nb)), 256, 0, h.stream>>>(n, nb, h.dc_ptr.as<int64_t>(), h.dc_idx.as<int64_t>(),
-                                                            nullptr, a.Kc, a.Mc, a.Dc, dom.as<double>(), h.beta,
+        spmv_kernel<<<dim3(spmv_rows(n), spmv_blocks(nb)), 256, 0, h.stream>>>(
+          n, nb, h.dc_ptr.as<int64_t>(), h.dc_idx.as<int64_t>(), nullptr, a.Kc, a.Mc, a.Dc, dom.as<double>(), h.beta,
                                                             b.as<cd>(), x.as<cd>(), r.as<cd>());
-        dotu_kernel<<<nb, 256, 0, h.stream>>>(n, mu.as<cd>(), r.as<cd>(), dQ.as<cd>() + B);
+        dotu_kernel<<<dim3(kRedCtas, nb), kRedThreads, 0, h.stream>>>(n, mu.as<cd>(), r.as<cd>(), dQ.as<cd>() + B);
         SS_CK(cudaMemcpyAsync(corr.data(), dQ.as<cd>() + B, nb * sizeof(cd), cudaMemcpyDeviceToHost, h.stream));
       }
       if (ex && ex->per_chunk) {
@@ -3707,7 +3643,7 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
         if (rc) return rc;
       }
     }
-    charge_kernel<<<nb, 256, 0, h.stream>>>(n, h.dks.as<cd>() + n, h.dcol_scale.as<double>(), x.as<cd>(),
+    charge_kernel<<<dim3(kRedCtas, nb), kRedThreads, 0, h.stream>>>(n, h.dks.as<cd>() + n, h.dcol_scale.as<double>(), x.as<cd>(),
                                             h.dQz.as<cd>(), V, dQ.as<cd>());
     SS_CK(cudaGetLastError());
     SS_CK(cudaMemcpyAsync(Qout + 2 * (int64_t)c0, dQ.p, nb * sizeof(cd), cudaMemcpyDeviceToHost, h.stream));
