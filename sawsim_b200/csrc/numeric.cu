@@ -1773,6 +1773,44 @@ __global__ void __launch_bounds__(256) front_tbwd_kernel(FrontArgs<T> a, cd *__r
   for (int i = threadIdx.x; i < k; i += blockDim.x) xf[p0 + i] = cd{(double)z[i].x, (double)z[i].y};
 }
 
+// s[f] = the least-squares ratio (b_f^H c_f) / (b_f^H b_f);  grid (8, nb)
+__global__ void __cluster_dims__(kRedCtas, 1, 1) __launch_bounds__(kRedThreads)
+    ratio_kernel(int64_t n, const cd *__restrict__ b, const cd *__restrict__ c, cd *__restrict__ s) {
+  const int f = blockIdx.y;
+  cd num{0.0, 0.0}, den{0.0, 0.0};
+  SS_RED_LOOP(R, n) {
+    const cd u = b[(int64_t)f * n + R], v = c[(int64_t)f * n + R];
+    num.x += u.x * v.x + u.y * v.y;
+    num.y += u.x * v.y - u.y * v.x;
+    den.x += cabs2(u);
+  }
+  num = cluster_reduce(num, SumOp{});
+  den = cluster_reduce(den, SumOp{});
+  if (threadIdx.x == 0 && blockIdx.x == 0) s[f] = den.x > 0.0 ? num * (1.0 / den.x) : cd{0.0, 0.0};
+}
+// nrm[2f], nrm[2f+1] = max |c_f - s_f b_f|, max |c_f| (infinite where c_f - s_f b_f is not a
+// number, so that the comparison fails);  grid (8, nb)
+__global__ void __cluster_dims__(kRedCtas, 1, 1) __launch_bounds__(kRedThreads)
+    ratio_check_kernel(int64_t n, const cd *__restrict__ b, const cd *__restrict__ c, const cd *__restrict__ s,
+                       double *__restrict__ nrm) {
+  const int f = blockIdx.y;
+  const cd sf = s[f];
+  cd mx{0.0, 0.0};
+  SS_RED_LOOP(R, n) {
+    const cd v = c[(int64_t)f * n + R];
+    const double d = sqrt(cabs2(v - cmul(sf, b[(int64_t)f * n + R])));
+    mx.x = fmax(mx.x, d == d ? d : INFINITY);
+    mx.y = fmax(mx.y, sqrt(cabs2(v)));
+  }
+  mx = cluster_reduce(mx, MaxOp{});
+  if (threadIdx.x == 0 && blockIdx.x == 0) nrm[2 * f] = mx.x, nrm[2 * f + 1] = mx.y;
+}
+// y_f = s_f x_f
+__global__ void scale_by_kernel(int64_t n, const cd *__restrict__ x, const cd *__restrict__ s, cd *__restrict__ y) {
+  const int64_t R = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (R < n) y[(int64_t)blockIdx.y * n + R] = cmul(s[blockIdx.y], x[(int64_t)blockIdx.y * n + R]);
+}
+
 // out[f] = sum_R u[f][R] * v[f][R] (bilinear, no conjugate);  grid (8, nb)
 __global__ void __cluster_dims__(kRedCtas, 1, 1) __launch_bounds__(kRedThreads)
     dotu_kernel(int64_t n, const cd *__restrict__ u, const cd *__restrict__ v, cd *__restrict__ out) {
@@ -3610,9 +3648,30 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
       const MatOp opT{h.dct_ptr.as<int64_t>(), h.dct_idx.as<int64_t>(), h.dct_src.as<int64_t>()};
       charge_row_kernel<<<dim3(vb, nb), 256, 0, h.stream>>>(n, nb, h.dks.as<cd>() + n, h.dcol_scale.as<double>(),
                                                           cvec.as<cd>());
-      rc = sw.solve_graphed(2, nb, cvec.as<cd>(), mu.as<cd>());
-      if (rc) return rc;
-      if (use_krylov) {
+      // On the symmetric path A'^T = A'; the charge functional is the electrode's row and
+      // the right-hand side its column, so c = s b as well and mu = s x: no second solve.
+      // Checked entry by entry for every point (dielectric or Rayleigh losses in the
+      // electrode's column, or an M that couples to it, end the proportion).
+      bool reuse = P.sym;
+      if (reuse) {
+        ratio_kernel<<<dim3(kRedCtas, nb), kRedThreads, 0, h.stream>>>(n, b.as<cd>(), cvec.as<cd>(), dQ.as<cd>());
+        ratio_check_kernel<<<dim3(kRedCtas, nb), kRedThreads, 0, h.stream>>>(n, b.as<cd>(), cvec.as<cd>(),
+                                                                            dQ.as<cd>(), nrm.as<double>());
+        std::vector<double> off(2 * nb);
+        SS_CK(cudaMemcpyAsync(off.data(), nrm.p, 2 * nb * sizeof(double), cudaMemcpyDeviceToHost, h.stream));
+        SS_CK(cudaStreamSynchronize(h.stream));
+        for (int f = 0; f < nb; ++f) reuse = reuse && off[2 * f] <= kSymTol * off[2 * f + 1];
+      }
+      if (reuse) {
+        scale_by_kernel<<<dim3(vb, nb), 256, 0, h.stream>>>(n, x.as<cd>(), dQ.as<cd>(), mu.as<cd>());
+        for (int f = 0; f < nb; ++f) aconv[f] = !use_krylov || conv[f];
+      } else {
+        rc = sw.solve_graphed(2, nb, cvec.as<cd>(), mu.as<cd>());
+        if (rc) return rc;
+      }
+      if (reuse) {
+        // nothing left to refine
+      } else if (use_krylov) {
         std::vector<int> kits;
         std::vector<char> kconv;
         auto pre = [&](const cd *src, cd *dst) { return sw.solve_graphed(2, nb, src, dst); };

@@ -106,3 +106,35 @@ def test_anisotropic_pml_slab_keeps_the_general_path(built_lib):
         assert e.stats()['symmetric'] == 0.0
     finally:
         e.close()
+
+
+@pytest.mark.parametrize('kind,size', [('me0_16x64', (8, 13)), ('me1_64x256', (8, 17))])
+@pytest.mark.parametrize('scale', [1.0, 1.5])
+def test_adjoint_solutions_of_a_symmetric_system(built_lib, kind, size, scale):
+    """The adjoint fields A^T l = kq, with the electrode's column proportional to its row
+    (one solve serves both) and with half of it scaled (two solves), in the oracle's system:
+    backward errors as for the fields."""
+    from oracle.solver import FrequencySolver as Oracle
+    c, make = _build(kind, size)
+    g = make()
+    K, M = g.export(L.SS_MAT_K), g.export(L.SS_MAT_M)
+    g.close()
+    zheng = np.asarray(c.bc[1], dtype=np.int64)
+    row = np.repeat(np.arange(K.shape[0]), np.diff(K.indptr))
+    K.data[np.isin(K.indices, zheng) & ~np.isin(row, zheng) & (row % 2 == 0)] *= scale
+    o = Oracle(K, M, *c.bc)
+    e = FrequencySolver.from_matrices(K, M, *c.bc)
+    try:
+        for f in c.freqs[:2]:
+            w = 2 * np.pi * f
+            A, _ = o.system(w)
+            lam = e.solve_adjoint(w, 'fp64')
+            Q, st, _ = e.charges(np.array([w]), 1.0, 'mixed')
+            Q0, st0, _ = e.charges(np.array([w]), 1.0, 'fp64')
+            kq = (o._T.T @ o.kts)[o.active]
+            r = A.T @ lam - kq
+            assert np.linalg.norm(r) / (sp.linalg.norm(A) * np.linalg.norm(lam) + np.linalg.norm(kq)) < 1e-12
+            assert st[0] == 0 and st0[0] == 0 and abs(Q[0] - Q0[0]) < 1e-6 * abs(Q0[0])
+        assert e.stats()['symmetric'] == 1.0
+    finally:
+        e.close()
