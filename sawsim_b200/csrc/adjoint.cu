@@ -347,45 +347,30 @@ int run_adjoint_gradient(Handle &h, int n_f, const double *omega, double V, int 
   const int npe = h.npe, dim = h.dim;
   const int64_t N = h.N, ne = h.ne, G = h.gdof, n = h.sym.n;
   // device copies of the mesh, materials and PML
-  DBuf dp, dcn, dem, drh, dCm, deM, depsM, dax, dnp, dreg, ddm, din, dout;
-  AD_CK(dupload(dp, h.pos));
-  AD_CK(dupload(dcn, h.conn));
-  AD_CK(dupload(dem, h.emat));
-  AD_CK(dupload(drh, h.rho[0]));
-  AD_CK(dupload(dCm, h.C[0]));
-  AD_CK(dupload(deM, h.e[0]));
-  AD_CK(dupload(depsM, h.eps[0]));
   PmlDev pml{};
-  pml.clip = h.pml_clip;
-  pml.omega = h.omega_top;
-  if (npml > 0) {
-    AD_CK(dupload(dax, h.pml_axis));
-    AD_CK(dupload(dnp, h.pml_npow));
-    AD_CK(dupload(dreg, h.elem_region));
-    AD_CK(dupload(ddm, h.pml_dmax));
-    AD_CK(dupload(din, h.pml_inner));
-    AD_CK(dupload(dout, h.pml_outer));
-    pml.axis = dax.as<int32_t>();
-    pml.npow = dnp.as<int32_t>();
-    pml.elem_region = dreg.as<int32_t>();
-    pml.dmax = ddm.as<double>();
-    pml.inner = din.as<double>();
-    pml.outer = dout.as<double>();
+  int rc0 = mesh_device(h);
+  if (!rc0) rc0 = material_device(h, 0, pml);
+  if (rc0) return rc0;
+  const MeshDev &md = h.mesh;
+  // seeds, parameter-major, one buffer: positions, C, e, eps, rho, PML inner and outer bounds
+  struct SeedArray {
+    const double *src;
+    size_t each, at;
+  } seeds[7] = {{dpos, (size_t)(N * dim), 0}, {dC, (size_t)nm * 72, 0},  {de, (size_t)nm * 36, 0},
+                {deps, (size_t)nm * 18, 0},   {drho, (size_t)nm, 0},     {npml ? dinner : nullptr, (size_t)npml * 3, 0},
+                {npml ? douter : nullptr, (size_t)npml * 3, 0}};
+  DBuf dgn, dsp, dseed, own;
+  {
+    std::vector<double> all;
+    for (SeedArray &a : seeds) {
+      a.at = all.size();
+      if (a.src) all.insert(all.end(), a.src, a.src + (size_t)n_params * a.each);
+    }
+    AD_CK(dupload(dseed, all, h.stream));
   }
-  // seeds, parameter-major
-  auto up = [&](DBuf &b, const double *src, size_t cnt) -> cudaError_t {
-    if (!src) return cudaSuccess;
-    std::vector<double> v(src, src + cnt);
-    return dupload(b, v);
+  auto seed = [&](int i, int p) -> const double * {
+    return seeds[i].src ? dseed.as<double>() + seeds[i].at + (size_t)p * seeds[i].each : nullptr;
   };
-  DBuf sp, sC, se, seps, srho, sin, sout;
-  AD_CK(up(sp, dpos, (size_t)n_params * N * dim));
-  AD_CK(up(sC, dC, (size_t)n_params * nm * 72));
-  AD_CK(up(se, de, (size_t)n_params * nm * 36));
-  AD_CK(up(seps, deps, (size_t)n_params * nm * 18));
-  AD_CK(up(srho, drho, (size_t)n_params * nm));
-  AD_CK(up(sin, npml ? dinner : nullptr, (size_t)n_params * npml * 3));
-  AD_CK(up(sout, npml ? douter : nullptr, (size_t)n_params * npml * 3));
   // DOF maps: new index of each DOF's master, -1 on the + electrode, -2 otherwise
   std::vector<int64_t> gnew(G, -2);
   std::vector<unsigned char> splus(G, 0);
@@ -395,58 +380,58 @@ int run_adjoint_gradient(Handle &h, int n_f, const double *omega, double V, int 
   }
   for (int64_t z : h.zheng) gnew[z] = -1, splus[z] = 1;
   for (int64_t z : h.fu) gnew[z] = -2;
-  DBuf dgn, dsp, dK, dM, dd, dm, dpart, dout2, dom;
-  AD_CK(dupload(dgn, gnew));
-  AD_CK(dupload(dsp, splus));
-  AD_CK(dalloc(dK, (size_t)ne * nc * nc * npe * npe * sizeof(cd)));
-  AD_CK(dalloc(dM, (size_t)ne * npe * npe * sizeof(cd)));
+  AD_CK(dupload(dgn, gnew, h.stream));
+  AD_CK(dupload(dsp, splus, h.stream));
+  auto seed_of = [&](int p) {
+    Seed sd{};
+    sd.dpos = seed(0, p);
+    sd.dC = seed(1, p);
+    sd.de = seed(2, p);
+    sd.deps = seed(3, p);
+    sd.drho = seed(4, p);
+    sd.dinner = seed(5, p);
+    sd.douter = seed(6, p);
+    return sd;
+  };
   SweepExtra ex;
   ex.per_chunk = [&](int c0, int nb, const cplx<double> *x, const cplx<double> *mu) -> int {
-    AD_CK(dalloc(dd, (size_t)nb * G * sizeof(cd)));
-    AD_CK(dalloc(dm, (size_t)nb * G * sizeof(cd)));
-    AD_CK(dalloc(dpart, (size_t)nb * ne * sizeof(cd)));
-    AD_CK(dalloc(dout2, (size_t)nb * sizeof(cd)));
-    AD_CK(dalloc(dom, (size_t)nb * sizeof(double)));
-    AD_CK(cudaMemcpyAsync(dom.p, omega + c0, nb * sizeof(double), cudaMemcpyHostToDevice, h.stream));
+    // the fronts of this chunk are done with: their arena holds the element tangents, the
+    // expanded vectors and the partial sums
+    const int64_t kel = ne * nc * nc * npe * npe, mel = ne * npe * npe;
+    cd *dK = nullptr;
+    AD_CK(element_scratch(h, own, (size_t)(kel + mel + 2 * nb * G + nb * ne + nb * n_params + nb) * sizeof(cd), dK));
+    cd *dM = dK + kel, *dd = dM + mel, *dm = dd + nb * G, *dpart = dm + nb * G, *dout2 = dpart + nb * ne;
+    double *dom = reinterpret_cast<double *>(dout2 + (int64_t)nb * n_params);
+    AD_CK(cudaMemcpyAsync(dom, omega + c0, nb * sizeof(double), cudaMemcpyHostToDevice, h.stream));
     expand_kernel<<<dim3((unsigned)((G + 255) / 256), nb), 256, 0, h.stream>>>(
-        G, nb, n, dgn.as<int64_t>(), h.dcol_scale.as<double>(), h.drow_scale.as<double>(), x, mu, V, dd.as<cd>(),
-        dm.as<cd>());
-    std::vector<cd> out(nb);
+        G, nb, n, dgn.as<int64_t>(), h.dcol_scale.as<double>(), h.drow_scale.as<double>(), x, mu, V, dd, dm);
     for (int p = 0; p < n_params; ++p) {
-      Seed sd{};
-      sd.dpos = sp.p ? sp.as<double>() + (size_t)p * N * dim : nullptr;
-      sd.dC = sC.p ? sC.as<double>() + (size_t)p * nm * 72 : nullptr;
-      sd.de = se.p ? se.as<double>() + (size_t)p * nm * 36 : nullptr;
-      sd.deps = seps.p ? seps.as<double>() + (size_t)p * nm * 18 : nullptr;
-      sd.drho = srho.p ? srho.as<double>() + (size_t)p * nm : nullptr;
-      sd.dinner = sin.p ? sin.as<double>() + (size_t)p * npml * 3 : nullptr;
-      sd.douter = sout.p ? sout.as<double>() + (size_t)p * npml * 3 : nullptr;
+      const Seed sd = seed_of(p);
+      const double *pos = md.pos.as<double>(), *rho = md.mat[0].as<double>(), *C = md.mat[1].as<double>(),
+                   *em = md.mat[2].as<double>(), *epsm = md.mat[3].as<double>();
+      const int64_t *cn = md.conn.as<int64_t>();
+      const int32_t *mat = md.emat.as<int32_t>();
       if (hex) {
-        AD_CK(launch_hex27_tangent(h.stream, ne, dp.as<double>(), dcn.as<int64_t>(), dem.as<int32_t>(),
-                                   drh.as<double>(), dCm.as<double>(), deM.as<double>(), depsM.as<double>(), pml, sd,
-                                   dK.as<cd>(), dM.as<cd>()));
-        contract_hex_kernel<<<(unsigned)ne, 256, 0, h.stream>>>(ne, N, nb, G, dcn.as<int64_t>(), dK.as<cd>(),
-                                                                dM.as<cd>(), dd.as<cd>(), dm.as<cd>(),
-                                                                dsp.as<unsigned char>(), dom.as<double>(),
-                                                                dpart.as<cd>());
+        AD_CK(launch_hex27_tangent(h.stream, ne, pos, cn, mat, rho, C, em, epsm, pml, sd, dK, dM));
+        contract_hex_kernel<<<(unsigned)ne, 256, 0, h.stream>>>(ne, N, nb, G, cn, dK, dM, dd, dm,
+                                                                dsp.as<unsigned char>(), dom, dpart);
       } else {
-        q9_tangent_kernel<<<(unsigned)((ne + 3) / 4), 128, 0, h.stream>>>(
-            ne, nc, dp.as<double>(), dcn.as<int64_t>(), dem.as<int32_t>(), drh.as<double>(), dCm.as<double>(),
-            deM.as<double>(), depsM.as<double>(), pml, sd, dK.as<cd>(), dM.as<cd>());
-        contract_kernel<<<(unsigned)ne, 128, 0, h.stream>>>(ne, nc, ndisp, N, nb, G, dcn.as<int64_t>(), dK.as<cd>(),
-                                                            dM.as<cd>(), dd.as<cd>(), dm.as<cd>(),
-                                                            dsp.as<unsigned char>(), dom.as<double>(),
-                                                            dpart.as<cd>());
+        q9_tangent_kernel<<<(unsigned)((ne + 3) / 4), 128, 0, h.stream>>>(ne, nc, pos, cn, mat, rho, C, em, epsm, pml,
+                                                                          sd, dK, dM);
+        contract_kernel<<<(unsigned)ne, 128, 0, h.stream>>>(ne, nc, ndisp, N, nb, G, cn, dK, dM, dd, dm,
+                                                            dsp.as<unsigned char>(), dom, dpart);
       }
-      sum_rows_kernel<<<nb, 256, 0, h.stream>>>(ne, dpart.as<cd>(), dout2.as<cd>());
+      sum_rows_kernel<<<nb, 256, 0, h.stream>>>(ne, dpart, dout2 + (int64_t)p * nb);
       AD_CK(cudaGetLastError());
-      AD_CK(cudaMemcpyAsync(out.data(), dout2.p, nb * sizeof(cd), cudaMemcpyDeviceToHost, h.stream));
-      AD_CK(cudaStreamSynchronize(h.stream));
-      for (int f = 0; f < nb; ++f) {
-        dQ[2 * ((int64_t)(c0 + f) * n_params + p)] = out[f].x;
-        dQ[2 * ((int64_t)(c0 + f) * n_params + p) + 1] = out[f].y;
-      }
     }
+    std::vector<cd> out((size_t)nb * n_params);
+    AD_CK(cudaMemcpyAsync(out.data(), dout2, out.size() * sizeof(cd), cudaMemcpyDeviceToHost, h.stream));
+    AD_CK(cudaStreamSynchronize(h.stream));
+    for (int p = 0; p < n_params; ++p)
+      for (int f = 0; f < nb; ++f) {
+        dQ[2 * ((int64_t)(c0 + f) * n_params + p)] = out[(size_t)p * nb + f].x;
+        dQ[2 * ((int64_t)(c0 + f) * n_params + p) + 1] = out[(size_t)p * nb + f].y;
+      }
     return SS_OK;
   };
   std::vector<int> st(n_f, 0), it(n_f, 0);

@@ -243,10 +243,14 @@ cudaError_t dalloc(DBuf &b, size_t bytes) {
   return e;
 }
 
-int launch_assemble(Handle &h, int which) {
-  const int npe = h.npe, nc = h.nc, npe2 = npe * npe;
+// The mesh's device copies and the node-pair gather lists (element-ascending sources of
+// every pair): they change with the mesh only, so a reassembly (new materials, PML or
+// freeze frequency) finds them here instead of rebuilding and uploading them (6 of the 10
+// ms that a reassembly of the 16x67 ME1 cell took).
+int mesh_device(Handle &h) {
+  if (h.mesh.ready) return SS_OK;
+  const int npe = h.npe, npe2 = npe * npe;
   const int64_t ne = h.ne, N = h.N;
-  // node-pair gather lists, element-ascending
   const int64_t npairs = h.nadj_ptr[N];
   std::vector<int64_t> cnt(npairs + 1, 0), src((size_t)ne * npe2);
   std::vector<int64_t> pidx((size_t)ne * npe2);
@@ -269,42 +273,79 @@ int launch_assemble(Handle &h, int which) {
   std::vector<int32_t> prow(npairs);
   for (int64_t i = 0; i < N; ++i)
     for (int64_t p = h.nadj_ptr[i]; p < h.nadj_ptr[i + 1]; ++p) prow[p] = (int32_t)i;
-  pidx.clear();
-
-  DBuf dpos, dconn, demat, drho, dC, de, deps, dax, dnp, dreg, ddm, din, dout, dKel, dMel, dprow, dnadj, dindptr,
-      dgp, dgs;
   cudaError_t err;
 #define SS_TRY(x)                                   \
   do {                                              \
     if ((err = (x)) != cudaSuccess) return cuda_fail(h, err, #x); \
   } while (0)
-  SS_TRY(dupload(dpos, h.pos));
-  SS_TRY(dupload(dconn, h.conn));
-  SS_TRY(dupload(demat, h.emat));
-  const int wm = which;
-  SS_TRY(dupload(drho, h.rho[wm]));
-  SS_TRY(dupload(dC, h.C[wm]));
-  SS_TRY(dupload(de, h.e[wm]));
-  SS_TRY(dupload(deps, h.eps[wm]));
-  PmlDev pml{};
+  SS_TRY(dupload(h.mesh.pos, h.pos, h.stream));
+  SS_TRY(dupload(h.mesh.conn, h.conn, h.stream));
+  SS_TRY(dupload(h.mesh.emat, h.emat, h.stream));
+  SS_TRY(dupload(h.mesh.prow, prow, h.stream));
+  SS_TRY(dupload(h.mesh.nadj, h.nadj_ptr, h.stream));
+  SS_TRY(dupload(h.mesh.indptr, h.indptr, h.stream));
+  SS_TRY(dupload(h.mesh.gp, cnt, h.stream));
+  SS_TRY(dupload(h.mesh.gs, src, h.stream));
+  h.mesh.ready = true;
+  return SS_OK;
+}
+
+// Device copies of the materials (0 K/M, 1 D) and the PML arrays
+int material_device(Handle &h, int which, PmlDev &pml) {
+  cudaError_t err;
+  MeshDev &d = h.mesh;
+  SS_TRY(dupload(d.mat[0], h.rho[which], h.stream));
+  SS_TRY(dupload(d.mat[1], h.C[which], h.stream));
+  SS_TRY(dupload(d.mat[2], h.e[which], h.stream));
+  SS_TRY(dupload(d.mat[3], h.eps[which], h.stream));
+  pml = PmlDev{};
   pml.clip = h.pml_clip;
   pml.omega = h.omega_top;
   if (h.npml > 0) {
-    SS_TRY(dupload(dax, h.pml_axis));
-    SS_TRY(dupload(dnp, h.pml_npow));
-    SS_TRY(dupload(dreg, h.elem_region));
-    SS_TRY(dupload(ddm, h.pml_dmax));
-    SS_TRY(dupload(din, h.pml_inner));
-    SS_TRY(dupload(dout, h.pml_outer));
-    pml.axis = dax.as<int32_t>();
-    pml.npow = dnp.as<int32_t>();
-    pml.elem_region = dreg.as<int32_t>();
-    pml.dmax = ddm.as<double>();
-    pml.inner = din.as<double>();
-    pml.outer = dout.as<double>();
+    SS_TRY(dupload(d.pml[0], h.pml_axis, h.stream));
+    SS_TRY(dupload(d.pml[1], h.pml_npow, h.stream));
+    SS_TRY(dupload(d.pml[2], h.elem_region, h.stream));
+    SS_TRY(dupload(d.pml[3], h.pml_dmax, h.stream));
+    SS_TRY(dupload(d.pml[4], h.pml_inner, h.stream));
+    SS_TRY(dupload(d.pml[5], h.pml_outer, h.stream));
+    pml.axis = d.pml[0].as<int32_t>();
+    pml.npow = d.pml[1].as<int32_t>();
+    pml.elem_region = d.pml[2].as<int32_t>();
+    pml.dmax = d.pml[3].as<double>();
+    pml.inner = d.pml[4].as<double>();
+    pml.outer = d.pml[5].as<double>();
   }
-  SS_TRY(dalloc(dKel, (size_t)ne * nc * nc * npe2 * sizeof(cd)));
-  SS_TRY(dalloc(dMel, (size_t)ne * npe2 * sizeof(cd)));
+  return SS_OK;
+}
+
+// Space for the element matrices of one assembly: the front arena of an earlier sweep
+// (nothing in it outlives its sweep) where that is large enough, else `own`
+cudaError_t element_scratch(Handle &h, DBuf &own, size_t bytes, cd *&p) {
+  p = h.wk[0].as<cd>();
+  if (h.wk[0].bytes >= bytes) return cudaSuccess;
+  const cudaError_t e = dalloc(own, bytes);
+  p = own.as<cd>();
+  return e;
+}
+
+int launch_assemble(Handle &h, int which) {
+  const int npe = h.npe, nc = h.nc, npe2 = npe * npe;
+  const int64_t ne = h.ne, N = h.N;
+  const int64_t npairs = h.nadj_ptr[N];
+  cudaError_t err;
+  int rc0 = mesh_device(h);
+  if (rc0) return rc0;
+  PmlDev pml{};
+  rc0 = material_device(h, which, pml);
+  if (rc0) return rc0;
+  const MeshDev &d = h.mesh;
+  const double *drho = d.mat[0].as<double>(), *dC = d.mat[1].as<double>(), *de = d.mat[2].as<double>(),
+               *deps = d.mat[3].as<double>();
+  DBuf own;
+  cd *Kel = nullptr;
+  const int64_t kel = ne * nc * nc * npe2;
+  SS_TRY(element_scratch(h, own, (size_t)(kel + ne * npe2) * sizeof(cd), Kel));
+  cd *Mel = Kel + kel;
   // the element and scatter kernels are timed by events (stats slots 34 and 35)
   cudaEvent_t ev[3];
   for (auto &x : ev) SS_TRY(cudaEventCreate(&x));
@@ -314,22 +355,15 @@ int launch_assemble(Handle &h, int which) {
   } ev_free{ev};
   SS_TRY(cudaEventRecord(ev[0], h.stream));
   if (h.kind == SS_HEX27) {
-    int rc = launch_hex27_elements(h, which, pml, dKel.as<cd>(), dMel.as<cd>(), dpos.as<double>(),
-                                   dconn.as<int64_t>(), demat.as<int32_t>(), drho.as<double>(), dC.as<double>(),
-                                   de.as<double>(), deps.as<double>());
+    int rc = launch_hex27_elements(h, which, pml, Kel, Mel, d.pos.as<double>(), d.conn.as<int64_t>(),
+                                   d.emat.as<int32_t>(), drho, dC, de, deps);
     if (rc) return rc;
   } else {
     q9_element_kernel<<<(unsigned)((ne + 3) / 4), 128, 0, h.stream>>>(
-        ne, nc, dpos.as<double>(), dconn.as<int64_t>(), demat.as<int32_t>(), drho.as<double>(), dC.as<double>(),
-        de.as<double>(), deps.as<double>(), pml, dKel.as<cd>(), dMel.as<cd>());
+        ne, nc, d.pos.as<double>(), d.conn.as<int64_t>(), d.emat.as<int32_t>(), drho, dC, de, deps, pml, Kel, Mel);
     SS_TRY(cudaGetLastError());
   }
   SS_TRY(cudaEventRecord(ev[1], h.stream));
-  SS_TRY(dupload(dprow, prow));
-  SS_TRY(dupload(dnadj, h.nadj_ptr));
-  SS_TRY(dupload(dindptr, h.indptr));
-  SS_TRY(dupload(dgp, cnt));
-  SS_TRY(dupload(dgs, src));
   DBuf &dst = which ? h.dD : h.dK;
   SS_TRY(dalloc(dst, (size_t)h.nnz * sizeof(cd)));
   SS_TRY(cudaMemsetAsync(dst.p, 0, (size_t)h.nnz * sizeof(cd), h.stream));
@@ -345,8 +379,8 @@ int launch_assemble(Handle &h, int which) {
   SS_TRY(cudaEventCreate(&g0));
   SS_TRY(cudaEventRecord(g0, h.stream));
   gather_pairs_kernel<<<(unsigned)((nt + 255) / 256), 256, 0, h.stream>>>(
-      npairs, nc, npe2, h.kind == SS_HEX27, ndisp, N, dprow.as<int32_t>(), dnadj.as<int64_t>(),
-      dindptr.as<int64_t>(), dgp.as<int64_t>(), dgs.as<int64_t>(), dKel.as<cd>(), dMel.as<cd>(), dst.as<cd>(), dM);
+      npairs, nc, npe2, h.kind == SS_HEX27, ndisp, N, d.prow.as<int32_t>(), d.nadj.as<int64_t>(),
+      d.indptr.as<int64_t>(), d.gp.as<int64_t>(), d.gs.as<int64_t>(), Kel, Mel, dst.as<cd>(), dM);
   SS_TRY(cudaGetLastError());
   SS_TRY(cudaEventRecord(ev[2], h.stream));
   SS_TRY(cudaStreamSynchronize(h.stream));

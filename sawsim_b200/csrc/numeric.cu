@@ -2515,33 +2515,32 @@ static int equilibrate_sym(Handle &h, double w, bool &ok) {
   constexpr int kParts = 592;
   SS_CK(dalloc(h.drow_scale, n * sizeof(double)));
   SS_CK(dalloc(h.dcol_scale, n * sizeof(double)));
-  DBuf phi, part, t, d, flag;
-  SS_CK(dalloc(phi, n));
-  SS_CK(dalloc(part, 2 * kParts * sizeof(double)));
-  SS_CK(dalloc(t, n * sizeof(double)));
-  SS_CK(dalloc(d, n * sizeof(double)));
-  SS_CK(dalloc(flag, sizeof(int)));
+  // workspace: t, d (n doubles each), the ratio's partial sums, the flag, phi (n bytes)
+  SS_CK(dalloc(h.eq_ws, (2 * n + 2 * kParts + 1) * sizeof(double) + n));
+  double *t = h.eq_ws.as<double>(), *d = t + n, *part = d + n;
+  int *flag = reinterpret_cast<int *>(part + 2 * kParts);
+  unsigned char *phi = reinterpret_cast<unsigned char *>(part + 2 * kParts + 1);
   const int64_t *rp = h.dc_ptr.as<int64_t>(), *ci = h.dc_idx.as<int64_t>();
   const cd *D = h.have_D && h.beta ? h.dDc.as<cd>() : nullptr;
-  sym_phi_kernel<<<nb, 256, 0, h.stream>>>(n, rp, ci, h.dMc.as<cd>(), phi.as<unsigned char>());
-  sym_ratio_kernel<<<kParts, 256, 0, h.stream>>>(n, rp, ci, h.dKc.as<cd>(), phi.as<unsigned char>(), part.as<double>());
-  sym_factor_kernel<<<std::min(nb, 148u), 256, 0, h.stream>>>(n, kParts, part.as<double>(), phi.as<unsigned char>(),
-                                                              t.as<double>(), d.as<double>());
+  sym_phi_kernel<<<nb, 256, 0, h.stream>>>(n, rp, ci, h.dMc.as<cd>(), phi);
+  sym_ratio_kernel<<<kParts, 256, 0, h.stream>>>(n, rp, ci, h.dKc.as<cd>(), phi, part);
+  sym_factor_kernel<<<std::min(nb, 148u), 256, 0, h.stream>>>(n, kParts, part, phi,
+                                                              t, d);
   // three Ruiz steps, from d to drow_scale and back (the third ends in drow_scale)
-  double *from = d.as<double>(), *to = h.drow_scale.as<double>();
+  double *from = d, *to = h.drow_scale.as<double>();
   for (int it = 0; it < 3; ++it) {
     sym_ruiz_kernel<<<wb, 256, 0, h.stream>>>(n, rp, ci, h.dKc.as<cd>(), h.dMc.as<cd>(), D, w * w, w * h.beta,
-                                              t.as<double>(), from, to);
+                                              t, from, to);
     std::swap(from, to);
   }
-  sym_cols_kernel<<<nb, 256, 0, h.stream>>>(n, t.as<double>(), h.drow_scale.as<double>(), h.dcol_scale.as<double>());
+  sym_cols_kernel<<<nb, 256, 0, h.stream>>>(n, t, h.drow_scale.as<double>(), h.dcol_scale.as<double>());
   int rc = scale_values(h);
   if (rc) return rc;
-  SS_CK(cudaMemsetAsync(flag.p, 0, sizeof(int), h.stream));
+  SS_CK(cudaMemsetAsync(flag, 0, sizeof(int), h.stream));
   sym_check_kernel<<<wb, 256, 0, h.stream>>>(n, rp, ci, h.dKs.as<cd>(), h.dMs.as<cd>(),
-                                             D ? h.dDs.as<cd>() : nullptr, w * w, w * h.beta, kSymTol, flag.as<int>());
+                                             D ? h.dDs.as<cd>() : nullptr, w * w, w * h.beta, kSymTol, flag);
   int bad = 0;
-  SS_CK(cudaMemcpyAsync(&bad, flag.p, sizeof(int), cudaMemcpyDeviceToHost, h.stream));
+  SS_CK(cudaMemcpyAsync(&bad, flag, sizeof(int), cudaMemcpyDeviceToHost, h.stream));
   SS_CK(cudaStreamSynchronize(h.stream));
   ok = bad == 0;
   if (ok) h.scale_w = w;
@@ -3498,8 +3497,6 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
   if (need_adjoint) {
     SS_CK(dalloc(mu, (size_t)B * n * sizeof(cd)));
     SS_CK(dalloc(cvec, (size_t)B * n * sizeof(cd)));
-    int rc = build_transpose(h);
-    if (rc) return rc;
   }
   DBuf &stb = h.wk[14], &stx = h.wk[15];
   SS_CK(dalloc(stb, (size_t)B * n * sizeof(cd)));
@@ -3645,7 +3642,6 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
     std::vector<cd> corr(nb, cd{0.0, 0.0});
     std::vector<char> aconv(nb, 1);
     if (need_adjoint) {
-      const MatOp opT{h.dct_ptr.as<int64_t>(), h.dct_idx.as<int64_t>(), h.dct_src.as<int64_t>()};
       charge_row_kernel<<<dim3(vb, nb), 256, 0, h.stream>>>(n, nb, h.dks.as<cd>() + n, h.dcol_scale.as<double>(),
                                                           cvec.as<cd>());
       // On the symmetric path A'^T = A'; the charge functional is the electrode's row and
@@ -3666,9 +3662,12 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
         scale_by_kernel<<<dim3(vb, nb), 256, 0, h.stream>>>(n, x.as<cd>(), dQ.as<cd>(), mu.as<cd>());
         for (int f = 0; f < nb; ++f) aconv[f] = !use_krylov || conv[f];
       } else {
+        rc = build_transpose(h);
+        if (rc) return rc;
         rc = sw.solve_graphed(2, nb, cvec.as<cd>(), mu.as<cd>());
         if (rc) return rc;
       }
+      const MatOp opT{h.dct_ptr.as<int64_t>(), h.dct_idx.as<int64_t>(), h.dct_src.as<int64_t>()};
       if (reuse) {
         // nothing left to refine
       } else if (use_krylov) {

@@ -78,6 +78,7 @@ extern "C" int ss_set_mesh(ss_handle *hp, int kind, int64_t n_nodes, const doubl
   if (kind < SS_Q9_ME0 || kind > SS_HEX27) return fail(h, SS_EINVAL, "unknown element kind (SS_MATRIX: ss_set_csr)");
   if (n_nodes <= 0 || n_elem <= 0 || !pos || !conn || !emat) return fail(h, SS_EINVAL, "empty mesh or null array");
   if (!all_finite(pos, n_nodes * (kind == SS_HEX27 ? 3 : 2))) return fail(h, SS_EINVAL, "non-finite coordinate");
+  h.mesh.release();
   h.kind = kind;
   h.npe = kind == SS_HEX27 ? 27 : 9;
   h.dim = kind == SS_HEX27 ? 3 : 2;
@@ -230,6 +231,7 @@ extern "C" int ss_set_csr(ss_handle *hp, int64_t gdof, const int64_t *indptr, co
   if (node_xyz && (dim < 2 || dim > 3)) return fail(h, SS_EINVAL, "csr: dim must be 2 or 3");
   if (node_xyz && !all_finite(node_xyz, n_nodes * dim)) return fail(h, SS_EINVAL, "csr: non-finite coordinate");
   reset_derived(h);
+  h.mesh.release();
   h.kind = SS_MATRIX;
   h.npe = 0;
   h.nc = 0;

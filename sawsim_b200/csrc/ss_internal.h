@@ -25,6 +25,19 @@ struct DBuf {
   template <class T> T *as() const { return reinterpret_cast<T *>(p); }
 };
 
+// Device copies that depend on the mesh alone (its arrays and the gather lists of the
+// assembly), built by the first assembly and kept until the next mesh; and small buffers
+// of the material and PML arrays, filled on every use
+struct MeshDev {
+  bool ready = false;
+  DBuf pos, conn, emat, prow, nadj, indptr, gp, gs;
+  DBuf mat[4], pml[6];
+  void release() {
+    ready = false;
+    for (DBuf *b : {&pos, &conn, &emat, &prow, &nadj, &indptr, &gp, &gs}) b->release();
+  }
+};
+
 // FGMRES workspace (basis, preconditioned basis, Hessenberg data); held by the
 // handle so that repeated mixed sweeps reuse it
 struct KrylovWork {
@@ -46,6 +59,14 @@ cudaError_t dupload(DBuf &b, const std::vector<T> &v) {
   cudaError_t e = dalloc(b, v.size() * sizeof(T) + 16);
   if (e != cudaSuccess) return e;
   return v.empty() ? cudaSuccess : cudaMemcpy(b.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
+}
+
+// the same in the stream's order (the host vector may go once this returns)
+template <class T>
+cudaError_t dupload(DBuf &b, const std::vector<T> &v, cudaStream_t stream) {
+  const cudaError_t e = dalloc(b, v.size() * sizeof(T) + 16);
+  if (e != cudaSuccess || v.empty()) return e;
+  return cudaMemcpyAsync(b.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, stream);
 }
 
 // ---------------------------------------------------------------- symbolic data
@@ -137,6 +158,8 @@ struct Handle {
   // numeric work
   DBuf arena, piv, dperm_new, work;
   DBuf wk[16];                           // sweep work buffers, kept across calls
+  MeshDev mesh;                          // device copies of the mesh, kept until the next one
+  DBuf eq_ws;                            // equilibration workspace (about 18 bytes per row)
   DBuf dct_ptr, dct_idx, dct_src;        // transposed condensed pattern (new order) and value slots
   size_t arena_chunk = 0;
   // factorisation plans: complex128 and complex64 of the general path, then of the
@@ -171,6 +194,10 @@ struct Handle {
 // ---------------------------------------------------------------- kernels
 // assemble.cu
 int launch_assemble(Handle &h, int which);  // which 0: K+M, 1: D
+int mesh_device(Handle &h);                 // h.mesh's copies of the mesh
+struct PmlDev;
+int material_device(Handle &h, int which, PmlDev &pml);   // h.mesh's copies of the materials and the PML
+cudaError_t element_scratch(Handle &h, DBuf &own, size_t bytes, cplx<double> *&p);
 // numeric.cu
 int launch_condense(Handle &h);
 int gather_values(Handle &h);   // condensed values again after a value-only reassembly
