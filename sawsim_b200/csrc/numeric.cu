@@ -338,46 +338,60 @@ __device__ __forceinline__ void st_el(cplx<T> *p, cplx<T> v) {
   *reinterpret_cast<typename VecOf<T>::V *>(p) = w;
 }
 // Entry of a pivot block from its sources: (i0, j0) are its row and column in source 0
-// and (i1, j1) in source 1, negative where a source does not have it.  `at` receives the
-// element offset of the first source that has it (the return value tells whether one
-// does) and `both` whether the second one has it too.  The offset is selected, not the
-// loaded value, so a batch of entries costs one round trip to memory.
-__device__ __forceinline__ bool sym_pick(const SymFront &s, int i0, int j0, int i1, int j1, int64_t &at, bool &both) {
-  const bool h0 = (i0 | j0) >= 0, h1 = (i1 | j1) >= 0;
-  at = h0 ? s.cb[0] + (int64_t)i0 * s.cld[0] + j0 : s.cb[1] + (int64_t)i1 * s.cld[1] + j1;
-  both = h0 && h1;
-  return h0 || h1;
+// and (i1, j1) in source 1, negative where a source does not have it.  Both loads are
+// issued at once; add them (v0 + v1) when the whole batch has been issued.
+template <class T>
+__device__ __forceinline__ void sym_pick(const SymFront &s, const cplx<T> *arena, bool in, int i0, int j0, int i1, int j1,
+                                         cplx<T> &v0, cplx<T> &v1) {
+  v0 = in && (i0 | j0) >= 0 ? ld_once(arena + s.cb[0] + (int64_t)i0 * s.cld[0] + j0) : cplx<T>{0, 0};
+  v1 = in && (i1 | j1) >= 0 ? ld_once(arena + s.cb[1] + (int64_t)i1 * s.cld[1] + j1) : cplx<T>{0, 0};
 }
-// Arrowhead entries [a0, a1) of a tile added at add(position, value): four per thread and
-// round, the positions and slots, then the values, then the sums.
-template <class T, class Add>
-__device__ __forceinline__ void add_arrows(const FrontArgs<T> &a, int a0, int a1, const uint16_t *__restrict__ apos,
-                                           const int *__restrict__ aslot, double om, Add add) {
-  constexpr int U = 4;
-  const double w2 = om * om;
-  for (int q0 = a0 + threadIdx.x; q0 < a1; q0 += U * blockDim.x) {
-    int pos[U], slot[U];
-    cd kv[U], mv[U];
+// Arrowhead entries of a tile, U per thread and round, in three parts so that a kernel
+// can put other loads between them: the positions and slots, then the matrices' entries,
+// then the sums at add(position, value).
+template <class T, int U>
+struct Arrows {
+  int pos[U], slot[U];
+  cd kv[U], mv[U];
+  __device__ __forceinline__ void index(int q0, int q1, const uint16_t *__restrict__ apos, const int *__restrict__ aslot) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int q = q0 + u * blockDim.x;
-      pos[u] = q < a1 ? apos[q] : -1;
-      slot[u] = q < a1 ? aslot[q] : 0;
+      const int q = q0 + threadIdx.x + u * blockDim.x;
+      pos[u] = q < q1 ? apos[q] : -1;
+      slot[u] = q < q1 ? aslot[q] : 0;
     }
+  }
+  __device__ __forceinline__ void load(const FrontArgs<T> &a) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      kv[u] = ld_el(a.Kc + slot[u]);
-      mv[u] = ld_el(a.Mc + slot[u]);
+      kv[u] = pos[u] >= 0 ? ld_el(a.Kc + slot[u]) : cd{0.0, 0.0};
+      mv[u] = pos[u] >= 0 ? ld_el(a.Mc + slot[u]) : cd{0.0, 0.0};
     }
+  }
+  template <class Add>
+  __device__ __forceinline__ void add(const FrontArgs<T> &a, double om, Add use) const {
+    const double w2 = om * om;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (pos[u] < 0) continue;
       cd v = kv[u] - mv[u] * w2;
       if (a.Dc) v = v + cmul(cd{0.0, om * a.beta}, a.Dc[slot[u]]);
-      add(pos[u], to_t<T>(v));
+      use(pos[u], to_t<T>(v));
     }
   }
-}
+  // this first round's sums and the entries past it
+  template <class Add>
+  __device__ __forceinline__ void add_all(const FrontArgs<T> &a, int q0, int q1, const uint16_t *__restrict__ apos,
+                                          const int *__restrict__ aslot, double om, Add use) {
+    for (;;) {
+      add(a, om, use);
+      q0 += U * blockDim.x;
+      if (q0 >= q1) break;
+      index(q0, q1, apos, aslot);
+      load(a);
+    }
+  }
+};
 // C tile of a symmetric Schur update (rows tk.r0.., columns tk.c0..) copied into shared
 // memory (row stride CS) by cp.async, each entry on or above the diagonal from the one
 // source that has it (zeros elsewhere); ir and ic receive the tile's source rows and

@@ -170,8 +170,8 @@ __global__ void __launch_bounds__(128, 3)
 // ------------------------------------------------------------------ pivot blocks
 // A pivot block takes two kernels (and the Schur update) instead of the assembly, panel
 // LU, row-swap, L21, U12 and panel-GEMM launches of every 32-pivot step:
-//  * sym_pivot_kernel assembles F11 in shared memory, factors it with a row in two
-//    threads' registers and writes it in pivot order, its 16 x 16 diagonal blocks as
+//  * sym_pivot_kernel assembles F11 in shared memory, factors it there four pivots at a
+//    time (block_lu) and writes it in pivot order, its 16 x 16 diagonal blocks as
 //    inverses (of the unit lower and of the upper triangle, in their places): the panel
 //    kernel and the solves multiply by them instead of substituting;
 //  * sym_panel_kernel takes one chunk of columns of F12: it assembles the chunk in shared
@@ -191,118 +191,281 @@ struct NarrowTask {
   int f, c0, a0, a1;
 };
 __host__ __device__ constexpr int pivot_class(int k) { return k <= 16 ? 16 : k <= 32 ? 32 : k <= 48 ? 48 : 64; }
+__host__ __device__ constexpr int pivot_ks(int k) { return (k + 3) / 4 * 4 + 1; }   // odd: columns without conflicts
 template <class T>
 __host__ __device__ constexpr size_t pivot_smem(int k) {
-  return (size_t)k * (k + 1) * sizeof(cplx<T>) + (size_t)2 * k * sizeof(int);
+  return (size_t)k * pivot_ks(k) * sizeof(cplx<T>) + (size_t)2 * k * sizeof(int);
 }
 
-// 1 / z without overflow or underflow in the squares
-template <class T>
-__device__ __forceinline__ cplx<T> crecip(cplx<T> z) {
-  const T r = (T)1 / fmax(fabs(z.x), fabs(z.y));
-  const T x = z.x * r, y = z.y * r, g = r / (x * x + y * y);
-  return {x * g, -y * g};
-}
-// magnitude of a pivot candidate as an ordered integer, its low 7 bits replaced by the
-// row (the lowest row wins among magnitudes equal to about 2^-13)
+// magnitude |x| + |y| of a pivot candidate as an ordered integer, its low 7 bits replaced by
+// the row (the lowest row wins among magnitudes equal to about 2^-13)
 __device__ __forceinline__ unsigned pivot_key(double v, int r) {
   return ((unsigned)__double2hiint(v) & ~127u) | (unsigned)(127 - r);
 }
 __device__ __forceinline__ unsigned pivot_key(float v, int r) {
   return (__float_as_uint(v) & ~127u) | (unsigned)(127 - r);
 }
+// l = v / z for a pivot z with its key: conj(z) v times 1 / |z|^2, z scaled by the power of
+// two that brings |x| + |y| into [1, 2), so no square over- or underflows.  In FP64 the
+// reciprocal of |z|^2 comes from the hardware's approximation (about 2^-20) by one Halley
+// iteration (cubic: 2^-60).
+struct PivotRecip {
+  cd z;          // conj(scaled pivot)
+  double g;      // scale / |scaled pivot|^2
+  __device__ __forceinline__ PivotRecip(cd p, unsigned key) {
+    const double r = __hiloint2double(min(max(2046 - (int)(key >> 20), 1), 2045) << 20, 0);
+    z = cd{p.x * r, -p.y * r};
+    const double d = z.x * z.x + z.y * z.y;
+    double q;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(q) : "d"(d));
+    const double h = fma(-d, q, 1.0);
+    g = fma(q, fma(h, h, h), q) * r;
+  }
+  __device__ __forceinline__ cd recip() const { return cd{z.x * g, z.y * g}; }
+  __device__ __forceinline__ cd times(cd v) const {
+    const cd t = cmul(v, z);     // beside the reciprocal's chain
+    return cd{t.x * g, t.y * g};
+  }
+};
+struct PivotRecipF {
+  cf z;
+  float g;
+  __device__ __forceinline__ PivotRecipF(cf p, unsigned key) {
+    const float r = __uint_as_float(min(max(254 - (int)(key >> 23), 1), 253) << 23);
+    z = cf{p.x * r, -p.y * r};
+    g = __frcp_rn(z.x * z.x + z.y * z.y) * r;
+  }
+  __device__ __forceinline__ cf recip() const { return cf{z.x * g, z.y * g}; }
+  __device__ __forceinline__ cf times(cf v) const {
+    const cf t = cmul(v, z);
+    return cf{t.x * g, t.y * g};
+  }
+};
+
+// A warp's 16 columns (from c0) of the block that block_lu factors, in registers: in
+// complex128 as accumulators of the FP64 tensor cores, in complex64 a row (KMAX > 32: two
+// rows) per lane.
+template <class T, int KMAX> struct LuTile;
+template <int KMAX> struct LuTile<double, KMAX> {
+  static constexpr int RB = KMAX / 8;
+  double cr[RB][2][2], ci[RB][2][2];
+  int g, t;
+  __device__ __forceinline__ void load(const cd *W, int ks, int k, int c0) {
+    g = (threadIdx.x & 31) >> 2;
+    t = threadIdx.x & 3;
+#pragma unroll
+    for (int i = 0; i < RB; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int r = 8 * i + g, c = c0 + 8 * j + 2 * t + e;
+          const cd z = r < k && c < k ? W[r * ks + c] : cd{0.0, 0.0};
+          cr[i][j][e] = z.x;
+          ci[i][j][e] = z.y;
+        }
+  }
+  // the columns [lo, hi) of the rows in the mask to W
+  __device__ __forceinline__ void put(cd *W, int ks, int c0, unsigned long long rows, int lo, int hi) const {
+    rows >>= g;
+    cd *Wg = W + g * ks + c0 + 2 * t;
+    bool in[2][2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int c = c0 + 8 * j + 2 * t + e;
+        in[j][e] = c >= lo && c < hi;
+      }
+#pragma unroll
+    for (int i = 0; i < RB; ++i)
+      if (rows >> (8 * i) & 1) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            if (in[j][e]) Wg[8 * i * ks + 8 * j + e] = cd{cr[i][j][e], ci[i][j][e]};
+      }
+  }
+  // open rows -= (columns j0 .. j0 + 3 of W) (rows perm[j0 + s] of W), columns >= j0 + 4
+  __device__ __forceinline__ void update(const cd *W, int ks, int k, int c0, int j0, const int *perm,
+                                         unsigned long long open) {
+    const cd *Wb = W + perm[j0 + t] * ks, *Wa = W + g * ks + j0 + t;
+    open >>= g;
+    cd b[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) b[j] = Wb[min(c0 + 8 * j + g, ks - 1)];
+#pragma unroll
+    for (int i = 0; i < RB; ++i) {
+      if (8 * i >= k) break;
+      const cd a = open >> (8 * i) & 1 ? Wa[8 * i * ks] : cd{0.0, 0.0};
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        if (c0 + 8 * j + 8 <= j0 + 4) continue;
+        dmma(cr[i][j][0], cr[i][j][1], -a.x, b[j].x);
+        dmma(ci[i][j][0], ci[i][j][1], -a.x, b[j].y);
+        dmma(cr[i][j][0], cr[i][j][1], a.y, b[j].y);
+        dmma(ci[i][j][0], ci[i][j][1], -a.y, b[j].x);
+      }
+    }
+  }
+};
+template <int KMAX> struct LuTile<float, KMAX> {
+  static constexpr int R = KMAX > 32 ? 2 : 1;
+  cf v[R][16];
+  int lane;
+  __device__ __forceinline__ void load(const cf *W, int ks, int k, int c0) {
+    lane = threadIdx.x & 31;
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+      for (int c = 0; c < 16; ++c)
+        v[i][c] = lane + 32 * i < k && c0 + c < k ? W[(lane + 32 * i) * ks + c0 + c] : cf{0.f, 0.f};
+  }
+  __device__ __forceinline__ void put(cf *W, int ks, int c0, unsigned long long rows, int lo, int hi) const {
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+      if (rows >> (lane + 32 * i) & 1) {
+#pragma unroll
+        for (int c = 0; c < 16; ++c)
+          if (c0 + c >= lo && c0 + c < hi) W[(lane + 32 * i) * ks + c0 + c] = v[i][c];
+      }
+  }
+  __device__ __forceinline__ void update(const cf *W, int ks, int k, int c0, int j0, const int *perm,
+                                         unsigned long long open) {
+    cf l[R][4];
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+      for (int s = 0; s < 4; ++s)
+        l[i][s] = open >> (lane + 32 * i) & 1 ? W[(lane + 32 * i) * ks + j0 + s] : cf{0.f, 0.f};
+    const cf *Wc[4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) Wc[s] = W + perm[j0 + s] * ks + c0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (c0 + 4 * q < j0 + 4 || c0 + 4 * q >= k) continue;
+#pragma unroll
+      for (int c = 4 * q; c < 4 * q + 4; ++c)
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+          const cf u = Wc[s][c];
+#pragma unroll
+          for (int i = 0; i < R; ++i) v[i][c] = cfms(v[i][c], l[i][s], u);
+        }
+    }
+  }
+};
 
 // LU of the k x k matrix W (row stride ks, shared memory; k <= KMAX) in place with
-// implicit row interchanges, by 2 KMAX threads: thread (r, h) holds the entries of row r
-// in columns 2 i + h, i counted from the current column pair (the registers shift down
-// once per pair), in registers.  Per pivot: the warps' candidate keys (one integer
-// reduction each) give the row; its two threads write it to W (it is final) with the
-// pivot's reciprocal; every open row takes its multiplier and updates its registers, so
-// shared memory carries one row per pivot instead of the whole trailing matrix.  The
-// register loop shrinks in four steps.  On return W holds the multipliers and U rows in
+// implicit row interchanges, by KMAX / 16 warps with 16 columns each in registers.  Four
+// columns at a time: their warp puts them into W, eliminates them with a row in each lane's
+// registers (the pivot by one integer reduction of candidate keys) and leaves the
+// multipliers there; then every warp with columns left takes its entries of the four pivot
+// rows through a 4 x 4 triangle and subtracts the rank-4 product.  One barrier per four
+// pivots, and a pivot's chain is one warp's; the next four columns start as soon as their
+// own warp has applied the last ones.
+//   Bound by the chain of a pivot (about 18 dependent FP64 operations of some 20 cycles,
+// one reduction, two trips through shared memory: 1100 cycles).  12 launches of one to ten
+// 48-pivot blocks (16x64 ME0, one point): 0.59 ms, against 0.69 with two threads per row and
+// a block-wide step per pivot; the 89 wide complex64 launches of the 12x4x48 slab: 4.0
+// against 6.1 ms.  On return W holds the multipliers and U rows in
 // the original row order, perm[j] the row of pivot j and dinv[j] the reciprocal pivots.
-// (One CTA, k = 64, complex128: 153 us with the trailing matrix in shared memory.)
 template <class T, int KMAX>
 __device__ __forceinline__ int block_lu(cplx<T> *W, int ks, int k, T tiny, int *perm, cplx<T> *dinv) {
-  constexpr int W2 = KMAX / 2, NW = KMAX / 16;
-  __shared__ unsigned s_key[2][NW];
-  const int tid = threadIdx.x, r = tid >> 1, h = tid & 1, lane = tid & 31, wid = tid >> 5;
-  cplx<T> v[W2];
-#pragma unroll
-  for (int i = 0; i < W2; ++i) {
-    const int c = 2 * i + h;
-    v[i] = r < k && c < k ? W[r * ks + c] : cplx<T>{0, 0};
-  }
-  bool open = r < k;
+  constexpr int R = KMAX > 32 ? 2 : 1;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, c0 = 16 * wid;
+  LuTile<T, KMAX> tile;
+  tile.load(W, ks, k, c0);
+  unsigned long long open = k < 64 ? (1ull << k) - 1 : ~0ull;     // rows without a pivot
   int npert = 0;
-  auto candidate = [&](int par, int hown) {
-    unsigned key = open && h == hown ? pivot_key(cabs1(v[0]), r) : 0u;
-    key = __reduce_max_sync(0xffffffffu, key);
-    if (lane == 0) s_key[par][wid] = key;
-  };
-  candidate(0, 0);
-  // one pivot step: HOWN = parity of column j; WC registers may be nonzero
-  auto step = [&](int j, auto hown_c, auto wc_c) {
-    constexpr int HOWN = decltype(hown_c)::value, WC = decltype(wc_c)::value;
-    __syncthreads();
-    unsigned key = s_key[HOWN][0];
+  for (int j0 = 0; j0 < k; j0 += 4) {
+    if (wid == j0 >> 4) {
+      tile.put(W, ks, c0, open, j0, j0 + 4);
+      __syncwarp();
+      cplx<T> v[R][4];
+      bool op[R];
 #pragma unroll
-    for (int q = 1; q < NW; ++q) key = max(key, s_key[HOWN][q]);
-    const int p = 127 - (int)(key & 127u);
-    cplx<T> *Wp = W + p * ks;
-    if (r == p) {
-      if (h == HOWN) {
-        cplx<T> pv = v[0];
-        if (cabs1(pv) < tiny) {
-          pv = cplx<T>{tiny, (T)0};
-          npert = npert + 1;
+      for (int i = 0; i < R; ++i) {
+        const int r = lane + 32 * i;
+        op[i] = open >> r & 1;
+#pragma unroll
+        for (int s = 0; s < 4; ++s) v[i][s] = op[i] ? W[r * ks + j0 + s] : cplx<T>{0, 0};
+      }
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        if (j0 + s >= k) break;
+        unsigned key = 0u;
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+          if (op[i]) key = max(key, pivot_key(cabs1(v[i][s]), lane + 32 * i));
+        key = __reduce_max_sync(0xffffffffu, key);
+        const int p = 127 - (int)(key & 127u);
+        cplx<T> *Wp = W + p * ks + j0;
+        if ((key | 127u) <= (pivot_key(tiny, 0) | 127u)) {      // at most about tiny
+#pragma unroll
+          for (int i = 0; i < R; ++i)
+            if (p == lane + 32 * i && cabs1(v[i][s]) < tiny) {
+              v[i][s] = cplx<T>{tiny, (T)0};
+              ++npert;
+            }
+          key = pivot_key(tiny, 0);
         }
-        Wp[j] = pv;
-        dinv[j] = crecip(pv);
-        perm[j] = p;
-      }
 #pragma unroll
-      for (int i = 0; i < WC; ++i) {
-        const int c = j - HOWN + 2 * i + h;
-        if (c > j && c < k) Wp[c] = v[i];
+        for (int i = 0; i < R; ++i)
+          if (p == lane + 32 * i) {
+#pragma unroll
+            for (int c = s; c < 4; ++c) Wp[c] = v[i][c];
+            perm[j0 + s] = p;
+            op[i] = false;
+          }
+        __syncwarp();
+        const std::conditional_t<sizeof(T) == 8, PivotRecip, PivotRecipF> rec(Wp[s], key);
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+          const cplx<T> l = rec.times(v[i][s]);
+          if (!op[i]) continue;
+          W[(lane + 32 * i) * ks + j0 + s] = l;
+#pragma unroll
+          for (int c = s + 1; c < 4; ++c) v[i][c] = cfms(v[i][c], l, Wp[c]);
+        }
+        if (lane == 0) dinv[j0 + s] = rec.recip();
       }
-      open = false;
     }
     __syncthreads();
-    const T ox = __shfl_xor_sync(0xffffffffu, v[0].x, 1), oy = __shfl_xor_sync(0xffffffffu, v[0].y, 1);
-    const cplx<T> vj = h == HOWN ? v[0] : cplx<T>{ox, oy};
-    cplx<T> l = cmul(vj, dinv[j]);
-    if (!open) l = cplx<T>{0, 0};
-    if (open && h == 0) W[r * ks + j] = l;
+    if (j0 + 4 >= k) break;
+    int p[4];
+    unsigned long long taken = 0;
 #pragma unroll
-    for (int i = 0; i < WC; ++i) {
-      const int c = j - HOWN + 2 * i + h;
-      const cplx<T> q = c > j && c < k ? Wp[c] : cplx<T>{0, 0};
-      const cplx<T> x = cfms(v[i], l, q);
-      if (HOWN == 0)
-        v[i] = x;
-      else if (i > 0)
-        v[i - 1] = x;      // the column pair is done: shift
+    for (int s = 0; s < 4; ++s) {
+      p[s] = perm[j0 + s];
+      taken |= 1ull << p[s];
     }
-    if (HOWN == 1) v[WC - 1] = cplx<T>{0, 0};
-    candidate(HOWN ^ 1, HOWN ^ 1);
-  };
-  using std::integral_constant;
-  auto pair = [&](int j, auto wc) {
-    step(j, integral_constant<int, 0>{}, wc);
-    if (j + 1 < k) step(j + 1, integral_constant<int, 1>{}, wc);
-  };
-  int j = 0;
-  for (; j < k && k - j > 2 * (3 * W2 / 4); j += 2) pair(j, integral_constant<int, W2>{});
-  for (; j < k && k - j > 2 * (W2 / 2); j += 2) pair(j, integral_constant<int, 3 * W2 / 4>{});
-  for (; j < k && k - j > 2 * (W2 / 4); j += 2) pair(j, integral_constant<int, W2 / 2>{});
-  for (; j < k; j += 2) pair(j, integral_constant<int, W2 / 4>{});
-  __syncthreads();
+    open &= ~taken;
+    if (c0 >= k || c0 + 16 <= j0 + 4) continue;
+    // the warp's columns of the pivot rows
+    tile.put(W, ks, c0, taken, j0 + 4, ks - 1);
+    __syncwarp();
+    const int c = c0 + lane;
+    if (lane < 16 && c >= j0 + 4 && c < ks - 1) {
+      cplx<T> u[4];
+#pragma unroll
+      for (int s = 0; s < 4; ++s) u[s] = W[p[s] * ks + c];
+#pragma unroll
+      for (int s = 1; s < 4; ++s) {
+#pragma unroll
+        for (int q = 0; q < s; ++q) u[s] = cfms(u[s], W[p[s] * ks + j0 + q], u[q]);
+        W[p[s] * ks + c] = u[s];
+      }
+    }
+    __syncwarp();
+    tile.update(W, ks, k, c0, j0, perm, open);
+  }
   return npert;
 }
 
 template <class T, int KMAX>
-__global__ void __launch_bounds__(2 * KMAX)
+__global__ void __launch_bounds__(2 * KMAX, KMAX == 64 ? 3 : KMAX == 48 ? 4 : KMAX == 32 ? 8 : 12)
     sym_pivot_kernel(FrontArgs<T> a, const NarrowTask *__restrict__ tasks, int nb, const uint16_t *__restrict__ apos,
                      const int *__restrict__ aslot) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -312,51 +475,50 @@ __global__ void __launch_bounds__(2 * KMAX)
   const NarrowTask tk = tasks[blockIdx.x / nb];
   const int fq = blockIdx.x % nb;
   const SymFront &s = a.sf[tk.f];
-  const int k = s.k, ks = k + 1;
+  const int k = s.k, ks = pivot_ks(k);
   cplx<T> *W = reinterpret_cast<cplx<T> *>(smem_raw);
   int *ir = reinterpret_cast<int *>(W + k * ks);
   cplx<T> *arena = a.arena + (int64_t)fq * a.stride;
   const double om = a.omega[fq];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int nch = s.nch;
+  // a load is a round trip of 1000 to 2000 cycles here: few of them in a row, many at once
+  Arrows<T, 2> arrows;
+  arrows.index(tk.a0, tk.a1, apos, aslot);
   if (nch) {
     for (int i = tid; i < k; i += NT) {
       ir[i] = a.imap[s.imap[0] + i];
       ir[k + i] = nch > 1 ? a.imap[s.imap[1] + i] : -1;
     }
+    arrows.load(a);
     __syncthreads();
-    // the sources' upper entries, mirrored: four rows of 32 columns in flight per warp
-    constexpr int U = 4;
+    // the sources' upper entries, mirrored: eight rows of 32 columns in flight per warp
+    constexpr int U = 8;
     for (int cb = 0; cb < k; cb += 32)
       for (int rb = wid; rb < min(k, cb + 32); rb += U * NW) {
-        const int c = cb + lane;
-        cplx<T> v[U];
-        bool both[U];
+        const int c = cb + lane, cc = min(c, k - 1);
+        cplx<T> v0[U], v1[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-          const int r = rb + u * NW;
-          const bool in = r < k && c < k && c >= r;
-          int64_t at;
-          const bool has = in && sym_pick(s, ir[min(r, k - 1)], ir[min(c, k - 1)], ir[k + min(r, k - 1)],
-                                          ir[k + min(c, k - 1)], at, both[u]);
-          v[u] = has ? ld_once(arena + at) : cplx<T>{0, 0};
-          both[u] = has && both[u];
+          const int r = rb + u * NW, rr = min(r, k - 1);
+          sym_pick<T>(s, arena, r < k && c < k && c >= r, ir[rr], ir[cc], ir[k + rr], ir[k + cc], v0[u], v1[u]);
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           const int r = rb + u * NW;
-          if (both[u]) v[u] = v[u] + ld_once(arena + s.cb[1] + (int64_t)ir[k + r] * s.cld[1] + ir[k + c]);
           if (r < k && c < k && c >= r) {
-            W[r * ks + c] = v[u];
-            W[c * ks + r] = v[u];
+            const cplx<T> v = v0[u] + v1[u];
+            W[r * ks + c] = v;
+            W[c * ks + r] = v;
           }
         }
       }
   } else {
+    arrows.load(a);
     for (int t = tid; t < k * ks; t += NT) W[t] = cplx<T>{0, 0};
   }
   __syncthreads();
-  add_arrows(a, tk.a0, tk.a1, apos, aslot, om, [&](int p, cplx<T> e) {
+  arrows.add_all(a, tk.a0, tk.a1, apos, aslot, om, [&](int p, cplx<T> e) {
     const int r = p >> 6, c = p & 63;
     const cplx<T> v = W[r * ks + c] + e;
     W[r * ks + c] = v;
@@ -374,35 +536,25 @@ __global__ void __launch_bounds__(2 * KMAX)
   }
   for (int i = tid; i < k; i += NT) a.piv[(int64_t)fq * a.n + s.p0 + i] = perm[i];
   // inverses of the diagonal blocks, one block per warp: lanes 0-15 a column of the
-  // inverted unit lower triangle each, lanes 16-31 of the inverted upper triangle
+  // inverted unit lower triangle each, lanes 16-31 of the inverted upper triangle with its
+  // rows and columns in reverse order, so that both halves run the same substitution
   const int h0 = kDiagB * wid, hw = min(kDiagB, k - h0);
   if (hw <= 0) return;
-  const int col = lane & 15;
+  const bool upper = lane >= 16;
+  const int col = lane & 15;                   // the column, counted as the rows are
+  const int first = h0 + (upper ? hw - 1 : 0), dir = upper ? -1 : 1;
   cplx<T> x[kDiagB];
-  if (lane < 16) {
 #pragma unroll
-    for (int i = 0; i < kDiagB; ++i) {
-      cplx<T> t{i == col ? (T)1 : (T)0, (T)0};
-      const cplx<T> *row = W + perm[h0 + min(i, hw - 1)] * ks + h0;
+  for (int i = 0; i < kDiagB; ++i) x[i] = cplx<T>{i == col ? (T)1 : (T)0, (T)0};
 #pragma unroll
-      for (int q = 0; q < i; ++q) t = cfms(t, row[q], x[q]);
-      x[i] = t;
-      if (i > col && i < hw && col < hw) st_el(F + (int64_t)(h0 + i) * ld + h0 + col, t);
-    }
-  } else {
+  for (int q = 0; q < kDiagB; ++q) {
+    if (q >= hw) break;
+    const int r = first + dir * q;
+    if (upper) x[q] = cmul(x[q], dinv[r]);
+    if ((upper ? q >= col : q > col) && col < hw) st_el(F + (int64_t)r * ld + first + dir * col, x[q]);
 #pragma unroll
-    for (int i = kDiagB - 1; i >= 0; --i) {
-      cplx<T> t{i == col ? (T)1 : (T)0, (T)0};
-      if (i < hw) {
-        const cplx<T> *row = W + perm[h0 + i] * ks + h0;
-#pragma unroll
-        for (int q = i + 1; q < kDiagB; ++q)
-          if (q < hw) t = cfms(t, row[q], x[q]);
-        t = cmul(t, dinv[h0 + i]);
-        if (i <= col && col < hw) st_el(F + (int64_t)(h0 + i) * ld + h0 + col, t);
-      }
-      x[i] = t;
-    }
+    for (int i = q + 1; i < kDiagB; ++i)
+      if (i < hw) x[i] = cfms(x[i], W[perm[first + dir * i] * ks + r], x[q]);
   }
 }
 
@@ -596,31 +748,27 @@ __global__ void __launch_bounds__(kPanelColThreads, sizeof(T) == 8 ? 3 : 4)
   const double om = a.omega[fq];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int nch = s.nch;
+  Arrows<T, 2> arrows;
   {
     const int64_t m0 = s.imap[0], m1 = s.imap[1];
     int j0[NH], j1[NH];
+    arrows.index(tk.a0, tk.a1, apos, aslot);
 #pragma unroll
     for (int h = 0; h < NH; ++h) {
       const int c = lane + 32 * h;
       j0[h] = nch > 0 && c < nc ? a.imap[m0 + k + tk.c0 + c] : -1;
       j1[h] = nch > 1 && c < nc ? a.imap[m1 + k + tk.c0 + c] : -1;
     }
+    arrows.load(a);
     constexpr int U = 4;
     for (int rb = wid; rb < kp; rb += U * NW) {
-      cplx<T> v[U][NH], d[U][2];
-      bool both[U][NH];
-      int i1[U];
+      cplx<T> v0[U][NH], v1[U][NH], d[U][2];
+      int i0[U], i1[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int r = rb + u * NW;
-        const int i0 = nch > 0 && r < k ? a.imap[m0 + r] : -1;
+        i0[u] = nch > 0 && r < k ? a.imap[m0 + r] : -1;
         i1[u] = nch > 1 && r < k ? a.imap[m1 + r] : -1;
-#pragma unroll
-        for (int h = 0; h < NH; ++h) {
-          int64_t at;
-          const bool has = sym_pick(s, i0, j0[h], i1[u], j1[h], at, both[u][h]);
-          v[u][h] = has ? ld_once(arena + at) : cplx<T>{0, 0};
-        }
         // F11 (at most 64 columns; the padding is zero)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -629,14 +777,15 @@ __global__ void __launch_bounds__(kPanelColThreads, sizeof(T) == 8 ? 3 : 4)
         }
       }
 #pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int h = 0; h < NH; ++h) sym_pick<T>(s, arena, true, i0[u], j0[h], i1[u], j1[h], v0[u][h], v1[u][h]);
+#pragma unroll
       for (int u = 0; u < U; ++u) {
         const int r = rb + u * NW;
         if (r >= kp) break;
 #pragma unroll
-        for (int h = 0; h < NH; ++h) {
-          if (both[u][h]) v[u][h] = v[u][h] + ld_once(arena + s.cb[1] + (int64_t)i1[u] * s.cld[1] + j1[h]);
-          Y[r * CS + lane + 32 * h] = v[u][h];
-        }
+        for (int h = 0; h < NH; ++h) Y[r * CS + lane + 32 * h] = v0[u][h] + v1[u][h];
 #pragma unroll
         for (int h = 0; h < 2; ++h)
           if (lane + 32 * h < ks) A[r * ks + lane + 32 * h] = d[u][h];
@@ -646,7 +795,7 @@ __global__ void __launch_bounds__(kPanelColThreads, sizeof(T) == 8 ? 3 : 4)
     for (int i = tid; i < k; i += kPanelColThreads) perm[i] = a.piv[(int64_t)fq * a.n + s.p0 + i];
   }
   __syncthreads();
-  add_arrows(a, tk.a0, tk.a1, apos, aslot, om, [&](int p, cplx<T> e) {
+  arrows.add_all(a, tk.a0, tk.a1, apos, aslot, om, [&](int p, cplx<T> e) {
     cplx<T> *d = Y + (p >> 6) * CS + (p & 63);
     *d = *d + e;
   });
