@@ -249,7 +249,8 @@ int ss_adjoint_gradient(ss_handle *h, int n_f, const double *omega, double V, in
  *  beside the DMMA tiles; 0 when the autotuner kept them in DMMA tiles), 38 1 when
  *  the scaled system is complex symmetric and its fronts took the symmetric path
  *  (only the upper triangle of every update block is formed; 12 then counts the
- *  symmetric update).
+ *  symmetric update, and 11 adds up the launches' own times, which they share with
+ *  other frequencies' kernels: up to three groups of a chunk's frequencies run at once).
  *  Slots past 38 read 0.
  */
 int ss_stats(const ss_handle *h, double *out, int n);

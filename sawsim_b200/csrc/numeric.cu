@@ -1944,12 +1944,17 @@ struct Plan {
   std::vector<SymFront> sf;
   std::vector<int> wide, wide_ptr;         // fronts of more than one pivot block, by level
   int sym_nev = 0;                         // timed Schur updates of one factorisation
+  // streams of the second and further groups of frequencies (Sweeper::branched)
+  std::vector<cudaStream_t> side;
+  std::vector<cudaEvent_t> side_ev;        // fork, then one join per side stream
   DBuf d_npiv[4], d_npan[2], d_apos, d_aslot, d_imap, d_sf, d_wide, d_soff, d_sld, d_sk, d_sm;
   CUtensorMap tmap{};                      // 2D map over the staging buffer (128-byte rows)
   ~Plan() {
     for (auto &g : graphs)
       if (g.exec) cudaGraphExecDestroy(g.exec);
     for (auto &e : ev) cudaEventDestroy(e);
+    for (auto &e : side_ev) cudaEventDestroy(e);
+    for (auto &st : side) cudaStreamDestroy(st);
   }
 };
 
@@ -2609,6 +2614,13 @@ static int equilibrate(Handle &h, double w) {
   return SS_OK;
 }
 
+// Groups of frequencies that run beside each other on the symmetric path: a level's pivot
+// blocks and its triangular solves wait for memory and for chains of dependent operations
+// with most of the GPU's issue slots free, its Schur updates fill them.  One, two, three
+// and four groups, milliseconds per pass: 64x256 ME1 (11 points) 77.3, 75.3, 75.3, 75.8;
+// 32x128 (51 points) 59.2, -, 57.8, 57.8; device time with one and three groups: 16x64 ME0
+// (101 points) 13.7, 13.2; lossy stack (51) 11.3, 10.8; 12x4x48 mixed (6) 60.1, 58.2.
+constexpr int kBranches = 3;
 template <class T>
 struct Sweeper {
   static constexpr size_t kDiagBytes = (size_t)kDiagElems * sizeof(cplx<T>);
@@ -2633,7 +2645,7 @@ struct Sweeper {
   explicit Sweeper(Handle &hh, Plan &pp) : h(hh), P(pp), ev(pp.ev) {
     pivb = ((size_t)std::max(1, h.sym.max_k) * sizeof(int) + 15) / 16 * 16;
     if (ev.empty()) {
-      ev.resize(2 * std::max(1, P.sym ? P.level_slot.back() : h.sym.nlevel));
+      ev.resize(2 * std::max(1, P.sym ? kBranches * P.level_slot.back() : h.sym.nlevel));
       // recorded once outside any capture: the graphs' event-record nodes then
       // re-record them at every replay and their elapsed times can be read
       for (auto &e : ev) {
@@ -2683,33 +2695,64 @@ struct Sweeper {
     SS_CK(cudaGraphLaunch(g.exec, h.stream));
     return SS_OK;
   }
+  // A group of a chunk's frequencies on the symmetric path and the stream that takes it.
+  struct Branch {
+    FrontArgs<T> a;
+    cudaStream_t st;
+    int f0, nb;
+  };
+  // The chunk's frequencies in up to kBranches groups that run beside each other: `body`
+  // (one group's whole launch chain) on h.stream and on the plan's side streams, forked
+  // from h.stream and joined to it again (also inside a capture).
+  template <class Body>
+  int branched(int nb, Body body) {
+    const int ng = std::min(nb, kBranches);
+    if (ng > 1) SS_CK(cudaEventRecord(P.side_ev[0], h.stream));
+    for (int g = 0; g < ng; ++g) {
+      Branch br{a, g ? P.side[g - 1] : h.stream, (int)((int64_t)nb * g / ng), 0};
+      br.nb = (int)((int64_t)nb * (g + 1) / ng) - br.f0;
+      br.a.arena += (int64_t)br.f0 * a.stride;
+      br.a.omega += br.f0;
+      br.a.piv += (int64_t)br.f0 * a.n;
+      br.a.nperturb += br.f0;
+      if (br.a.active) br.a.active += br.f0;
+      if (g) SS_CK(cudaStreamWaitEvent(br.st, P.side_ev[0], 0));
+      const int rc = body(br);
+      if (rc) return rc;
+      if (g) SS_CK(cudaEventRecord(P.side_ev[g], br.st));
+    }
+    for (int g = 1; g < ng; ++g) SS_CK(cudaStreamWaitEvent(h.stream, P.side_ev[g], 0));
+    return SS_OK;
+  }
   // Schur update of slot q on the symmetric path with candidate c (complex64: 0 / 1 TMA
   // tiles of 128 / 64 columns, 2 SIMT; complex128: one kernel)
-  void sym_schur(int q, int c, int nb) {
+  void sym_schur(const Branch &br, int q, int c) {
+    const FrontArgs<T> &a = br.a;
+    const int nb = br.nb;
     const int64_t t0 = P.schur_ptr[q], t1 = P.schur_ptr[q + 1];
     const GemmTask *tasks = P.d_tasks.template as<GemmTask>();
     const dim3 grid((unsigned)(t1 - t0), nb);
     if constexpr (sizeof(T) == 8) {
-      sym_schur_kernel<<<grid, 128, kSymSchurSmem, h.stream>>>(a, tasks + t0);
+      sym_schur_kernel<<<grid, 128, kSymSchurSmem, br.st>>>(a, tasks + t0);
     } else {
       if (c == 2 || !P.tma_ok || P.pk_ptr[q + 1] == P.pk_ptr[q]) {
         front_gemm_kernel<T, kSquare, false, true>
-            <<<grid, 256, gemm_cst_bytes<T, kSquare>(), h.stream>>>(a, tasks + t0);
+            <<<grid, 256, gemm_cst_bytes<T, kSquare>(), br.st>>>(a, tasks + t0);
         return;
       }
       const int64_t i0 = P.pi_ptr[q], i1 = P.pi_ptr[q + 1], q0 = P.tt_ptr[c][q], q1 = P.tt_ptr[c][q + 1];
       const int64_t *off = P.d_soff.template as<int64_t>();
       const int *ld = P.d_sld.template as<int>();
       cf *ar = reinterpret_cast<cf *>(a.arena);
-      tc::pack_kernel<<<dim3((unsigned)(i1 - i0), nb), tc::PACK_THREADS, 0, h.stream>>>(
+      tc::pack_kernel<<<dim3((unsigned)(i1 - i0), nb), tc::PACK_THREADS, 0, br.st>>>(
           ar, a.stride, off, ld, P.d_sk.template as<int>(), P.d_sm.template as<int>(),
-          P.d_pk.template as<tc::PackFront>(), P.d_pitems.template as<int2>() + i0, h.tc_stage.template as<float>(),
+          P.d_pk.template as<tc::PackFront>(), P.d_pitems.template as<int2>() + i0, h.tc_stage.template as<float>() + (int64_t)br.f0 * P.stage_rows * 32,
           P.stage_rows);
       const unsigned ctas = (unsigned)std::min<int64_t>((q1 - q0) * nb, h.num_sms);
       auto tma = [&](auto kernel, int threads, int smem) {
-        kernel<<<ctas, threads, smem, h.stream>>>(P.tmap, ar, a.stride, off, ld,
+        kernel<<<ctas, threads, smem, br.st>>>(P.tmap, ar, a.stride, off, ld,
                                                   P.d_tt[c].template as<tc::TmaTask>() + q0, (int)(q1 - q0), nb,
-                                                  P.stage_rows, tc_err, a.sf, a.imap);
+                                                  P.stage_rows, tc_err, a.sf, a.imap, br.f0);
       };
       if (c == 0)
         tma(tc::tma_gemm_kernel<128, 2, true>, tc::TmaCfg<128, 2>::THREADS, tc::TmaCfg<128, 2>::SMEM);
@@ -2731,7 +2774,7 @@ struct Sweeper {
       for (int q = 0; q < ns; ++q) {
         if (!has(q, c)) continue;
         cudaEventRecord(e[2 * (c * ns + q)], h.stream);
-        sym_schur(q, c, nb);
+        sym_schur(Branch{a, h.stream, 0, nb}, q, c);
         cudaEventRecord(e[2 * (c * ns + q) + 1], h.stream);
       }
     SS_CK(cudaGetLastError());
@@ -2751,45 +2794,49 @@ struct Sweeper {
     return SS_OK;
   }
   template <int KMAX>
-  void pivot_launch(int q, int nb) {
+  void pivot_launch(const Branch &br, int q) {
     constexpr int c = KMAX / 16 - 1;
     const int64_t t0 = P.npiv_ptr[c][q], t1 = P.npiv_ptr[c][q + 1];
     if (t1 == t0) return;
-    sym_pivot_kernel<T, KMAX><<<(unsigned)((t1 - t0) * nb), 2 * KMAX, pivot_smem<T>(P.slot_maxk[c][q]), h.stream>>>(
-        a, P.d_npiv[c].template as<NarrowTask>() + t0, nb, P.d_apos.template as<uint16_t>(), P.d_aslot.template as<int>());
+    sym_pivot_kernel<T, KMAX><<<(unsigned)((t1 - t0) * br.nb), 2 * KMAX, pivot_smem<T>(P.slot_maxk[c][q]), br.st>>>(
+        br.a, P.d_npiv[c].template as<NarrowTask>() + t0, br.nb, P.d_apos.template as<uint16_t>(), P.d_aslot.template as<int>());
     ++launches;
   }
   template <int CW>
-  void panel_launch(int q, int nb) {
+  void panel_launch(const Branch &br, int q) {
     constexpr int c = CW == 64 ? 0 : 1;
     const int64_t t0 = P.npan_ptr[c][q], t1 = P.npan_ptr[c][q + 1];
     if (t1 == t0) return;
     sym_panel_kernel<T, CW>
-        <<<(unsigned)((t1 - t0) * nb), kPanelColThreads, panel_smem<T>(P.slot_pank[c][q], CW), h.stream>>>(
-            a, P.d_npan[c].template as<NarrowTask>() + t0, nb, P.d_apos.template as<uint16_t>(),
+        <<<(unsigned)((t1 - t0) * br.nb), kPanelColThreads, panel_smem<T>(P.slot_pank[c][q], CW), br.st>>>(
+            br.a, P.d_npan[c].template as<NarrowTask>() + t0, br.nb, P.d_apos.template as<uint16_t>(),
             P.d_aslot.template as<int>());
     ++launches;
   }
   // the symmetric factorisation's launch sequence
   int sym_factor(int nb) {
     nev = 0;
+    const int rc = branched(nb, [&](const Branch &br) { return sym_factor_branch(br); });
+    P.sym_nev = nev;
+    return rc;
+  }
+  int sym_factor_branch(const Branch &br) {
     for (int l = 0; l < h.sym.nlevel; ++l)
       for (int q = P.level_slot[l]; q < P.level_slot[l + 1]; ++q) {
-        pivot_launch<16>(q, nb);
-        pivot_launch<32>(q, nb);
-        pivot_launch<48>(q, nb);
-        pivot_launch<64>(q, nb);
-        panel_launch<64>(q, nb);
-        if constexpr (sizeof(T) == 8) panel_launch<32>(q, nb);
+        pivot_launch<16>(br, q);
+        pivot_launch<32>(br, q);
+        pivot_launch<48>(br, q);
+        pivot_launch<64>(br, q);
+        panel_launch<64>(br, q);
+        if constexpr (sizeof(T) == 8) panel_launch<32>(br, q);
         if (P.schur_ptr[q + 1] == P.schur_ptr[q]) continue;
-        SS_CK(cudaEventRecordWithFlags(ev[2 * nev], h.stream, cudaEventRecordExternal));
-        sym_schur(q, P.pick[q], nb);
-        SS_CK(cudaEventRecordWithFlags(ev[2 * nev + 1], h.stream, cudaEventRecordExternal));
+        SS_CK(cudaEventRecordWithFlags(ev[2 * nev], br.st, cudaEventRecordExternal));
+        sym_schur(br, q, P.pick[q]);
+        SS_CK(cudaEventRecordWithFlags(ev[2 * nev + 1], br.st, cudaEventRecordExternal));
         ++nev;
         ++launches;
         ++schur_launches;
       }
-    P.sym_nev = nev;
     SS_CK(cudaGetLastError());
     return SS_OK;
   }
@@ -3194,6 +3241,13 @@ struct Sweeper {
 
   // the symmetric path's solve of A' x = b, which is also A'^T x = b
   int sym_solve(int nb, const cd *b, cd *x, cplx<T> *wv) {
+    return branched(nb, [&](const Branch &br) {
+      const int64_t o = (int64_t)br.f0 * h.sym.n;
+      return sym_solve_branch(br, b + o, x + o, wv + br.f0 * wstride);
+    });
+  }
+  int sym_solve_branch(const Branch &br, const cd *b, cd *x, cplx<T> *wv) {
+    const int nb = br.nb;
     const Symbolic &S = h.sym;
     const int *lf = h.d_level_fronts.as<int>(), *wide = P.d_wide.template as<int>();
     for (int pass = 0; pass < 2; ++pass)
@@ -3205,23 +3259,23 @@ struct Sweeper {
         const int maxb = mk <= kNarrowK ? sym_block(mk) : kNarrowK;
         const int bs = mk + mu <= 192 ? 128 : 256;
         const size_t sm = ((size_t)maxb * (maxb + 1) + mk + mu) * sizeof(cplx<T>);
-        FrontArgs<T> c = a, cw = a;
+        FrontArgs<T> c = br.a, cw = br.a;
         c.fronts = lf + S.level_ptr[l];
         cw.fronts = wide + P.wide_ptr[l];
         if (pass == 0) {
-          sym_fwd_kernel<T><<<dim3(nf, nb), bs, sm, h.stream>>>(c, b, x, wv, wstride, maxb);
+          sym_fwd_kernel<T><<<dim3(nf, nb), bs, sm, br.st>>>(c, b, x, wv, wstride, maxb);
           if (nw && mu > 0) {
             const unsigned z = (unsigned)((mu + kSolveRows - 1) / kSolveRows);
-            front_fwd_l21_kernel<T><<<dim3(nw, nb, z), 256, mk * sizeof(cplx<T>), h.stream>>>(cw, x, wv, wstride);
+            front_fwd_l21_kernel<T><<<dim3(nw, nb, z), 256, mk * sizeof(cplx<T>), br.st>>>(cw, x, wv, wstride);
             ++launches;
           }
         } else {
           if (nw && mu > 0) {
             const unsigned z = (unsigned)((mk + kSolveRows - 1) / kSolveRows);
-            front_bwd_u12_kernel<T><<<dim3(nw, nb, z), 256, (size_t)mu * sizeof(cplx<T>), h.stream>>>(cw, x);
+            front_bwd_u12_kernel<T><<<dim3(nw, nb, z), 256, (size_t)mu * sizeof(cplx<T>), br.st>>>(cw, x);
             ++launches;
           }
-          sym_bwd_kernel<T><<<dim3(nf, nb), bs, sm, h.stream>>>(c, x, maxb);
+          sym_bwd_kernel<T><<<dim3(nf, nb), bs, sm, br.st>>>(c, x, maxb);
         }
         ++launches;
       }
@@ -3384,6 +3438,10 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
       std::vector<int64_t> off;
       std::vector<int> ld, sk, sm;
       for (const SymFront &s : P->sf) off.push_back(s.off), ld.push_back(s.ld), sk.push_back(s.k), sm.push_back(s.m);
+      P->side.resize(kBranches - 1);
+      P->side_ev.resize(kBranches);
+      for (auto &st : P->side) SS_CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+      for (auto &e : P->side_ev) SS_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
       SS_CK(dupload(P->d_soff, off));
       SS_CK(dupload(P->d_sld, ld));
       SS_CK(dupload(P->d_sk, sk));

@@ -291,13 +291,14 @@ struct TmaCfg {
 
 // SYM: the tasks cover the upper triangle of symmetric update blocks, and the epilogue
 // writes (children's entries) - L21 U12 at the entries on and above the diagonal, the
-// children gathered through their inverse row maps, instead of updating C in place.
+// children gathered through their inverse row maps, instead of updating C in place.  `f0`
+// is the first frequency's place in the packed operands (the arena pointer is already there).
 template <int BNC, int STG, bool SYM = false>
 __global__ void __launch_bounds__(TmaCfg<BNC, STG>::THREADS, 1)
     tma_gemm_kernel(const __grid_constant__ CUtensorMap tmap, cf *__restrict__ arena, int64_t stride,
                     const int64_t *__restrict__ off, const int *__restrict__ ldv, const TmaTask *__restrict__ tasks,
                     int ntasks, int nb, int64_t stage_rows, int *__restrict__ err, const SymFront *__restrict__ sf = nullptr,
-                    const int *__restrict__ imap = nullptr) {
+                    const int *__restrict__ imap = nullptr, int f0 = 0) {
   using Cfg = TmaCfg<BNC, STG>;
   constexpr int NR = Cfg::NR;
   extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
@@ -347,7 +348,7 @@ __global__ void __launch_bounds__(TmaCfg<BNC, STG>::THREADS, 1)
       int64_t gc = 0;
       for (int64_t it = blockIdx.x; it < n_items && !abort_s; it += gridDim.x) {
         const TmaTask tk = tasks[it % ntasks];
-        const int64_t fb = (it / ntasks) * stage_rows + tk.base;   // this frequency's packed front
+        const int64_t fb = (f0 + it / ntasks) * stage_rows + tk.base;   // this frequency's packed front
         const int64_t bofs = fb + 2 * (int64_t)tk.kc * tk.au;
         for (int c = 0; c < tk.kc; ++c) {
           const int s = (int)(gc % STG);
