@@ -176,8 +176,7 @@ __global__ void __launch_bounds__(128, 3)
 //    kernel and the solves multiply by them instead of substituting;
 //  * sym_panel_kernel takes one chunk of columns of F12: it assembles the chunk in shared
 //    memory and solves it as rows of F21 = F12^T (z U11 = f^T: L21) and as columns of F12
-//    (L11 y = P f: U12), 16 unknowns at a time: a product with the rows or columns
-//    already solved, then one with the inverted diagonal block.
+//    (L11 y = P f: U12), 16 unknowns at a time with the inverted diagonal blocks.
 // With the block's LU in shared memory, one thread per panel column and a 16-step
 // substitution in the solves, a pass over the 32x128 ME1 cell at 51 points took 89 ms and
 // one over 16x64 at 101 points 21 ms; so, 61 and 15 ms.
@@ -569,85 +568,119 @@ __device__ __forceinline__ cplx<T> diag_coef(const cplx<T> *A, int ks, int i, in
   return LOWER ? A[i * ks + t] : A[t * ks + i];
 }
 
-// complex128: 8 NJ columns of the chunk tile Y (row stride CS, rows padded to a multiple
-// of 8) solved in place by one warp on the FP64 tensor cores: for 16 rows at a time, the
-// product with the rows already solved (three real products per complex block, fragments
-// as in front_dmma3_kernel), then with the inverted diagonal block.  Bound by the FP64
-// pipe: one thread per column with broadcast coefficients moved 4 x 16 bytes of shared
-// memory per complex multiply-add and took 27 us per 64-pivot, 64-column chunk.
-template <bool LOWER, int NJ>
-__device__ __forceinline__ void panel_dmma(const cd *A, int ks, cd *Y, int CS, int k) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  for (int h0 = 0; h0 < k; h0 += kDiagB) {
-    const int ni = k - h0 > 8 ? 2 : 1;
-    double p1[2][NJ][2], p2[2][NJ][2], p3[2][NJ][2];
-    auto clear = [&] {
+// complex128: 8 MB columns of the chunk (from cb) solved by one warp as 8 MB rows of the
+// transposed system, U12^T L11^T = (P F12)^T (LOWER) or L21 U11 = F12^T, on the FP64 tensor
+// cores.  The rows stay in accumulator registers; 16 pivots at a time they are multiplied
+// by the inverted diagonal block, written out, and subtracted from the columns to the
+// right (three real products per complex 8x8x4 block); an accumulator becomes the next
+// product's operand by shuffles within four lanes.
+template <bool LOWER, int KB, int MB>
+__device__ __forceinline__ void panel_dmma(const cd *A, int ks, const cd *Y, int CS, const int *perm, int k, int cb,
+                                           int nc, cd *out, int64_t ld) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, nbk = (k + 7) >> 3;
+  double xr[MB][KB][2], xi[MB][KB][2];
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
+  for (int j = 0; j < KB; ++j)
 #pragma unroll
-        for (int j = 0; j < NJ; ++j)
+    for (int e = 0; e < 2; ++e) {
+      const int r = 8 * j + 2 * t + e;
+      const int row = j < nbk ? (LOWER ? perm[r] : r) : 0;
 #pragma unroll
-          for (int e = 0; e < 2; ++e) p1[i][j][e] = p2[i][j][e] = p3[i][j][e] = 0.0;
-    };
-    auto mma = [&](const cd (&av)[2], int row) {
-#pragma unroll
-      for (int j = 0; j < NJ; ++j) {
-        const cd bv = Y[row * CS + j * 8 + g];
-        const double bs = bv.x + bv.y;
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          if (i >= ni) break;
-          dmma(p1[i][j][0], p1[i][j][1], av[i].x, bv.x);
-          dmma(p2[i][j][0], p2[i][j][1], av[i].y, bv.y);
-          dmma(p3[i][j][0], p3[i][j][1], av[i].x + av[i].y, bs);
-        }
+      for (int b = 0; b < MB; ++b) {
+        const cd z = j < nbk ? Y[row * CS + cb + 8 * b + g] : cd{0.0, 0.0};
+        xr[b][j][e] = z.x;
+        xi[b][j][e] = z.y;
       }
-    };
-    if (h0) {
+    }
+  // columns 4 h + t of an 8-column block held as columns 2 t, 2 t + 1
+  auto turn = [&](const double (&x)[2], int h) {
+    const int src = (lane & ~3) | (2 * h + (t >> 1));
+    const double x0 = __shfl_sync(0xffffffffu, x[0], src), x1 = __shfl_sync(0xffffffffu, x[1], src);
+    return t & 1 ? x1 : x0;
+  };
+  double ar[MB][2][2], ai[MB][2][2];      // operand: two 8-column blocks of two steps
+  auto operand = [&](int j, int kb) {
+#pragma unroll
+    for (int b = 0; b < MB; ++b)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        ar[b][kb][h] = turn(xr[b][j], h);
+        ai[b][kb][h] = turn(xi[b][j], h);
+      }
+  };
+  double p[MB][3][2];
+  auto clear = [&] {
+#pragma unroll
+    for (int b = 0; b < MB; ++b)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) p[b][q][0] = p[b][q][1] = 0.0;
+  };
+  auto mma = [&](int kb, int h, cd bv) {
+    const double bs = bv.x + bv.y;
+#pragma unroll
+    for (int b = 0; b < MB; ++b) {
+      dmma(p[b][0][0], p[b][0][1], ar[b][kb][h], bv.x);
+      dmma(p[b][1][0], p[b][1][1], ai[b][kb][h], bv.y);
+      dmma(p[b][2][0], p[b][2][1], ar[b][kb][h] + ai[b][kb][h], bs);
+    }
+  };
+#pragma unroll
+  for (int q = 0; q < (KB + 1) / 2; ++q) {
+    if (2 * q >= nbk) break;
+    const cd *D = A + 16 * q * (ks + 1);
+    const int nb2 = min(2, nbk - 2 * q);         // 8-column blocks of this diagonal block
+    operand(2 * q, 0);
+    if (2 * q + 1 < KB && nb2 > 1) operand(2 * q + 1, 1);
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      if (2 * q + n >= KB || n >= nb2) break;
       clear();
-#pragma unroll 2
-      for (int kk = 0; kk < h0; kk += 4) {
-        cd av[2];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const int row = h0 + (i < ni ? i * 8 : 0) + g;
-          av[i] = LOWER ? A[row * ks + kk + t] : A[(kk + t) * ks + row];
-        }
-        mma(av, kk + t);
-      }
+      for (int kb = 0; kb <= n; ++kb)
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < NJ; ++j)
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            if (i >= ni) continue;
-            cd *y = Y + (h0 + i * 8 + g) * CS + j * 8 + 2 * t + e;
-            *y = cd{y->x - (p1[i][j][e] - p2[i][j][e]), y->y - (p3[i][j][e] - p1[i][j][e] - p2[i][j][e])};
+        for (int h = 0; h < 2; ++h) {
+          const int kk = 8 * kb + 4 * h + t, nn = 8 * n + g;
+          cd bv = LOWER ? D[nn * ks + kk] : D[kk * ks + nn];
+          if (kb == n) {
+            if (kk > nn) bv = cd{0.0, 0.0};
+            if (LOWER && kk == nn) bv = cd{1.0, 0.0};
           }
-      __syncwarp();
+          mma(kb, h, bv);
+        }
+      const int j = 2 * q + n;
+#pragma unroll
+      for (int b = 0; b < MB; ++b)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const double re = p[b][0][e] - p[b][1][e], im = p[b][2][e] - p[b][0][e] - p[b][1][e];
+          xr[b][j][e] = re;
+          xi[b][j][e] = im;
+          const int c = cb + 8 * b + g, r = 8 * j + 2 * t + e;
+          if (c < nc && r < k) st_el(LOWER ? out + r * ld + c : out + c * ld + r, cd{re, im});
+        }
     }
-    clear();
+    if (2 * q + 2 >= KB || 2 * q + 2 >= nbk) break;
+    operand(2 * q, 0);
+    operand(2 * q + 1, 1);
 #pragma unroll
-    for (int kk = 0; kk < kDiagB; kk += 4) {
-      if (kk >= 8 * ni) break;
-      cd av[2];
+    for (int n = 2 * q + 2; n < KB; ++n) {
+      if (n >= nbk) break;
+      clear();
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
-        av[i] = diag_coef<double, LOWER>(A + h0 * ks + h0, ks, (i < ni ? i * 8 : 0) + g, kk + t);
-      mma(av, h0 + kk + t);
+      for (int kb = 0; kb < 2; ++kb)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int kk = 16 * q + 8 * kb + 4 * h + t, nn = 8 * n + g;
+          mma(kb, h, LOWER ? A[nn * ks + kk] : A[kk * ks + nn]);
+        }
+#pragma unroll
+      for (int b = 0; b < MB; ++b)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          xr[b][n][e] -= p[b][0][e] - p[b][1][e];
+          xi[b][n][e] -= p[b][2][e] - p[b][0][e] - p[b][1][e];
+        }
     }
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int j = 0; j < NJ; ++j)
-#pragma unroll
-        for (int e = 0; e < 2; ++e)
-          if (i < ni)
-            Y[(h0 + i * 8 + g) * CS + j * 8 + 2 * t + e] =
-                cd{p1[i][j][e] - p2[i][j][e], p3[i][j][e] - p1[i][j][e] - p2[i][j][e]};
-    __syncwarp();
   }
 }
 
@@ -709,7 +742,12 @@ __device__ __forceinline__ void panel_simt(const cf *A, int ks, cf *Y, int CS, i
   }
 }
 
-constexpr int kPanelColThreads = 128;
+// complex128: four warps for L21 and four for U12 of the same chunk (four warps that solved
+// one after the other, with P F12 through global memory and the tile in shared memory:
+// 45.5 against 42.6 ms for the factorisation of the 32x128 ME1 cell at 51 points, 16.4 against
+// 15.2 for the 8x2x26 Hex27 slab at 33); complex64: four warps, one after the other
+template <class T>
+__host__ __device__ constexpr int panel_threads() { return sizeof(T) == 8 ? 256 : 128; }
 // chunk width and padded sizes: the tile and F11 of one chunk leave room for at least two
 // CTAs per SM (complex128, 64 pivots: 104 KB at 32 columns; 64 would take 137)
 template <class T>
@@ -730,11 +768,11 @@ __host__ __device__ constexpr size_t panel_smem(int k, int cw) {
 }
 
 template <class T, int CW>
-__global__ void __launch_bounds__(kPanelColThreads, sizeof(T) == 8 ? 3 : 4)
+__global__ void __launch_bounds__(panel_threads<T>(), sizeof(T) == 8 ? 2 : 4)
     sym_panel_kernel(FrontArgs<T> a, const NarrowTask *__restrict__ tasks, int nb, const uint16_t *__restrict__ apos,
                      const int *__restrict__ aslot) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int NW = kPanelColThreads / 32, CS = CW + 2, NH = CW / 32;
+  constexpr int NT = panel_threads<T>(), NW = NT / 32, CS = CW + 2, NH = CW / 32;
   const NarrowTask tk = tasks[blockIdx.x / nb];
   const int fq = blockIdx.x % nb;
   const SymFront &s = a.sf[tk.f];
@@ -792,7 +830,7 @@ __global__ void __launch_bounds__(kPanelColThreads, sizeof(T) == 8 ? 3 : 4)
         if (lane + 64 < ks) A[r * ks + lane + 64] = cplx<T>{0, 0};
       }
     }
-    for (int i = tid; i < k; i += kPanelColThreads) perm[i] = a.piv[(int64_t)fq * a.n + s.p0 + i];
+    for (int i = tid; i < kp; i += NT) perm[i] = i < k ? a.piv[(int64_t)fq * a.n + s.p0 + i] : i;
   }
   __syncthreads();
   arrows.add_all(a, tk.a0, tk.a1, apos, aslot, om, [&](int p, cplx<T> e) {
@@ -800,38 +838,41 @@ __global__ void __launch_bounds__(kPanelColThreads, sizeof(T) == 8 ? 3 : 4)
     *d = *d + e;
   });
   __syncthreads();
-  // P F12 to the U12 rows; the tile is first solved as rows of L21
-  cplx<T> *U = F + k + tk.c0;
-  for (int r = wid; r < k; r += NW)
-#pragma unroll
-    for (int h = 0; h < NH; ++h) {
-      const int c = lane + 32 * h;
-      if (c < nc) st_el(U + r * ld + c, Y[perm[r] * CS + c]);
-    }
-  __syncthreads();
-  // each warp on its own columns from here on
-  constexpr int WC = CW / NW;
-  const int cb = wid * WC;
-  auto solve = [&](auto lower) {
-    constexpr bool LOWER = decltype(lower)::value;
-    if constexpr (sizeof(T) == 8)
-      panel_dmma<LOWER, WC / 8>(A, ks, Y + cb, CS, k);
+  if constexpr (sizeof(T) == 8) {
+    constexpr int MB = CW / 32, KB = CW == 64 ? 5 : 8;
+    const int cb = (wid & 3) * 8 * MB;
+    if (cb >= nc) return;
+    if (wid < 4)
+      panel_dmma<false, KB, MB>(A, ks, Y, CS, perm, k, cb, nc, F + (k + tk.c0) * ld, ld);
     else
-      panel_simt<LOWER>(A, ks, Y + cb, CS, k);
-  };
-  solve(std::false_type{});
-  for (int q = 0; q < WC; ++q)
-    if (cb + q < nc)
-      for (int r = lane; r < k; r += 32) st_el(F + (k + tk.c0 + cb + q) * ld + r, Y[r * CS + cb + q]);
-  __syncwarp();
-  const int c = lane % WC;
+      panel_dmma<true, KB, MB>(A, ks, Y, CS, perm, k, cb, nc, F + k + tk.c0, ld);
+  } else {
+    // P F12 to the U12 rows; the tile is first solved as rows of L21
+    cplx<T> *U = F + k + tk.c0;
+    for (int r = wid; r < k; r += NW)
+#pragma unroll
+      for (int h = 0; h < NH; ++h) {
+        const int c = lane + 32 * h;
+        if (c < nc) st_el(U + r * ld + c, Y[perm[r] * CS + c]);
+      }
+    __syncthreads();
+    // each warp on its own columns from here on
+    constexpr int WC = CW / NW;
+    const int cb = wid * WC;
+    panel_simt<false>(A, ks, Y + cb, CS, k);
+    for (int q = 0; q < WC; ++q)
+      if (cb + q < nc)
+        for (int r = lane; r < k; r += 32) st_el(F + (k + tk.c0 + cb + q) * ld + r, Y[r * CS + cb + q]);
+    __syncwarp();
+    const int c = lane % WC;
 #pragma unroll 4
-  for (int r = lane / WC; r < kp; r += 32 / WC)
-    Y[r * CS + cb + c] = r < k && cb + c < nc ? ld_el(U + r * ld + cb + c) : cplx<T>{0, 0};
-  __syncwarp();
-  solve(std::true_type{});
-  for (int r = lane / WC; r < k; r += 32 / WC)
-    if (cb + c < nc) st_el(U + r * ld + cb + c, Y[r * CS + cb + c]);
+    for (int r = lane / WC; r < kp; r += 32 / WC)
+      Y[r * CS + cb + c] = r < k && cb + c < nc ? ld_el(U + r * ld + cb + c) : cplx<T>{0, 0};
+    __syncwarp();
+    panel_simt<true>(A, ks, Y + cb, CS, k);
+    for (int r = lane / WC; r < k; r += 32 / WC)
+      if (cb + c < nc) st_el(U + r * ld + cb + c, Y[r * CS + cb + c]);
+  }
 }
 
 }  // namespace ss
