@@ -1937,6 +1937,7 @@ struct Plan {
   bool sym = false;
   std::vector<int> level_slot;
   std::vector<int> slot_maxk[4], slot_pank[2];   // most pivots: by pivot class, by chunk width
+  std::vector<int64_t> schur_mid;          // per slot: end of its 64-column FP64 tiles (32-column ones follow)
   std::vector<int64_t> npiv_ptr[4], npan_ptr[2];
   std::vector<NarrowTask> npiv[4], npan[2];
   std::vector<uint16_t> apos;
@@ -2013,6 +2014,12 @@ static void add_upper_tiles(std::vector<GemmTask> &v, int bm, int bn, int f, int
 // The trailing block is then read and written once per group instead of once per block,
 // with a four times longer K loop behind each tile's epilogue.
 constexpr int kGroup = 256;
+// FP64 updates of at most so many pivots take 32 x 32 tiles, longer ones 32 x 64: a short
+// product waits for its sources and operands, not for the tensor cores, so more and smaller
+// CTAs win, while the longer ones gain from the wider tile's reuse.  The line at 0, 32, 64,
+// 128 and 256: 32x128 ME1 (51 points) 55.2, 54.2, 53.2, 53.1, 53.2 ms; 64x256 (11 points)
+// 72.3, 71.4, 70.2, 70.2, 70.8; 16x64 ME0 (101 points) 13.0, 12.3, 12.2, 12.1, 12.1.
+constexpr int kShortUpdate = 128;
 
 // Launch plan of the symmetric path.
 Plan *build_sym_plan(Handle &h, bool tensor_schur) {
@@ -2151,13 +2158,17 @@ Plan *build_sym_plan(Handle &h, bool tensor_schur) {
       for (const Update &t : upd[i]) {
         if (tensor_schur)
           add_upper_tiles(P->tasks, tile_bm(kSquare), tile_bn(kSquare), t.id, t.k, t.rhi, t.m);
-        else
+        else if (t.k > kShortUpdate)
           add_upper_tiles(P->tasks, 32, 64, t.id, t.k, t.rhi, t.m);
         const int ur = t.rhi - t.k, uc = t.m - t.k;
         const double ar = (ur + tc::PADC - 1) / tc::PADC * tc::PADC, ac = (uc + tc::PADC - 1) / tc::PADC * tc::PADC;
         work += (double)ur * uc * t.k;
         padded += ar * ac * ((t.k + tc::KCH - 1) / tc::KCH * tc::KCH);
       }
+      P->schur_mid.push_back((int64_t)P->tasks.size());
+      if (!tensor_schur)
+        for (const Update &t : upd[i])
+          if (t.k <= kShortUpdate) add_upper_tiles(P->tasks, 32, 32, t.id, t.k, t.rhi, t.m);
       P->schur_ptr.push_back((int64_t)P->tasks.size());
       P->pick.push_back(tensor_schur ? 2 : 3);
       if (!tensor_schur) continue;
@@ -2733,7 +2744,11 @@ struct Sweeper {
     const GemmTask *tasks = P.d_tasks.template as<GemmTask>();
     const dim3 grid((unsigned)(t1 - t0), nb);
     if constexpr (sizeof(T) == 8) {
-      sym_schur_kernel<<<grid, 128, kSymSchurSmem, br.st>>>(a, tasks + t0);
+      const int64_t tm = P.schur_mid[q];
+      if (tm > t0)
+        sym_schur_kernel<64><<<dim3((unsigned)(tm - t0), nb), 128, sym_schur_smem<64>(), br.st>>>(a, tasks + t0);
+      if (t1 > tm)
+        sym_schur_kernel<32><<<dim3((unsigned)(t1 - tm), nb), 128, sym_schur_smem<32>(), br.st>>>(a, tasks + tm);
     } else {
       if (c == 2 || !P.tma_ok || P.pk_ptr[q + 1] == P.pk_ptr[q]) {
         front_gemm_kernel<T, kSquare, false, true>
@@ -3463,7 +3478,7 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
       if constexpr (sizeof(T) == 4)
         SS_CK(cudaFuncSetAttribute(front_gemm_kernel<T, kSquare, false, true>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_cst_bytes<T, kSquare>()));
-      SS_CK(cudaFuncSetAttribute(sym_schur_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSymSchurSmem));
+      SS_CK(cudaFuncSetAttribute(sym_schur_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, sym_schur_smem<64>()));
       SS_CK(cudaFuncSetAttribute(tc::tma_gemm_kernel<128, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  tc::TmaCfg<128, 2>::SMEM));
       SS_CK(cudaFuncSetAttribute(tc::tma_gemm_kernel<64, 3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -26,23 +26,26 @@
 namespace ss {
 
 // Upper triangle of an update block = (its sources) - L21 U12 on the FP64 tensor cores,
-// in tiles of 32 x 64 by four warps of 16 x 32 each (three real products per complex
+// in tiles of 32 x BN by four warps of 16 x BN / 2 each (three real products per complex
 // 8x8x4 block, operands staged as in front_dmma3_kernel).  The sources' entries are
 // copied into the staged C tile by cp.async when the CTA starts, so their latency overlaps
 // the K loop; entries that both sources have take the second one in the epilogue.  Tiles
 // below the diagonal are not launched; in the others a warp skips its 8x8 blocks below it,
 // and the K loop its last half chunk when that is empty.
+//   32 x 32, for short products: four CTAs per SM, the first operands are asked for before the
+// sources' row maps, and the second source's entries with the first ones.
 //   32 x 64: 96 accumulator registers, three CTAs per SM.  64 x 64 tiles (two CTAs) wait
 // for C more and leave more of a diagonal tile unused: 40.2 against 33.7 ms for the updates
 // of the 64x256 ME1 cell at 11 points, 10.5 against 8.6 ms for the 8x2x26 Hex27 slab at 33.
-constexpr int kSymCS = 65;
-constexpr int kSymSchurSmem = 32 * kSymCS * (int)sizeof(cd);
-__global__ void __launch_bounds__(128, 3)
+template <int BN>
+constexpr int sym_schur_smem() { return 32 * (BN + 1) * (int)sizeof(cd); }
+template <int BN>
+__global__ void __launch_bounds__(128, BN == 64 ? 3 : 4)
     sym_schur_kernel(FrontArgs<double> a, const GemmTask *__restrict__ tasks) {
-  constexpr int MB = 2, BM = 16 * MB, WR = 8 * MB, BS = 64 + 2;
+  constexpr int MB = 2, BM = 16 * MB, WR = 8 * MB, BS = BN + 2, WC = BN / 2, NJ = WC / 8, CS = BN + 1;
   __shared__ __align__(16) cd As[2][BM * kDmmaAS];
   __shared__ __align__(16) cd Bs[2][kDmmaBK * BS];
-  __shared__ int ir[2][BM], ic[2][64];
+  __shared__ int ir[2][BM], ic[2][BN];
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cd *Cs = reinterpret_cast<cd *>(smem_raw);
   const GemmTask tk = tasks[blockIdx.x];
@@ -64,9 +67,9 @@ __global__ void __launch_bounds__(128, 3)
                     ok ? F + (int64_t)gr * ld + gk : F, ok ? 16u : 0u);
     }
 #pragma unroll
-    for (int q = 0; q < kDmmaBK * 64 / 128; ++q) {
+    for (int q = 0; q < kDmmaBK * BN / 128; ++q) {
       const int idx = threadIdx.x + 128 * q;
-      const int k = idx / 64, c = idx % 64;
+      const int k = idx / BN, c = idx % BN;
       const int gk = kb + k, gc = tk.c0 + c;
       const bool ok = gk < tk.kk1 && gc < tk.chi;
       cp_async16_cd((uint32_t)__cvta_generic_to_shared(&Bs[buf][k * BS + c]), ok ? F + (int64_t)gk * ld + gc : F,
@@ -75,28 +78,55 @@ __global__ void __launch_bounds__(128, 3)
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   const int nk = (tk.kk1 - tk.kk0 + kDmmaBK - 1) / kDmmaBK;
+  if (BN == 32) issue(0, tk.kk0);
   if (nch) {
-    sym_stage<double, BM, 64, 128, kSymCS>(Cs, s, arena, a.imap, tk, ir, ic);
+    sym_stage<double, BM, BN, 128, CS>(Cs, s, arena, a.imap, tk, ir, ic);
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
   // first column block of the warp with an entry on or above the diagonal, per row block:
   // row block i needs column blocks j with 8 j + 7 >= 8 i + dr
-  const int dr = tk.r0 + wm * WR - (tk.c0 + wn * 32);
+  const int dr = tk.r0 + wm * WR - (tk.c0 + wn * WC);
   auto j0 = [&](int i) { return (8 * i + dr - 7 + 7) >> 3; };    // ceil((8 i + dr - 7) / 8)
   const int rows = min(tk.rhi, tk.r0 + BM) - (tk.r0 + wm * WR);  // the warp's rows inside the tile
-  double p1[MB][4][2], p2[MB][4][2], p3[MB][4][2];
+  // entries that both sources have: the second source's
+  cd cv[BN == 64 ? 1 : MB][NJ][2];
+  auto second = [&](int i) {
+    const int rl = wm * WR + i * 8 + g, r = tk.r0 + rl;
+    const bool two = nch > 1 && r < tk.rhi;
+    const int i0 = two ? ir[0][rl] : -1, i1 = two ? ir[1][rl] : -1;
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int cl = wn * WC + j * 8 + 2 * t + e, c = tk.c0 + cl;
+        cd &v = cv[BN == 64 ? 0 : i][j][e];
+        v = cd{0.0, 0.0};
+        if ((i0 | i1) >= 0 && c >= r && c < tk.chi && (ic[0][cl] | ic[1][cl]) >= 0)
+          v = ld_once(arena + s.cb[1] + (int64_t)i1 * s.cld[1] + ic[1][cl]);
+      }
+  };
+  if (BN == 32) {       // all of them with the first loads
+#pragma unroll
+    for (int i = 0; i < MB; ++i) second(i);
+  }
+  double p1[MB][NJ][2], p2[MB][NJ][2], p3[MB][NJ][2];
 #pragma unroll
   for (int i = 0; i < MB; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < NJ; ++j)
 #pragma unroll
       for (int e = 0; e < 2; ++e) p1[i][j][e] = p2[i][j][e] = p3[i][j][e] = 0.0;
-  const bool whole = j0(MB - 1) <= 0 && rows >= WR, some = rows > 0 && j0(0) < 4;
-  issue(0, tk.kk0);
+  const bool whole = j0(MB - 1) <= 0 && rows >= WR, some = rows > 0 && j0(0) < NJ;
+  if (BN == 64) issue(0, tk.kk0);
   for (int kc = 0; kc < nk; ++kc) {
     const int buf = kc & 1;
     if (kc + 1 < nk) {
       issue(buf ^ 1, tk.kk0 + (kc + 1) * kDmmaBK);
+      if (BN == 32 && kc == 0 && nch)
+        asm volatile("cp.async.wait_group 2;" ::: "memory");     // the C tile may still be on its way
+      else
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else if (BN == 32 && kc == 0 && nch) {
       asm volatile("cp.async.wait_group 1;" ::: "memory");
     } else {
       asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -113,9 +143,9 @@ __global__ void __launch_bounds__(128, 3)
         as[i] = av[i].x + av[i].y;
       }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
+      for (int j = 0; j < NJ; ++j) {
         if (!WHOLE && j < j0(0)) continue;
-        const cd bv = Bs[buf][(kk + t) * BS + wn * 32 + j * 8 + g];
+        const cd bv = Bs[buf][(kk + t) * BS + wn * WC + j * 8 + g];
         const double bs = bv.x + bv.y;
 #pragma unroll
         for (int i = 0; i < MB; ++i) {
@@ -136,33 +166,27 @@ __global__ void __launch_bounds__(128, 3)
     }
     __syncthreads();
   }
-  const bool two = nch > 1;
+  if (BN == 32 && nk == 1 && nch) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+  }
 #pragma unroll
   for (int i = 0; i < MB; ++i) {
     const int rl = wm * WR + i * 8 + g, r = tk.r0 + rl;
     if (r >= tk.rhi) continue;
     cd *Fr = F + (int64_t)r * ld;
-    const int i0 = nch ? ir[0][rl] : -1, i1 = two ? ir[1][rl] : -1;
-    cd cv[4][2];
+    if (BN == 64) second(i);
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int cl = wn * 32 + j * 8 + 2 * t + e, c = tk.c0 + cl;
-        cv[j][e] = cd{0.0, 0.0};
-        if (two && (i0 | i1) >= 0 && c >= r && c < tk.chi && (ic[0][cl] | ic[1][cl]) >= 0)
-          cv[j][e] = ld_once(arena + s.cb[1] + (int64_t)i1 * s.cld[1] + ic[1][cl]);
-      }
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < NJ; ++j)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int cl = wn * 32 + j * 8 + 2 * t + e, c = tk.c0 + cl;
+        const int cl = wn * WC + j * 8 + 2 * t + e, c = tk.c0 + cl;
         if (c < r || c >= tk.chi) continue;
-        if (nch) cv[j][e] = Cs[rl * kSymCS + cl] + cv[j][e];
+        cd v = cv[BN == 64 ? 0 : i][j][e];
+        if (nch) v = Cs[rl * CS + cl] + v;
         const double re = p1[i][j][e] - p2[i][j][e];
         const double im = p3[i][j][e] - p1[i][j][e] - p2[i][j][e];
-        st_el(Fr + c, cv[j][e] - cd{re, im});
+        st_el(Fr + c, v - cd{re, im});
       }
   }
 }
