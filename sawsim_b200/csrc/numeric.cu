@@ -2823,7 +2823,7 @@ struct Sweeper {
     const int64_t t0 = P.npan_ptr[c][q], t1 = P.npan_ptr[c][q + 1];
     if (t1 == t0) return;
     sym_panel_kernel<T, CW>
-        <<<(unsigned)((t1 - t0) * br.nb), panel_threads<T>(), panel_smem<T>(P.slot_pank[c][q], CW), br.st>>>(
+        <<<(unsigned)((t1 - t0) * br.nb), kPanelThreadsSym, panel_smem<T>(P.slot_pank[c][q], CW), br.st>>>(
             br.a, P.d_npan[c].template as<NarrowTask>() + t0, br.nb, P.d_apos.template as<uint16_t>(),
             P.d_aslot.template as<int>());
     ++launches;

@@ -766,12 +766,10 @@ __device__ __forceinline__ void panel_simt(const cf *A, int ks, cf *Y, int CS, i
   }
 }
 
-// complex128: four warps for L21 and four for U12 of the same chunk (four warps that solved
-// one after the other, with P F12 through global memory and the tile in shared memory:
-// 45.5 against 42.6 ms for the factorisation of the 32x128 ME1 cell at 51 points, 16.4 against
-// 15.2 for the 8x2x26 Hex27 slab at 33); complex64: four warps, one after the other
-template <class T>
-__host__ __device__ constexpr int panel_threads() { return sizeof(T) == 8 ? 256 : 128; }
+// Four warps for L21 and four for U12 of the same chunk.  (Four warps that solved one after
+// the other, with P F12 through global memory: 45.5 against 42.6 ms for the factorisation of
+// the 32x128 ME1 cell at 51 points, where complex128 keeps its rows in registers too.)
+constexpr int kPanelThreadsSym = 256;
 // chunk width and padded sizes: the tile and F11 of one chunk leave room for at least two
 // CTAs per SM (complex128, 64 pivots: 104 KB at 32 columns; 64 would take 137)
 template <class T>
@@ -788,15 +786,17 @@ __host__ __device__ constexpr int panel_ks(int k) {
 }
 template <class T>
 __host__ __device__ constexpr size_t panel_smem(int k, int cw) {
-  return ((size_t)panel_rows<T>(k) * (panel_ks<T>(k) + cw + 2)) * sizeof(cplx<T>) + (size_t)panel_rows<T>(k) * sizeof(int);
+  // (complex64 solves L21 and U12 in tiles of their own)
+  return ((size_t)panel_rows<T>(k) * (panel_ks<T>(k) + (sizeof(T) == 8 ? 1 : 2) * (cw + 2))) * sizeof(cplx<T>) +
+         (size_t)panel_rows<T>(k) * sizeof(int);
 }
 
 template <class T, int CW>
-__global__ void __launch_bounds__(panel_threads<T>(), sizeof(T) == 8 ? 2 : 4)
+__global__ void __launch_bounds__(kPanelThreadsSym, 2)
     sym_panel_kernel(FrontArgs<T> a, const NarrowTask *__restrict__ tasks, int nb, const uint16_t *__restrict__ apos,
                      const int *__restrict__ aslot) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int NT = panel_threads<T>(), NW = NT / 32, CS = CW + 2, NH = CW / 32;
+  constexpr int NT = kPanelThreadsSym, NW = NT / 32, CS = CW + 2, NH = CW / 32;
   const NarrowTask tk = tasks[blockIdx.x / nb];
   const int fq = blockIdx.x % nb;
   const SymFront &s = a.sf[tk.f];
@@ -804,7 +804,7 @@ __global__ void __launch_bounds__(panel_threads<T>(), sizeof(T) == 8 ? 2 : 4)
   const int64_t ld = s.ld;
   cplx<T> *A = reinterpret_cast<cplx<T> *>(smem_raw);   // F11 in pivot order, zero past k
   cplx<T> *Y = A + kp * ks;                             // the chunk
-  int *perm = reinterpret_cast<int *>(Y + kp * CS);
+  int *perm = reinterpret_cast<int *>(Y + (sizeof(T) == 8 ? 1 : 2) * kp * CS);
   cplx<T> *arena = a.arena + (int64_t)fq * a.stride;
   cplx<T> *F = arena + s.off;
   const double om = a.omega[fq];
@@ -871,31 +871,26 @@ __global__ void __launch_bounds__(panel_threads<T>(), sizeof(T) == 8 ? 2 : 4)
     else
       panel_dmma<true, KB, MB>(A, ks, Y, CS, perm, k, cb, nc, F + k + tk.c0, ld);
   } else {
-    // P F12 to the U12 rows; the tile is first solved as rows of L21
-    cplx<T> *U = F + k + tk.c0;
-    for (int r = wid; r < k; r += NW)
+    // P F12 in a tile of its own; each warp on its own columns of one of the tiles
+    constexpr int WC = CW / 4;
+    cplx<T> *Z = Y + kp * CS;
+    for (int r = wid; r < kp; r += NW)
 #pragma unroll
-      for (int h = 0; h < NH; ++h) {
-        const int c = lane + 32 * h;
-        if (c < nc) st_el(U + r * ld + c, Y[perm[r] * CS + c]);
-      }
+      for (int h = 0; h < NH; ++h) Z[r * CS + lane + 32 * h] = Y[perm[r] * CS + lane + 32 * h];
     __syncthreads();
-    // each warp on its own columns from here on
-    constexpr int WC = CW / NW;
-    const int cb = wid * WC;
-    panel_simt<false>(A, ks, Y + cb, CS, k);
-    for (int q = 0; q < WC; ++q)
-      if (cb + q < nc)
-        for (int r = lane; r < k; r += 32) st_el(F + (k + tk.c0 + cb + q) * ld + r, Y[r * CS + cb + q]);
-    __syncwarp();
-    const int c = lane % WC;
-#pragma unroll 4
-    for (int r = lane / WC; r < kp; r += 32 / WC)
-      Y[r * CS + cb + c] = r < k && cb + c < nc ? ld_el(U + r * ld + cb + c) : cplx<T>{0, 0};
-    __syncwarp();
-    panel_simt<true>(A, ks, Y + cb, CS, k);
-    for (int r = lane / WC; r < k; r += 32 / WC)
-      if (cb + c < nc) st_el(U + r * ld + cb + c, Y[r * CS + cb + c]);
+    const int cb = (wid & 3) * WC;
+    if (cb >= nc) return;
+    if (wid < 4) {
+      panel_simt<false>(A, ks, Y + cb, CS, k);
+      for (int q = 0; q < WC; ++q)
+        if (cb + q < nc)
+          for (int r = lane; r < k; r += 32) st_el(F + (k + tk.c0 + cb + q) * ld + r, Y[r * CS + cb + q]);
+    } else {
+      panel_simt<true>(A, ks, Z + cb, CS, k);
+      const int c = lane % WC;
+      for (int r = lane / WC; r < k; r += 32 / WC)
+        if (cb + c < nc) st_el(F + r * ld + k + tk.c0 + cb + c, Z[r * CS + cb + c]);
+    }
   }
 }
 
