@@ -2156,8 +2156,11 @@ Plan *build_sym_plan(Handle &h, bool tensor_schur) {
       }
       double work = 0, padded = 0;
       for (const Update &t : upd[i]) {
+        // complex64 tiles off the tensor cores: 64 x 64 leave less of a narrow front's tiles
+        // below the diagonal than 128 x 64 (8x4x48 mixed at 16 points 64.4 against 61.5 ms,
+        // 12x4x48 at 6 points 56.7 against 54.8)
         if (tensor_schur)
-          add_upper_tiles(P->tasks, tile_bm(kSquare), tile_bn(kSquare), t.id, t.k, t.rhi, t.m);
+          add_upper_tiles(P->tasks, tile_bm(kSquare64), tile_bn(kSquare64), t.id, t.k, t.rhi, t.m);
         else if (t.k > kShortUpdate)
           add_upper_tiles(P->tasks, 32, 64, t.id, t.k, t.rhi, t.m);
         const int ur = t.rhi - t.k, uc = t.m - t.k;
@@ -2751,8 +2754,8 @@ struct Sweeper {
         sym_schur_kernel<32><<<dim3((unsigned)(t1 - tm), nb), 128, sym_schur_smem<32>(), br.st>>>(a, tasks + tm);
     } else {
       if (c == 2 || !P.tma_ok || P.pk_ptr[q + 1] == P.pk_ptr[q]) {
-        front_gemm_kernel<T, kSquare, false, true>
-            <<<grid, 256, gemm_cst_bytes<T, kSquare>(), br.st>>>(a, tasks + t0);
+        front_gemm_kernel<T, kSquare64, false, true>
+            <<<grid, 256, gemm_cst_bytes<T, kSquare64>(), br.st>>>(a, tasks + t0);
         return;
       }
       const int64_t i0 = P.pi_ptr[q], i1 = P.pi_ptr[q + 1], q0 = P.tt_ptr[c][q], q1 = P.tt_ptr[c][q + 1];
@@ -3476,8 +3479,8 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
         SS_CK(cudaFuncSetAttribute(sym_panel_kernel<T, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)panel_smem<T>(64, 32)));
       if constexpr (sizeof(T) == 4)
-        SS_CK(cudaFuncSetAttribute(front_gemm_kernel<T, kSquare, false, true>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_cst_bytes<T, kSquare>()));
+        SS_CK(cudaFuncSetAttribute(front_gemm_kernel<T, kSquare64, false, true>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_cst_bytes<T, kSquare64>()));
       SS_CK(cudaFuncSetAttribute(sym_schur_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, sym_schur_smem<64>()));
       SS_CK(cudaFuncSetAttribute(tc::tma_gemm_kernel<128, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  tc::TmaCfg<128, 2>::SMEM));
