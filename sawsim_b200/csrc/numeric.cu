@@ -993,7 +993,7 @@ constexpr int gemm_cst_bytes() { return Tile<S>::BM * (Tile<S>::BN + 1) * (int)s
 // SYM: the tile belongs to the upper triangle of a symmetric update block and is
 // written as (its sources' entries) - A B (sym_front.cuh; tasks name pivot blocks).
 template <class T, int S, bool CST = false, bool SYM = false>
-__global__ void __launch_bounds__(256, (S == kThinCol || S == kThinRow) ? 4 : sizeof(T) == 4 ? 2 : 1)
+__global__ void __launch_bounds__(256, (S == kThinCol || S == kThinRow) ? 4 : (SYM && S == kSquare64) ? 3 : sizeof(T) == 4 ? 2 : 1)
     front_gemm_kernel(FrontArgs<T> a, const GemmTask *__restrict__ tasks) {
   constexpr int BM = Tile<S>::BM, BN = Tile<S>::BN, TM = Tile<S>::TM, TN = Tile<S>::TN, BK = kGemmBK;
   constexpr int TX = BN / TN, TY = BM / TM, CS = BN + 1;
