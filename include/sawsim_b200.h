@@ -250,8 +250,10 @@ int ss_adjoint_gradient(ss_handle *h, int n_f, const double *omega, double V, in
  *  the scaled system is complex symmetric and its fronts took the symmetric path
  *  (only the upper triangle of every update block is formed; 12 then counts the
  *  symmetric update, and 11 adds up the launches' own times, which they share with
- *  other frequencies' kernels: up to three groups of a chunk's frequencies run at once).
- *  Slots past 38 read 0.
+ *  other frequencies' kernels: up to three groups of a chunk's frequencies run at once),
+ *  39 points of the last sweep solved again on the general path because their symmetric
+ *  factors (pivots from blocks of at most 64 rows) were not good enough.
+ *  Slots past 39 read 0.
  */
 int ss_stats(const ss_handle *h, double *out, int n);
 

@@ -15,6 +15,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <limits>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -2473,6 +2474,8 @@ struct SweepOpts {
   int krylov_m = 30;
   int restarts = 1;
   double tol = 1e-8;
+  bool general = false;      // keep to the general path
+  char *weak = nullptr;      // out: points whose symmetric factors were not good enough (run_sweep)
 };
 
 // Fronts with m up to this are factored whole in shared memory (one CTA each);
@@ -2583,8 +2586,10 @@ static int equilibrate_sym(Handle &h, double w, bool &ok) {
 // Whether the symmetric path can take this handle's fronts at all: at most two
 // children per front (its kernels' gathers), 32-bit entry slots, and no forced general
 // tile (SS_SCHUR_TILE, SS_SCHUR_TILE_C64: measurement and test overrides of the
-// general path; SS_SYMMETRIC=0 switches the symmetric path off).
+// general path; SS_SYMMETRIC=0 switches the symmetric path off).  A system whose
+// symmetric factors failed every point of a sweep (run_sweep) keeps to the general path.
 static bool sym_possible(const Handle &h) {
+  if (h.sym_weak) return false;
   if (getenv("SS_SCHUR_TILE") || getenv("SS_SCHUR_TILE_C64")) return false;
   if (const char *e = getenv("SS_SYMMETRIC"))
     if (!atoi(e)) return false;
@@ -3404,7 +3409,7 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
   const int64_t n = S.n;
   double wmax = 0;
   for (int i = 0; i < n_f; ++i) wmax = std::max(wmax, std::fabs(omega[i]));
-  const bool try_sym = sym_possible(h);
+  const bool try_sym = !opt.general && sym_possible(h);
   if (h.scale_w != wmax || h.scale_tried != try_sym) {
     bool sym = false;
     if (try_sym) {
@@ -3646,7 +3651,34 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
   double fac_ms = 0, sol_ms = 0;
   std::vector<double> hn(2 * B);
   std::vector<int> hp(B), hit(B);
-  std::vector<char> conv(B);
+  std::vector<char> conv(B), weak(B);
+  // Points whose direct solve left a residual and a step that one refinement step does not
+  // make good.  With factors of growth g the solve has a backward error of about g u (u the
+  // unit roundoff) and its step a relative size of g u cond, so the step leaves an error of
+  // the square of that, and a stable factorisation (g of order 1) would leave u cond: the
+  // first is the larger one where their ratio, step size times backward error over u, passes
+  // 1.  (Entries of the scaled matrix are at most about 1, so |r| / |x| is the backward error.
+  // Measured: 16x64 ME0, 101 points, steps up to 5e-7 and 64x256 ME1 up to 1e-5, both at 5e-3
+  // of that bound; a dense front with a leading block of smallest singular value 1e-12 passes
+  // it by 1e5.)  The residual is read only if some step is larger than 1e-8: below that its
+  // square is under u.
+  auto mark_weak = [&](int nb, const double *step, const cd *res, const cd *sol) -> int {
+    bool look = false;
+    for (int f = 0; f < nb; ++f) look = look || !(step[2 * f] <= 1e-8 * step[2 * f + 1]);
+    if (!look) return SS_OK;
+    norm2_kernel<<<dim3(kRedCtas, nb), kRedThreads, 0, h.stream>>>(n, res, nrm.as<double>());
+    norm2_kernel<<<dim3(kRedCtas, nb), kRedThreads, 0, h.stream>>>(n, sol, nrm.as<double>() + nb);
+    std::vector<double> q(2 * nb);
+    SS_CK(cudaMemcpyAsync(q.data(), nrm.p, 2 * nb * sizeof(double), cudaMemcpyDeviceToHost, h.stream));
+    SS_CK(cudaStreamSynchronize(h.stream));
+    for (int f = 0; f < nb; ++f)
+      if (!(step[2 * f] * q[f] <= std::numeric_limits<double>::epsilon() * step[2 * f + 1] * q[nb + f])) weak[f] = 1;
+    if (getenv("SS_DEBUG_IR"))
+      for (int f = 0; f < nb; ++f)
+        fprintf(stderr, "point %d: step %.2e, backward error %.2e%s\n", f, step[2 * f] / step[2 * f + 1], q[f] / q[nb + f],
+                weak[f] ? " (weak)" : "");
+    return SS_OK;
+  };
   const unsigned vb = (unsigned)((n + 255) / 256);
   auto t_start = std::chrono::steady_clock::now();
   cudaEvent_t eall0, eall1;
@@ -3678,6 +3710,7 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
     sw.collect(nb);
     std::fill(conv.begin(), conv.end(), 0);
     std::fill(hit.begin(), hit.end(), 0);
+    std::fill(weak.begin(), weak.end(), 0);
     const bool use_krylov = sizeof(T) == 4 || getenv("SS_FP64_KRYLOV") != nullptr;
     const MatOp opA{h.dc_ptr.as<int64_t>(), h.dc_idx.as<int64_t>(), nullptr};
     if (use_krylov) {
@@ -3728,6 +3761,10 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
       }
       if (all) break;
     }
+    if (P.sym && sizeof(T) == 8 && !use_krylov) {
+      rc = mark_weak(nb, hn.data(), r.as<cd>(), x.as<cd>());
+      if (rc) return rc;
+    }
     // adjoint of the charge functional: A'^T mu = c with c = cs * kq (Q = c^T x' + V Qz)
     std::vector<cd> corr(nb, cd{0.0, 0.0});
     std::vector<char> aconv(nb, 1);
@@ -3776,6 +3813,13 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
         rc = sw.solve_graphed(2, nb, r.as<cd>(), dx.as<cd>());
         if (rc) return rc;
         axpy_norm_kernel<<<dim3(kRedCtas, nb), kRedThreads, 0, h.stream>>>(n, mu.as<cd>(), dx.as<cd>(), nrm.as<double>());
+        if (P.sym) {
+          std::vector<double> step(2 * nb);
+          SS_CK(cudaMemcpyAsync(step.data(), nrm.p, 2 * nb * sizeof(double), cudaMemcpyDeviceToHost, h.stream));
+          SS_CK(cudaStreamSynchronize(h.stream));
+          rc = mark_weak(nb, step.data(), r.as<cd>(), mu.as<cd>());
+          if (rc) return rc;
+        }
       }
       if (correct) {
         // dual-weighted correction: Q = c^T x + mu^T (b - A' x) is exact up to
@@ -3811,6 +3855,9 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
       const bool finite = std::isfinite(Qout[2 * (int64_t)(c0 + f)]) && std::isfinite(Qout[2 * (int64_t)(c0 + f) + 1]);
       const bool moved = !use_krylov && hp[f] > 0 && !(hn[2 * f] <= 1e-6 * hn[2 * f + 1]);
       if (status) status[c0 + f] = (!finite || moved) ? SS_ESINGULAR : ok ? SS_OK : SS_ENOCONV;
+      // (a Krylov loop that ran out may also have been slowed down by its factors)
+      if (opt.weak)
+        opt.weak[c0 + f] = P.sym && (weak[f] || !finite || moved || (use_krylov && !(conv[f] && aconv[f])));
       if (iters) iters[c0 + f] = hit[f];
     }
     if (disp) {
@@ -3892,6 +3939,13 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
 // A mixed sweep whose refinement leaves points unconverged re-solves those points
 // with the FP64 path in the same call (option fp64_fallback, on by default), so
 // every point returned has SS_OK unless FP64 fails too.
+//
+// The symmetric path looks for pivots in blocks of at most 64 rows, the general one in all
+// of a front's pivot rows, so a symmetric matrix whose leading blocks are (nearly) singular
+// can grow on the first and not on the second.  Points that show it (sweep_impl: their
+// residuals, non-finite or singular results; without fp64_fallback also mixed points that did
+// not converge) are solved again on the general path in the same call.  A system that
+// needed it at every point of a sweep goes there directly until its values change.
 int run_sweep(Handle &h, int n_f, const double *omega, double V, int precision, double *Q, int *status,
               int *iters, double *disp_out, const SweepExtra *ex) {
   SweepOpts opt;
@@ -3929,6 +3983,8 @@ int run_sweep(Handle &h, int n_f, const double *omega, double V, int precision, 
     probe_launches = h.st[15];
     h.st[28] = probe_ms;
   }
+  std::vector<char> weak(n_f, 0);
+  opt.weak = weak.data();
   if (precision == SS_PREC_MIXED)
     rc = sweep_impl<float>(h, n_f, omega, V, Q, status, iters, disp_out, ex, opt);
   else
@@ -3937,46 +3993,60 @@ int run_sweep(Handle &h, int n_f, const double *omega, double V, int precision, 
   h.st[19] = precision;
   h.st[29] = 0;
   h.st[33] = 0;
-  if (precision == SS_PREC_MIXED && h.opt.fp64_fallback) {
-    // maximal runs of consecutive unconverged points, each re-solved in FP64
-    std::vector<std::pair<int, int>> runs;
-    for (int i = 0; i < n_f;) {
-      if (status[i] != SS_ENOCONV) {
-        ++i;
-        continue;
-      }
-      int j = i;
-      while (j < n_f && status[j] == SS_ENOCONV) ++j;
-      runs.emplace_back(i, j);
-      i = j;
+  h.st[39] = 0;
+  // the marked points again, in maximal runs of consecutive ones (mark: also the runs' own
+  // `weak` flags); the statistics stay those of the first sweep
+  auto again = [&](std::vector<char> &mark, bool mixed, bool general, double &ms, int &points) -> int {
+    double keep[Handle::kStats];
+    std::copy(h.st, h.st + Handle::kStats, keep);
+    double launches = 0;
+    for (int i0 = 0, i1; i0 < n_f; i0 = i1) {
+      i1 = i0 + 1;
+      if (!mark[i0]) continue;
+      while (i1 < n_f && mark[i1]) ++i1;
+      const int len = i1 - i0;
+      SweepExtra exr;
+      if (ex && ex->per_chunk)
+        exr.per_chunk = [ex, i0](int c0, int nb, const cplx<double> *x, const cplx<double> *mu) {
+          return ex->per_chunk(c0 + i0, nb, x, mu);
+        };
+      SweepOpts o = opt;
+      o.general = general;
+      o.weak = mark.data() + i0;
+      std::vector<int> it2(len, 0);
+      const int rc = mixed ? sweep_impl<float>(h, len, omega + i0, V, Q + 2 * (int64_t)i0, status + i0, it2.data(),
+                                               disp_out, ex ? &exr : nullptr, o)
+                           : sweep_impl<double>(h, len, omega + i0, V, Q + 2 * (int64_t)i0, status + i0, it2.data(),
+                                                disp_out, ex ? &exr : nullptr, o);
+      if (rc) return rc;
+      for (int f = 0; f < len; ++f) iters[i0 + f] += it2[f];
+      ms += h.st[17];
+      launches += h.st[15];
+      points += len;
     }
-    if (!runs.empty()) {
-      double keep[Handle::kStats];
-      std::copy(h.st, h.st + Handle::kStats, keep);
-      double fb_ms = 0, fb_launches = 0;
-      int resolved = 0;
-      for (const auto &r : runs) {
-        const int i0 = r.first, len = r.second - r.first;
-        SweepExtra exr;
-        if (ex && ex->per_chunk)
-          exr.per_chunk = [ex, i0](int c0, int nb, const cplx<double> *x, const cplx<double> *mu) {
-            return ex->per_chunk(c0 + i0, nb, x, mu);
-          };
-        std::vector<int> it2(len, 0);
-        rc = sweep_impl<double>(h, len, omega + i0, V, Q + 2 * (int64_t)i0, status + i0, it2.data(),
-                                disp_out, ex ? &exr : nullptr, opt);
-        if (rc) return rc;
-        for (int f = 0; f < len; ++f) iters[i0 + f] += it2[f];
-        fb_ms += h.st[17];
-        fb_launches += h.st[15];
-        resolved += len;
-      }
-      std::copy(keep, keep + Handle::kStats, h.st);
-      h.st[17] += fb_ms;
-      h.st[15] += fb_launches;
-      h.st[29] = resolved;
-      h.st[33] = fb_ms;
-    }
+    std::copy(keep, keep + Handle::kStats, h.st);
+    h.st[17] += ms;
+    h.st[15] += launches;
+    return SS_OK;
+  };
+  const bool mixed = precision == SS_PREC_MIXED;
+  if (mixed && h.opt.fp64_fallback) {
+    for (int i = 0; i < n_f; ++i) weak[i] = weak[i] || status[i] == SS_ENOCONV;
+    double ms = 0;
+    int points = 0;
+    rc = again(weak, false, false, ms, points);
+    if (rc) return rc;
+    h.st[29] = points;
+    h.st[33] = ms;
+  }
+  if (std::find(weak.begin(), weak.end(), 1) != weak.end()) {
+    double ms = 0;
+    int points = 0;
+    rc = again(weak, mixed && !h.opt.fp64_fallback, true, ms, points);
+    if (rc) return rc;
+    h.st[39] = points;
+    if (mixed && !h.opt.fp64_fallback) h.st[32] = (double)std::count(status, status + n_f, SS_ENOCONV);
+    h.sym_weak = points == n_f;
   }
   h.st[17] += probe_ms;        // the probe is part of an AUTO sweep's device time
   h.st[15] += probe_launches;

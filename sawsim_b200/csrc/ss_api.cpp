@@ -66,9 +66,16 @@ extern "C" void ss_destroy(ss_handle *hp) {
 
 extern "C" const char *ss_last_error(const ss_handle *hp) { return hp ? hp->h.err.c_str() : kNoHandle; }
 
+// what was kept for the old values: the scaling, the choice of path and SS_PREC_AUTO's
+static void new_values(Handle &h) {
+  h.scale_w = -1;
+  h.sym_weak = false;
+  h.auto_prec = -1;
+}
+
 static void reset_derived(Handle &h) {
   h.analyzed = false;
-  h.scale_w = -1;
+  new_values(h);
   free_plans(h);
 }
 
@@ -201,8 +208,7 @@ extern "C" int ss_assemble(ss_handle *hp) {
       reset_derived(h);
       return rc;
     }
-    h.scale_w = -1;      // equilibrate again at the next sweep
-    h.auto_prec = -1;    // a kept SS_PREC_AUTO decision was for the old values
+    new_values(h);
   } else {
     reset_derived(h);
   }
@@ -281,8 +287,7 @@ extern "C" int ss_set_values(ss_handle *hp, int which, const double *vals) {
       reset_derived(h);
       return rc;
     }
-    h.scale_w = -1;
-    h.auto_prec = -1;
+    new_values(h);
   }
   return SS_OK;
 }
@@ -381,7 +386,7 @@ extern "C" int ss_set_damping(ss_handle *hp, double beta) {
   if (!std::isfinite(beta) || beta < 0.0) return fail(h, SS_EINVAL, "damping: beta must be finite and >= 0");
   if (beta != 0.0 && !h.have_D) return fail(h, SS_ESTATE, "damping: assemble D first (damping materials, or ss_set_values)");
   h.beta = beta;
-  h.scale_w = -1;
+  new_values(h);
   free_plans(h);   // the captured launch graphs bake beta and the damping matrix in
   return SS_OK;
 }
@@ -437,6 +442,7 @@ extern "C" int ss_set_option(ss_handle *hp, const char *name, double value) {
     if (!(value >= 0.0 && value < 1.0)) return fail(h, SS_EINVAL, "option pivot_tiny: in [0, 1)");
     (k == "pivot_tiny_c128" ? o.tiny_c128 : o.tiny_c64) = value;
     free_plans(h);   // the captured factorisation graphs bake the threshold in
+    new_values(h);
   } else if (k == "fp64_fallback") {
     if (!whole(0, 1)) return fail(h, SS_EINVAL, "option fp64_fallback: 0 or 1");
     o.fp64_fallback = (int)value;

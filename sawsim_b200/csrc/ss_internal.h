@@ -176,6 +176,7 @@ struct Handle {
   double scale_w = -1;                   // frequency the scaling was computed at
   bool scale_sym = false;                // the scaled system is symmetric (the symmetric scaling was kept)
   bool scale_tried = false;              // the symmetric scaling was tried
+  bool sym_weak = false;                 // every point of a sweep had to leave the symmetric path (run_sweep)
   // solver options (ss_set_option); kept until changed
   struct Options {
     int krylov_m = 30;                   // FGMRES restart length of the mixed sweep
@@ -187,7 +188,7 @@ struct Handle {
     int auto_probe_m = 12;               // Krylov steps of SS_PREC_AUTO's probe
   } opt;
   // stats
-  static constexpr int kStats = 39;
+  static constexpr int kStats = 40;
   double st[kStats] = {0};
 };
 
