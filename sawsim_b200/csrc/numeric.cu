@@ -1888,6 +1888,7 @@ struct Plan {
   int small_m = 0;                         // threshold used
   double schur_flops = 0;
   std::vector<int> lvl_maxk, lvl_maxu;     // per level max k and max m-k (solve grids)
+  std::vector<int> lvl_maxm;               // per level max m (symmetric solves)
   // CUDA graphs of the per-chunk launch sequences, replayed for every chunk with
   // the same batch size and buffers (key: nb and the device pointers they bake in)
   struct Graph {
@@ -2044,7 +2045,7 @@ Plan *build_sym_plan(Handle &h, bool tensor_schur) {
   };
   std::vector<std::vector<Update>> upd;
   for (int l = 0; l < S.nlevel; ++l) {
-    int lk = 0, lu = 0, steps = 0;
+    int lk = 0, lu = 0, lm = 0, steps = 0;
     piv.assign(0, {});
     pan.assign(0, {});
     upd.assign(0, {});
@@ -2052,6 +2053,7 @@ Plan *build_sym_plan(Handle &h, bool tensor_schur) {
       const int f = S.level_fronts[q], k = S.k[f], m = S.m[f], ld = S.ld[f];
       lk = std::max(lk, k);
       lu = std::max(lu, m - k);
+      lm = std::max(lm, m);
       const int bs = sym_block(k), nblk = (k + bs - 1) / bs;
       const int cw = tensor_schur ? panel_cols<float>(bs) : panel_cols<double>(bs);   // chunk width
       steps = std::max(steps, nblk);
@@ -2140,6 +2142,7 @@ Plan *build_sym_plan(Handle &h, bool tensor_schur) {
     P->wide_ptr.push_back((int)P->wide.size());
     P->lvl_maxk.push_back(lk);
     P->lvl_maxu.push_back(lu);
+    P->lvl_maxm.push_back(lm);
     for (int i = 0; i < steps; ++i) {
       for (int c = 0; c < 4; ++c) {
         int mk = 0;
@@ -2583,12 +2586,22 @@ static int equilibrate_sym(Handle &h, double w, bool &ok) {
   return SS_OK;
 }
 
+// Shared memory, in elements, of the symmetric solve kernels on a level whose fronts have
+// at most k pivots and m rows: the widest staged block (sym_block is not monotone in k) and
+// one front's vector.
+static size_t sym_solve_elems(int k, int m) {
+  const int b = k <= kNarrowK ? sym_block(k) : kNarrowK;
+  return (size_t)b * (b + 1) + m;
+}
+
 // Whether the symmetric path can take this handle's fronts at all: at most two
-// children per front (its kernels' gathers), 32-bit entry slots, and no forced general
+// children per front (its kernels' gathers), 32-bit entry slots, a front's vector in the
+// shared memory of one solve CTA beside a block (element size eb: 10,368 rows in complex128,
+// where the general solves go a little further), and no forced general
 // tile (SS_SCHUR_TILE, SS_SCHUR_TILE_C64: measurement and test overrides of the
 // general path; SS_SYMMETRIC=0 switches the symmetric path off).  A system whose
 // symmetric factors failed every point of a sweep (run_sweep) keeps to the general path.
-static bool sym_possible(const Handle &h) {
+static bool sym_possible(const Handle &h, size_t eb) {
   if (h.sym_weak) return false;
   if (getenv("SS_SCHUR_TILE") || getenv("SS_SCHUR_TILE_C64")) return false;
   if (const char *e = getenv("SS_SYMMETRIC"))
@@ -2596,6 +2609,15 @@ static bool sym_possible(const Handle &h) {
   const Symbolic &S = h.sym;
   for (int f = 0; f < S.nfront; ++f)
     if (S.child_ptr[f + 1] - S.child_ptr[f] > 2) return false;
+  if (sym_solve_elems(S.max_k, S.max_m) * eb > 227 * 1024)
+    for (int l = 0; l < S.nlevel; ++l) {
+      int k = 0, m = 0;
+      for (int64_t q = S.level_ptr[l]; q < S.level_ptr[l + 1]; ++q) {
+        k = std::max(k, S.k[S.level_fronts[q]]);
+        m = std::max(m, S.m[S.level_fronts[q]]);
+      }
+      if (sym_solve_elems(k, m) * eb > 227 * 1024) return false;
+    }
   return h.c_nnz < ((int64_t)1 << 31);
 }
 
@@ -3278,10 +3300,9 @@ struct Sweeper {
         const int l = pass == 0 ? i : S.nlevel - 1 - i;
         const int mk = P.lvl_maxk[l], mu = P.lvl_maxu[l];
         const int nf = (int)(S.level_ptr[l + 1] - S.level_ptr[l]), nw = P.wide_ptr[l + 1] - P.wide_ptr[l];
-        // the widest block of the level (sym_block is not monotone in k)
         const int maxb = mk <= kNarrowK ? sym_block(mk) : kNarrowK;
         const int bs = mk + mu <= 192 ? 128 : 256;
-        const size_t sm = ((size_t)maxb * (maxb + 1) + mk + mu) * sizeof(cplx<T>);
+        const size_t sm = sym_solve_elems(mk, P.lvl_maxm[l]) * sizeof(cplx<T>);
         FrontArgs<T> c = br.a, cw = br.a;
         c.fronts = lf + S.level_ptr[l];
         cw.fronts = wide + P.wide_ptr[l];
@@ -3409,7 +3430,7 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
   const int64_t n = S.n;
   double wmax = 0;
   for (int i = 0; i < n_f; ++i) wmax = std::max(wmax, std::fabs(omega[i]));
-  const bool try_sym = !opt.general && sym_possible(h);
+  const bool try_sym = !opt.general && sym_possible(h, sizeof(cplx<T>));
   if (h.scale_w != wmax || h.scale_tried != try_sym) {
     bool sym = false;
     if (try_sym) {
@@ -3504,7 +3525,7 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
     const int vecd = (int)std::min<int64_t>(227 * 1024, vec + (int64_t)kDiagElems * sizeof(cplx<T>) +
                                                            ((int64_t)std::max(1, S.max_k) * 4 + 15) / 16 * 16);
     if (P->sym) {
-      const int sm = (int)std::min<int64_t>(227 * 1024, (int64_t)(kNarrowK * (kNarrowK + 1) + S.max_k + S.max_m) * (int64_t)sizeof(cplx<T>));
+      const int sm = (int)std::min<size_t>(227 * 1024, sym_solve_elems(kNarrowK, S.max_m) * sizeof(cplx<T>));
       SS_CK(cudaFuncSetAttribute(sym_fwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
       SS_CK(cudaFuncSetAttribute(sym_bwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
     }
