@@ -1897,6 +1897,7 @@ struct Plan {
     const void *key[10];
     cudaGraphExec_t exec = nullptr;
     int launches = 0, schur_launches = 0;
+    int nev = 0;                           // timed Schur updates (pairs of P.ev) in the graph
   };
   std::vector<Graph> graphs;
   std::vector<cudaEvent_t> ev;             // Schur GEMM timing, one pair per level (owned here so
@@ -1946,7 +1947,6 @@ struct Plan {
   std::vector<int> aslot, imap;
   std::vector<SymFront> sf;
   std::vector<int> wide, wide_ptr;         // fronts of more than one pivot block, by level
-  int sym_nev = 0;                         // timed Schur updates of one factorisation
   // streams of the second and further groups of frequencies (Sweeper::branched)
   std::vector<cudaStream_t> side;
   std::vector<cudaEvent_t> side_ev;        // fork, then one join per side stream
@@ -2711,9 +2711,10 @@ struct Sweeper {
       SS_CK(cudaGraphLaunch(g.exec, h.stream));
       launches += g.launches;
       schur_launches += g.schur_launches;
+      nev += g.nev;
       return SS_OK;
     }
-    const int l0 = launches, s0 = schur_launches;
+    const int l0 = launches, s0 = schur_launches, v0 = nev;
     cudaGraph_t graph = nullptr;
     SS_CK(cudaStreamBeginCapture(h.stream, cudaStreamCaptureModeThreadLocal));
     const int rc = body();
@@ -2732,6 +2733,7 @@ struct Sweeper {
     SS_CK(ie);
     g.launches = launches - l0;
     g.schur_launches = schur_launches - s0;
+    g.nev = nev - v0;
     P.graphs.push_back(g);
     SS_CK(cudaGraphLaunch(g.exec, h.stream));
     return SS_OK;
@@ -2860,10 +2862,7 @@ struct Sweeper {
   }
   // the symmetric factorisation's launch sequence
   int sym_factor(int nb) {
-    nev = 0;
-    const int rc = branched(nb, [&](const Branch &br) { return sym_factor_branch(br); });
-    P.sym_nev = nev;
-    return rc;
+    return branched(nb, [&](const Branch &br) { return sym_factor_branch(br); });
   }
   int sym_factor_branch(const Branch &br) {
     for (int l = 0; l < h.sym.nlevel; ++l)
@@ -2888,14 +2887,13 @@ struct Sweeper {
   // factorisation of a chunk as one graph replay
   int factor_graphed(int nb) {
     if (P.sym) {
-      int rc = sym_tune(nb);
+      const int rc = sym_tune(nb);
       if (rc) return rc;
+      nev = 0;
       // (the tensor map baked into the graph depends on the staging buffer and its rows)
-      rc = graphed(100, nb, {a.arena, a.piv, a.omega, a.Kc, a.Mc, a.Dc, a.nperturb, tc_err, h.tc_stage.p,
-                             reinterpret_cast<const void *>((uintptr_t)chunk)},
-                   [&] { return sym_factor(nb); });
-      nev = P.sym_nev;
-      return rc;
+      return graphed(100, nb, {a.arena, a.piv, a.omega, a.Kc, a.Mc, a.Dc, a.nperturb, tc_err, h.tc_stage.p,
+                               reinterpret_cast<const void *>((uintptr_t)chunk)},
+                     [&] { return sym_factor(nb); });
     }
     {
       const int rc = tune(nb);
