@@ -37,7 +37,8 @@ CPU_SAMPLE = {'me0_16x64': [dict(cols=8, rows=32), dict(cols=16, rows=64)],
               'me1_64x256': [dict(cols=16, rows=64), dict(cols=32, rows=128)],
               'me1_128x512': [dict(cols=16, rows=64), dict(cols=32, rows=128)],
               'hex_8x4x48': [dict(nx=8, ny=1, nz=12), dict(nx=8, ny=2, nz=24)]}
-SCHUR_DRAM_BYTES_PER_POINT = {'me1_64x256': 6.16e9}
+SCHUR_DRAM_BYTES_PER_POINT = {'me1_64x256': 6.16e9}            # general path
+SYM_FACTOR_DRAM_BYTES_PER_POINT = {'me1_64x256': 5.60e9}       # symmetric path, the whole factorisation
 FULL_POINT_LIMIT_S = 300.0     # the measured full-size CPU point gives up after this (a lower bound)
 METRIC = 'Y11 points/s, 1 B200: batched FP32-TC+refine vs FP64 sweep, fr/fa within 1 kHz'
 
@@ -258,6 +259,20 @@ def workload_name(c):
             f'{c.freqs[0] / 1e9:.1f}-{c.freqs[-1] / 1e9:.1f} GHz, seed {i["seed"]}')
 
 
+def factor_kernel_name(s, used):
+    """The kernels of a symmetric factorisation; in mixed precision with the updates per
+    candidate of the plan's autotuner."""
+    if used == 'fp64':
+        update = 'sym_schur_kernel<64> / <32> (FP64 tensor cores, upper triangles)'
+    else:
+        names = ['tc::pack_kernel + tc::tma_gemm_kernel<128,2,true> (TMA + tcgen05 3xTF32)',
+                 'tc::pack_kernel + tc::tma_gemm_kernel<64,3,true> (TMA + tcgen05 3xTF32)',
+                 'front_gemm_kernel<float,kSquare64,false,true> (SIMT FP32 64x64)']
+        update = ', '.join(f'{n} for {int(s[k])} updates' for n, k in
+                           zip(names, ('schur_candidate0', 'schur_candidate1', 'schur_candidate2')) if s.get(k, 0) > 0)
+    return f'symmetric factorisation: sym_pivot_kernel, sym_panel_kernel, {update}'
+
+
 def schur_kernel_name(s, used):
     """The Schur-update kernels the plan's autotuner picked, with their level counts."""
     if used == 'mixed':
@@ -324,14 +339,24 @@ def mode_comparison(eng, f, w, reps):
 def rooflines(eng, c, s, st0, used, schur_ms, nf, pk, pk_kind, ceilings):
     """Roofline entries: the Schur update (tensor), the triangular solves and the
     assembly (HBM), each from this run's CUDA-event times and the algorithmic work
-    of the project's symbolic analysis."""
+    of the project's symbolic analysis.  On the symmetric path the first entry is the
+    whole factorisation: its launches of up to three groups of frequencies run beside
+    each other, so a launch has no time of its own."""
     out = []
+    symmetric = s.get('symmetric', 0) > 0
     launches = max(1.0, s['schur_launches'])
-    flops_launch = s['schur_gemm_flops'] / launches
-    ms_launch = float(np.mean(schur_ms)) / launches
+    if symmetric:      # a symmetric factorisation's operations: half of the general one's
+        launches, ms_launch, flops_launch = 1.0, s['factor_ms'], 0.5 * st0['factor_flops_per_point'] * nf
+    else:
+        flops_launch = s['schur_gemm_flops'] / launches
+        ms_launch = float(np.mean(schur_ms)) / launches
     achieved = flops_launch / (ms_launch * 1e-3) / 1e12 if ms_launch > 0 else None
     traffic, traffic_note = None, None
-    if used == 'fp64' and c.name in SCHUR_DRAM_BYTES_PER_POINT:
+    if symmetric and used == 'fp64' and c.name in SYM_FACTOR_DRAM_BYTES_PER_POINT:
+        traffic = SYM_FACTOR_DRAM_BYTES_PER_POINT[c.name] * nf
+        traffic_note = ('dram__bytes_read.sum + dram__bytes_write.sum of the factorisation kernels in an ncu capture of '
+                        "2 points of this cell, scaled to this run's points; not measured in this run")
+    elif not symmetric and used == 'fp64' and c.name in SCHUR_DRAM_BYTES_PER_POINT:
         traffic = SCHUR_DRAM_BYTES_PER_POINT[c.name] * nf / launches
         traffic_note = ('dram__bytes_read.sum + dram__bytes_write.sum of the Schur launches in an ncu capture of '
                         '1 and 2 points of this cell (bytes grow in proportion to the points), scaled to this '
@@ -348,10 +373,10 @@ def rooflines(eng, c, s, st0, used, schur_ms, nf, pk, pk_kind, ceilings):
                      'with 512 pivots (ss_measure_gemm_ceiling, median of 5 launches; DMMA with three real products '
                      'per complex block counts the algorithmic complex flops, so it can exceed the nominal FP64 '
                      'tensor peak of 37-40 TFLOP/s)')
-    out.append(dict(kernel=schur_kernel_name(s, used), bound='tensor', achieved=achieved, peak=peak, unit='TFLOP/s',
+    out.append(dict(kernel=(factor_kernel_name if symmetric else schur_kernel_name)(s, used), bound='tensor', achieved=achieved, peak=peak, unit='TFLOP/s',
                     frac=(achieved / peak) if achieved and peak else None, traffic=traffic,
-                    traffic_unit='bytes per launch', traffic_note=traffic_note, peak_note=peak_note,
-                    flops_per_launch=flops_launch))
+                    traffic_unit='bytes per sweep' if symmetric else 'bytes per launch', traffic_note=traffic_note, peak_note=peak_note,
+                    **{'flops_per_sweep' if symmetric else 'flops_per_launch': flops_launch}))
     hbm = pk.get('hbm_gbs', 6650.0)
     # triangular solves: the first solve of every chunk (forward + backward over all
     # fronts), algorithmic bytes nnz(L+U) x scalar + 2 n x 16 per point
@@ -360,8 +385,9 @@ def rooflines(eng, c, s, st0, used, schur_ms, nf, pk, pk_kind, ceilings):
     sb = nf * (st0['nnz_lu'] * scal + 2 * n * 16)
     if s['solve_ms'] > 0:
         ach = sb / (s['solve_ms'] * 1e-3) / 1e9
-        out.append(dict(kernel='front_fwd* / front_bwd* (batched forward + backward triangular solves, first solve '
-                               'of every chunk)', bound='hbm', achieved=ach, peak=hbm, unit='GB/s', frac=ach / hbm,
+        names = ('sym_fwd_kernel / sym_bwd_kernel, front_fwd_l21_kernel / front_bwd_u12_kernel of the wide fronts'
+                 if symmetric else 'front_fwd* / front_bwd*')
+        out.append(dict(kernel=f'{names} (batched forward + backward triangular solves, first solve of every chunk)', bound='hbm', achieved=ach, peak=hbm, unit='GB/s', frac=ach / hbm,
                         traffic=None, bytes_per_point=sb / nf,
                         peak_note=f'{pk_kind} copy bandwidth (MEASURED_PEAKS.json hbm_gbs)'))
     # assembly: K and M written on the CSR pattern + coordinates + connectivity +
@@ -486,7 +512,7 @@ def b200_arm(a, rank, world, local):
                                 setup_s=setup_s, analyze_s=st0['analyze_s'], assemble_ms=st0['assemble_ms'],
                                 l2='inputs larger than L2 (front arena of GBs per chunk)',
                                 chunk=int(s['chunk']), points_not_converged=bad,
-                                panel_gemm=dict(tiles=int(s['panel_gemm_dmma']),
+                                panel_gemm=None if s['symmetric'] else dict(tiles=int(s['panel_gemm_dmma']),
                                                 thin_tiles_per_point=int(s['panel_thin_tiles']),
                                                 note='0 SIMT, 1 DMMA, 2 DMMA three products, 3 the same with C '
                                                      'staged, 4 SIMT with C staged; thin: tasks <= 8 wide in '

@@ -247,10 +247,15 @@ int ss_adjoint_gradient(ss_handle *h, int n_f, const double *omega, double V, in
  *  memory while the K loop runs), 37 panel-step GEMM tiles per point run as
  *  thin SIMT 128x8 / 8x128 tiles (tasks at most 8 columns wide or 8 rows high,
  *  beside the DMMA tiles; 0 when the autotuner kept them in DMMA tiles), 38 1 when
- *  the scaled system is complex symmetric and its fronts took the symmetric path
- *  (only the upper triangle of every update block is formed; 12 then counts the
- *  symmetric update, and 11 adds up the launches' own times, which they share with
- *  other frequencies' kernels: up to three groups of a chunk's frequencies run at once),
+ *  the scaled system is complex symmetric and its fronts took the symmetric path:
+ *  only the upper triangle of every update block is formed.  12 then counts the
+ *  symmetric update; 11 adds up the launches' own times, which they share with
+ *  other frequencies' kernels (up to three groups of a chunk's frequencies run at
+ *  once), so 12 / 11 is not a kernel's rate; 20-22 count the updates of one complex64
+ *  factorisation, not levels, by candidate: packed operands + TMA + tcgen05 3xTF32 with
+ *  128 / 64 complex columns, SIMT FP32 64x64 (a level has one update per pivot block of
+ *  its widest front), and read 0 in FP64, whose update has one kernel; 23-26, 36 and
+ *  37 describe kernels of the general path and read 0,
  *  39 points of the last sweep solved again on the general path because their symmetric
  *  factors (pivots from blocks of at most 64 rows) were not good enough.
  *  Slots past 39 read 0.

@@ -2177,7 +2177,7 @@ Plan *build_sym_plan(Handle &h, bool tensor_schur) {
         for (const Update &t : upd[i])
           if (t.k <= kShortUpdate) add_upper_tiles(P->tasks, 32, 32, t.id, t.k, t.rhi, t.m);
       P->schur_ptr.push_back((int64_t)P->tasks.size());
-      P->pick.push_back(tensor_schur ? 2 : 3);
+      P->pick.push_back(2);      // complex64: the tuner's choice
       if (!tensor_schur) continue;
       // packed operands and the TMA kernels' tiles; slots that are mostly padding in
       // 128-row tiles stay on the SIMT kernel
@@ -2768,8 +2768,8 @@ struct Sweeper {
     return SS_OK;
   }
   // Schur update of slot q on the symmetric path with candidate c (complex64: 0 / 1 TMA
-  // tiles of 128 / 64 columns, 2 SIMT; complex128: one kernel)
-  void sym_schur(const Branch &br, int q, int c) {
+  // tiles of 128 / 64 columns, 2 SIMT; complex128: one kernel); returns its launches
+  int sym_schur(const Branch &br, int q, int c) {
     const FrontArgs<T> &a = br.a;
     const int nb = br.nb;
     const int64_t t0 = P.schur_ptr[q], t1 = P.schur_ptr[q + 1];
@@ -2781,11 +2781,12 @@ struct Sweeper {
         sym_schur_kernel<64><<<dim3((unsigned)(tm - t0), nb), 128, sym_schur_smem<64>(), br.st>>>(a, tasks + t0);
       if (t1 > tm)
         sym_schur_kernel<32><<<dim3((unsigned)(t1 - tm), nb), 128, sym_schur_smem<32>(), br.st>>>(a, tasks + tm);
+      return (tm > t0) + (t1 > tm);
     } else {
       if (c == 2 || !P.tma_ok || P.pk_ptr[q + 1] == P.pk_ptr[q]) {
         front_gemm_kernel<T, kSquare64, false, true>
             <<<grid, 256, gemm_cst_bytes<T, kSquare64>(), br.st>>>(a, tasks + t0);
-        return;
+        return 1;
       }
       const int64_t i0 = P.pi_ptr[q], i1 = P.pi_ptr[q + 1], q0 = P.tt_ptr[c][q], q1 = P.tt_ptr[c][q + 1];
       const int64_t *off = P.d_soff.template as<int64_t>();
@@ -2805,6 +2806,7 @@ struct Sweeper {
         tma(tc::tma_gemm_kernel<128, 2, true>, tc::TmaCfg<128, 2>::THREADS, tc::TmaCfg<128, 2>::SMEM);
       else
         tma(tc::tma_gemm_kernel<64, 3, true>, tc::TmaCfg<64, 3>::THREADS, tc::TmaCfg<64, 3>::SMEM);
+      return 2;      // with the packing
     }
   }
   // complex64: the fastest Schur candidate of each slot
@@ -2875,10 +2877,9 @@ struct Sweeper {
         if constexpr (sizeof(T) == 8) panel_launch<32>(br, q);
         if (P.schur_ptr[q + 1] == P.schur_ptr[q]) continue;
         SS_CK(cudaEventRecordWithFlags(ev[2 * nev], br.st, cudaEventRecordExternal));
-        sym_schur(br, q, P.pick[q]);
+        launches += sym_schur(br, q, P.pick[q]);
         SS_CK(cudaEventRecordWithFlags(ev[2 * nev + 1], br.st, cudaEventRecordExternal));
         ++nev;
-        ++launches;
         ++schur_launches;
       }
     SS_CK(cudaGetLastError());
@@ -3936,8 +3937,9 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
   h.st[26] = (double)P.fronts_small.size();
   h.st[27] = 0;
   for (float t : P.tune_ms) h.st[27] += t;
-  for (size_t l = 0; l < P.pick.size(); ++l)
-    if (P.schur_ptr[l + 1] > P.schur_ptr[l]) h.st[P.pick[l] == 3 ? 36 : 20 + P.pick[l]] += 1;
+  if (!(P.sym && sizeof(T) == 8))      // (the symmetric FP64 update has one kernel: nothing was picked)
+    for (size_t l = 0; l < P.pick.size(); ++l)
+      if (P.schur_ptr[l + 1] > P.schur_ptr[l]) h.st[P.pick[l] == 3 ? 36 : 20 + P.pick[l]] += 1;
   {
     double tot = 0;
     if (iters)
