@@ -229,20 +229,14 @@ __device__ __forceinline__ unsigned pivot_key(float v, int r) {
   return (__float_as_uint(v) & ~127u) | (unsigned)(127 - r);
 }
 // l = v / z for a pivot z with its key: conj(z) v times 1 / |z|^2, z scaled by the power of
-// two that brings |x| + |y| into [1, 2), so no square over- or underflows.  In FP64 the
-// reciprocal of |z|^2 comes from the hardware's approximation (about 2^-20) by one Halley
-// iteration (cubic: 2^-60).
+// two that brings |x| + |y| into [1, 2), so no square over- or underflows.
 struct PivotRecip {
   cd z;          // conj(scaled pivot)
   double g;      // scale / |scaled pivot|^2
   __device__ __forceinline__ PivotRecip(cd p, unsigned key) {
     const double r = __hiloint2double(min(max(2046 - (int)(key >> 20), 1), 2045) << 20, 0);
     z = cd{p.x * r, -p.y * r};
-    const double d = z.x * z.x + z.y * z.y;
-    double q;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(q) : "d"(d));
-    const double h = fma(-d, q, 1.0);
-    g = fma(q, fma(h, h, h), q) * r;
+    g = __drcp_rn(z.x * z.x + z.y * z.y) * r;
   }
   __device__ __forceinline__ cd recip() const { return cd{z.x * g, z.y * g}; }
   __device__ __forceinline__ cd times(cd v) const {
