@@ -2809,10 +2809,17 @@ struct Sweeper {
       return 2;      // with the packing
     }
   }
-  // complex64: the fastest Schur candidate of each slot
+  // complex64: the fastest Schur candidate of each slot, or SS_SYM_TILE_C64=0|1|2 where the
+  // slot has it (a measurement and test override, read once per plan)
   int sym_tune(int nb) {
     if (P.tuned) return SS_OK;
     const int ns = P.level_slot.back();
+    if (const char *e = getenv("SS_SYM_TILE_C64")) {
+      const int c = std::max(0, std::min(2, atoi(e)));
+      for (int q = 0; q < ns; ++q) P.pick[q] = (char)(P.tma_ok && P.pk_ptr[q + 1] > P.pk_ptr[q] ? c : 2);
+      P.tuned = true;
+      return SS_OK;
+    }
     std::vector<cudaEvent_t> e(2 * 3 * ns);
     for (auto &x : e) SS_CK(cudaEventCreate(&x));
     P.tune_ms.assign(3 * (size_t)ns, 0.f);
