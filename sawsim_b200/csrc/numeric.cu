@@ -2434,6 +2434,7 @@ int launch_condense(Handle &h) {
       vp[w * n + R + 1] = (int64_t)vs.size();
     }
   std::vector<int64_t> qp = {0, (int64_t)h.qz_src.size()};
+  h.dct_ptr.release();      // the transposed pattern is built again when it is asked for
   SS_CK(dupload(h.dc_ptr, h.c_ptr));
   SS_CK(dupload(h.dc_idx, h.c_idx));
   SS_CK(dupload(h.dg_ptr, gp));
@@ -3419,9 +3420,9 @@ static int build_transpose(Handle &h) {
       ti[q] = R;
       ts[q] = t;
     }
-  SS_CK(dupload(h.dct_ptr, tp));
   SS_CK(dupload(h.dct_idx, ti));
   SS_CK(dupload(h.dct_src, ts));
+  SS_CK(dupload(h.dct_ptr, tp));      // last: it tells that all three are there
   return SS_OK;
 }
 
