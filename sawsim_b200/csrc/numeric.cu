@@ -16,6 +16,7 @@
 #include <algorithm>
 #include <chrono>
 #include <limits>
+#include <memory>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -1955,9 +1956,12 @@ struct Plan {
   ~Plan() {
     for (auto &g : graphs)
       if (g.exec) cudaGraphExecDestroy(g.exec);
-    for (auto &e : ev) cudaEventDestroy(e);
-    for (auto &e : side_ev) cudaEventDestroy(e);
-    for (auto &st : side) cudaStreamDestroy(st);
+    for (auto &e : ev)
+      if (e) cudaEventDestroy(e);
+    for (auto &e : side_ev)
+      if (e) cudaEventDestroy(e);
+    for (auto &st : side)
+      if (st) cudaStreamDestroy(st);
   }
 };
 
@@ -3439,6 +3443,7 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
   for (int i = 0; i < n_f; ++i) wmax = std::max(wmax, std::fabs(omega[i]));
   const bool try_sym = !opt.general && sym_possible(h, sizeof(cplx<T>));
   if (h.scale_w != wmax || h.scale_tried != try_sym) {
+    h.scale_w = -1;      // an error on the way leaves no scaling that could be taken for a finished one
     bool sym = false;
     if (try_sym) {
       const int rc = equilibrate_sym(h, wmax, sym);
@@ -3454,8 +3459,9 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
   // plans by precision and by symmetry of the scaled system
   const int pi = (sizeof(T) == 8 ? 0 : 1) + (h.scale_sym ? 2 : 0);
   if (!h.plan[pi]) {
-    Plan *P = h.scale_sym ? build_sym_plan(h, sizeof(T) == 4) : build_plan(h, small_limit<T>(), sizeof(T) == 4);
-    h.plan[pi] = P;
+    // (the handle takes the plan when all of its device arrays are there)
+    std::unique_ptr<Plan> P(h.scale_sym ? build_sym_plan(h, sizeof(T) == 4)
+                                        : build_plan(h, small_limit<T>(), sizeof(T) == 4));
     SS_CK(dupload(P->d_small, P->fronts_small));
     SS_CK(dupload(P->d_large, P->fronts_large));
     SS_CK(dupload(P->d_tasks, P->tasks));
@@ -3551,6 +3557,7 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
       SS_CK(cudaFuncSetAttribute(front_tbwd_l21_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  std::min(vec, 223 * 1024)));
     }
+    h.plan[pi] = P.release();
   }
   Plan &P = *static_cast<Plan *>(h.plan[pi]);
   const int64_t W = S.relpos_ptr[S.nfront];
