@@ -2591,6 +2591,8 @@ static int equilibrate_sym(Handle &h, double w, bool &ok) {
   return SS_OK;
 }
 
+constexpr int kSmemMax = 227 * 1024;      // shared memory of one CTA
+
 // Shared memory, in elements, of the symmetric solve kernels on a level whose fronts have
 // at most k pivots and m rows: the widest staged block (sym_block is not monotone in k) and
 // one front's vector.
@@ -2614,14 +2616,14 @@ static bool sym_possible(const Handle &h, size_t eb) {
   const Symbolic &S = h.sym;
   for (int f = 0; f < S.nfront; ++f)
     if (S.child_ptr[f + 1] - S.child_ptr[f] > 2) return false;
-  if (sym_solve_elems(S.max_k, S.max_m) * eb > 227 * 1024)
+  if (sym_solve_elems(S.max_k, S.max_m) * eb > (size_t)kSmemMax)
     for (int l = 0; l < S.nlevel; ++l) {
       int k = 0, m = 0;
       for (int64_t q = S.level_ptr[l]; q < S.level_ptr[l + 1]; ++q) {
         k = std::max(k, S.k[S.level_fronts[q]]);
         m = std::max(m, S.m[S.level_fronts[q]]);
       }
-      if (sym_solve_elems(k, m) * eb > 227 * 1024) return false;
+      if (sym_solve_elems(k, m) * eb > (size_t)kSmemMax) return false;
     }
   return h.c_nnz < ((int64_t)1 << 31);
 }
@@ -3532,30 +3534,18 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
       SS_CK(dupload(P->d_tt[0], P->tt[0]));
       SS_CK(dupload(P->d_tt[1], P->tt[1]));
     }
-    // solve kernels stage a whole front vector in shared memory
-    // (the four triangular kernels also hold one staged 32x32 diagonal block)
-    const int vec = (int)std::min<int64_t>(227 * 1024, (int64_t)S.max_m * (int64_t)sizeof(cplx<T>));
-    const int vecd = (int)std::min<int64_t>(227 * 1024, vec + (int64_t)kDiagElems * sizeof(cplx<T>) +
-                                                           ((int64_t)std::max(1, S.max_k) * 4 + 15) / 16 * 16);
-    if (P->sym) {
-      const int sm = (int)std::min<size_t>(227 * 1024, sym_solve_elems(kNarrowK, S.max_m) * sizeof(cplx<T>));
-      SS_CK(cudaFuncSetAttribute(sym_fwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-      SS_CK(cudaFuncSetAttribute(sym_bwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-    }
-    if (vecd > 48 * 1024) {
-      SS_CK(cudaFuncSetAttribute(front_fwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, vecd));
-      SS_CK(cudaFuncSetAttribute(front_tfwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, vecd));
-      SS_CK(cudaFuncSetAttribute(front_bwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, vecd));
-      SS_CK(cudaFuncSetAttribute(front_tbwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, vecd));
-    }
-    if (vec > 48 * 1024) {
-      SS_CK(cudaFuncSetAttribute(front_fwd_l21_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, vec));
-      // (these two also hold an 8 x 32 static reduction tile)
-      SS_CK(cudaFuncSetAttribute(front_tfwd_u12_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 std::min(vec, 223 * 1024)));
-      SS_CK(cudaFuncSetAttribute(front_bwd_u12_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, vec));
-      SS_CK(cudaFuncSetAttribute(front_tbwd_l21_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 std::min(vec, 223 * 1024)));
+    // The solve kernels stage a whole front vector in shared memory.  A kernel's limit is
+    // shared by all engines of the process, so it is the device's, not this system's: an
+    // engine of smaller fronts must not lower it for one of larger fronts.
+    for (const void *k : {(const void *)sym_fwd_kernel<T>, (const void *)sym_bwd_kernel<T>,
+                          (const void *)front_fwd_kernel<T>, (const void *)front_tfwd_kernel<T>,
+                          (const void *)front_bwd_kernel<T>, (const void *)front_tbwd_kernel<T>,
+                          (const void *)front_fwd_l21_kernel<T>, (const void *)front_tfwd_u12_kernel<T>,
+                          (const void *)front_bwd_u12_kernel<T>, (const void *)front_tbwd_l21_kernel<T>}) {
+      cudaFuncAttributes fa;
+      SS_CK(cudaFuncGetAttributes(&fa, k));
+      SS_CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 kSmemMax - (int)fa.sharedSizeBytes));
     }
     h.plan[pi] = P.release();
   }
