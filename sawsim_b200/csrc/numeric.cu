@@ -2606,10 +2606,11 @@ static size_t sym_solve_elems(int k, int m) {
 // shared memory of one solve CTA beside a block (element size eb: 10,368 rows in complex128,
 // where the general solves go a little further), and no forced general
 // tile (SS_SCHUR_TILE, SS_SCHUR_TILE_C64: measurement and test overrides of the
-// general path; SS_SYMMETRIC=0 switches the symmetric path off).  A system whose
-// symmetric factors failed every point of a sweep (run_sweep) keeps to the general path.
+// general path; SS_SYMMETRIC=0 switches the symmetric path off).  A system that is not
+// symmetric, or whose symmetric factors failed every point of a sweep (run_sweep), keeps to
+// the general path until its values change.
 static bool sym_possible(const Handle &h, size_t eb) {
-  if (h.sym_weak) return false;
+  if (h.sym_off) return false;
   if (getenv("SS_SCHUR_TILE") || getenv("SS_SCHUR_TILE_C64")) return false;
   if (const char *e = getenv("SS_SYMMETRIC"))
     if (!atoi(e)) return false;
@@ -3444,7 +3445,7 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
   double wmax = 0;
   for (int i = 0; i < n_f; ++i) wmax = std::max(wmax, std::fabs(omega[i]));
   const bool try_sym = !opt.general && sym_possible(h, sizeof(cplx<T>));
-  if (h.scale_w != wmax || h.scale_tried != try_sym) {
+  if (h.scale_w != wmax || h.scale_sym != try_sym) {
     h.scale_w = -1;      // an error on the way leaves no scaling that could be taken for a finished one
     bool sym = false;
     if (try_sym) {
@@ -3455,8 +3456,11 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
       const int rc = equilibrate(h, wmax);
       if (rc) return rc;
     }
+    // Not tried again at the next top frequency: the scaling and its check took 1.7 of the
+    // 48.9 ms of a one-point solve of an unsymmetric 8x4x48 slab at a frequency of its own
+    // (8x1x12: 0.4 of 5.5 ms).
+    if (try_sym && !sym) h.sym_off = true;
     h.scale_sym = sym;
-    h.scale_tried = try_sym;
   }
   // plans by precision and by symmetry of the scaled system
   const int pi = (sizeof(T) == 8 ? 0 : 1) + (h.scale_sym ? 2 : 0);
@@ -4072,7 +4076,7 @@ int run_sweep(Handle &h, int n_f, const double *omega, double V, int precision, 
     if (rc) return rc;
     h.st[39] = points;
     if (mixed && !h.opt.fp64_fallback) h.st[32] = (double)std::count(status, status + n_f, SS_ENOCONV);
-    h.sym_weak = points == n_f;
+    h.sym_off = points == n_f;
   }
   h.st[17] += probe_ms;        // the probe is part of an AUTO sweep's device time
   h.st[15] += probe_launches;

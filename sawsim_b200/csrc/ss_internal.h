@@ -175,8 +175,7 @@ struct Handle {
   DBuf dmask;                            // per chunk frequency: still iterating in a Krylov loop
   double scale_w = -1;                   // frequency the scaling was computed at
   bool scale_sym = false;                // the scaled system is symmetric (the symmetric scaling was kept)
-  bool scale_tried = false;              // the symmetric scaling was tried
-  bool sym_weak = false;                 // every point of a sweep had to leave the symmetric path (run_sweep)
+  bool sym_off = false;                  // the symmetric path is not for these values (sym_possible)
   // solver options (ss_set_option); kept until changed
   struct Options {
     int krylov_m = 30;                   // FGMRES restart length of the mixed sweep
