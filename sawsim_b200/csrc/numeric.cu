@@ -1944,8 +1944,7 @@ struct Plan {
   std::vector<int64_t> schur_mid;          // per slot: end of its 64-column FP64 tiles (32-column ones follow)
   std::vector<int64_t> npiv_ptr[4], npan_ptr[2];
   std::vector<NarrowTask> npiv[4], npan[2];
-  std::vector<uint16_t> apos;
-  std::vector<int> aslot, imap;
+  std::vector<int> imap;
   std::vector<SymFront> sf;
   std::vector<int> wide, wide_ptr;         // fronts of more than one pivot block, by level
   // streams of the second and further groups of frequencies (Sweeper::branched)
@@ -2027,10 +2026,57 @@ constexpr int kGroup = 256;
 // 72.3, 71.4, 70.2, 70.2, 70.8; 16x64 ME0 (101 points) 13.0, 12.3, 12.2, 12.1, 12.1.
 constexpr int kShortUpdate = 128;
 
+// Arrowhead entries on and above the diagonal by bucket: a pivot block's F11, then its chunks
+// of cw columns of F12 (bucket: the block's first one, by block; blk: a front's first block),
+// each entry as its place in the bucket's tile and its slot.  One thread per entry; FILL
+// false counts the buckets into `cnt`, true takes places from it (in any order inside a
+// bucket: no two entries of one have the same position).  The first one-point solve on a
+// 64x256 ME1 cell, whose 16.8 million entries the host sorted before: 166 ms, now 38; 16x64
+// ME0 9.2 and 5.7 (the general path, which needs no buckets: 134 and 9.7).
+struct ArrowSplit {
+  int64_t n;
+  int nfront;
+  const int64_t *arrow_ptr, *arrow_slot;
+  const int32_t *arrow_pos;
+  const int *k, *m, *ld, *blk, *bucket;
+};
+template <class T, bool FILL>
+__global__ void __launch_bounds__(256)
+    split_arrows_kernel(ArrowSplit a, int *__restrict__ cnt, uint16_t *__restrict__ apos, int *__restrict__ aslot) {
+  const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  int b = -1, pos = 0;
+  if (e < a.n) {
+    int f = 0;                   // the last front whose entries start at e or before
+    for (int hi = a.nfront; hi - f > 1;) {
+      const int mid = (f + hi) / 2;
+      if (a.arrow_ptr[mid] <= e) f = mid; else hi = mid;
+    }
+    const int k = a.k[f], ld = a.ld[f], bs = sym_block(k), cw = panel_cols<T>(bs);
+    const int r = a.arrow_pos[e] / ld, c = a.arrow_pos[e] % ld;
+    if (r <= c) {
+      const int i = r / bs, b0 = bs * i, b1 = min(k, b0 + bs);
+      b = a.bucket[a.blk[f] + i] + (c < b1 ? 0 : 1 + (c - b1) / cw);
+      pos = (r - b0) * 64 + (c < b1 ? c - b0 : (c - b1) % cw);
+    }
+  }
+  // one atomic per bucket and warp
+  const unsigned peers = __match_any_sync(0xffffffffu, b);
+  const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
+  int at = 0;
+  if (lane == leader && b >= 0) at = atomicAdd(cnt + b, __popc(peers));
+  if (!FILL) return;
+  at = __shfl_sync(0xffffffffu, at, leader) + __popc(peers & ((1u << lane) - 1));
+  if (b >= 0) {
+    apos[at] = (uint16_t)pos;
+    aslot[at] = (int)a.arrow_slot[e];
+  }
+}
+
 // Launch plan of the symmetric path.
-Plan *build_sym_plan(Handle &h, bool tensor_schur) {
+template <class T>
+static int build_sym_plan(Handle &h, Plan *P) {
+  constexpr bool tensor_schur = sizeof(T) == 4;
   const Symbolic &S = h.sym;
-  Plan *P = new Plan();
   P->sym = true;
   P->tuned = !tensor_schur;
   for (int i = 0; i < S.max_m; ++i) P->imap.push_back(i);   // the identity map, at 0
@@ -2039,8 +2085,46 @@ Plan *build_sym_plan(Handle &h, bool tensor_schur) {
   for (auto *v : {&P->npiv_ptr[0], &P->npiv_ptr[1], &P->npiv_ptr[2], &P->npiv_ptr[3], &P->npan_ptr[0], &P->npan_ptr[1], &P->schur_ptr, &P->pk_ptr, &P->pi_ptr, &P->tt_ptr[0],
                   &P->tt_ptr[1]})
     v->assign(1, 0);
-  std::vector<int> key;
-  std::vector<int64_t> cnt;
+  // buckets of arrowhead entries, and the entries in their order
+  std::vector<int> blk(1, 0), bucket, bptr;
+  int nbucket = 0;
+  for (int f = 0; f < S.nfront; ++f) {
+    const int k = S.k[f], m = S.m[f], bs = sym_block(k), cw = panel_cols<T>(bs);
+    for (int b0 = 0; b0 < k; b0 += bs) {
+      bucket.push_back(nbucket);
+      nbucket += 1 + (m - std::min(k, b0 + bs) + cw - 1) / cw;
+    }
+    blk.push_back((int)bucket.size());
+  }
+  {
+    DBuf dblk, dbucket, dcnt;
+    SS_CK(dupload(dblk, blk, h.stream));
+    SS_CK(dupload(dbucket, bucket, h.stream));
+    SS_CK(dalloc(dcnt, (size_t)(nbucket + 1) * sizeof(int)));
+    SS_CK(cudaMemsetAsync(dcnt.p, 0, (size_t)(nbucket + 1) * sizeof(int), h.stream));
+    const ArrowSplit a{h.c_nnz, S.nfront, h.d_arrow_ptr.as<int64_t>(),
+                       h.d_arrow_slot.as<int64_t>(), h.d_arrow_pos.as<int32_t>(), h.d_k.as<int>(), h.d_m.as<int>(),
+                       h.d_ld.as<int>(), dblk.as<int>(), dbucket.as<int>()};
+    const unsigned grid = (unsigned)((h.c_nnz + 255) / 256);
+    split_arrows_kernel<T, false><<<grid, 256, 0, h.stream>>>(a, dcnt.as<int>(), nullptr, nullptr);
+    SS_CK(cudaGetLastError());
+    bptr.assign(nbucket + 1, 0);
+    SS_CK(cudaMemcpyAsync(bptr.data(), dcnt.p, (size_t)(nbucket + 1) * sizeof(int), cudaMemcpyDeviceToHost, h.stream));
+    SS_CK(cudaStreamSynchronize(h.stream));
+    int sum = 0;
+    for (int &c : bptr) {
+      const int n = c;
+      c = sum;
+      sum += n;
+    }
+    SS_CK(dalloc(P->d_apos, (size_t)sum * sizeof(uint16_t) + 16));
+    SS_CK(dalloc(P->d_aslot, (size_t)sum * sizeof(int) + 16));
+    SS_CK(cudaMemcpyAsync(dcnt.p, bptr.data(), (size_t)(nbucket + 1) * sizeof(int), cudaMemcpyHostToDevice, h.stream));
+    split_arrows_kernel<T, true><<<grid, 256, 0, h.stream>>>(a, dcnt.as<int>(), P->d_apos.as<uint16_t>(),
+                                                          P->d_aslot.as<int>());
+    SS_CK(cudaGetLastError());
+    SS_CK(cudaStreamSynchronize(h.stream));      // the buffers above go
+  }
   std::vector<std::vector<NarrowTask>> piv;
   std::vector<std::vector<std::pair<NarrowTask, int>>> pan;      // with the chunk width
   // Schur updates of a step: pivot block (or group), last row and last column
@@ -2059,41 +2143,12 @@ Plan *build_sym_plan(Handle &h, bool tensor_schur) {
       lu = std::max(lu, m - k);
       lm = std::max(lm, m);
       const int bs = sym_block(k), nblk = (k + bs - 1) / bs;
-      const int cw = tensor_schur ? panel_cols<float>(bs) : panel_cols<double>(bs);   // chunk width
+      const int cw = panel_cols<T>(bs);
       steps = std::max(steps, nblk);
       if (nblk > 1) P->wide.push_back(f);
       if ((int)piv.size() < nblk) piv.resize(nblk), pan.resize(nblk), upd.resize(nblk);
       const int ng = std::max(1, kGroup / bs);      // blocks per group
       int group0 = 0;                               // first block of the group, as an index into P->sf
-      // arrowhead entries on and above the diagonal, by block and 64-column chunk
-      std::vector<int> chunk0(nblk + 1, 0);      // first bucket of each block (F11, then its chunks)
-      for (int i = 0; i < nblk; ++i) {
-        const int b1 = std::min(k, bs * (i + 1));
-        chunk0[i + 1] = chunk0[i] + 1 + (m - b1 + cw - 1) / cw;
-      }
-      const int64_t e0 = S.arrow_ptr[f], e1 = S.arrow_ptr[f + 1];
-      key.assign((size_t)(e1 - e0), -1);
-      cnt.assign((size_t)chunk0[nblk] + 1, 0);
-      for (int64_t e = e0; e < e1; ++e) {
-        const int r = S.arrow_pos[e] / ld, c = S.arrow_pos[e] % ld;
-        if (r > c) continue;
-        const int i = r / bs, b1 = std::min(k, bs * (i + 1));
-        key[e - e0] = chunk0[i] + (c < b1 ? 0 : 1 + (c - b1) / cw);
-        ++cnt[key[e - e0] + 1];
-      }
-      for (size_t i = 0; i + 1 < cnt.size(); ++i) cnt[i + 1] += cnt[i];
-      const int64_t a0 = (int64_t)P->apos.size();
-      P->apos.resize(a0 + cnt.back());
-      P->aslot.resize(a0 + cnt.back());
-      std::vector<int64_t> fill(cnt.begin(), cnt.end());
-      for (int64_t e = e0; e < e1; ++e) {
-        if (key[e - e0] < 0) continue;
-        const int r = S.arrow_pos[e] / ld, c = S.arrow_pos[e] % ld;
-        const int i = r / bs, b0 = bs * i, b1 = std::min(k, b0 + bs);
-        const int64_t at = a0 + fill[key[e - e0]]++;
-        P->apos[at] = (uint16_t)((r - b0) * 64 + (c < b1 ? c - b0 : (c - b1) % cw));
-        P->aslot[at] = (int)S.arrow_slot[e];
-      }
       for (int i = 0; i < nblk; ++i) {
         const int b0 = bs * i, b1 = std::min(k, b0 + bs), id = (int)P->sf.size();
         SymFront s{};
@@ -2120,10 +2175,10 @@ Plan *build_sym_plan(Handle &h, bool tensor_schur) {
           s.imap[0] = 0;
         }
         P->sf.push_back(s);
-        const int64_t *cp = &cnt[chunk0[i]];
-        piv[i].push_back(NarrowTask{id, -1, (int)(a0 + cp[0]), (int)(a0 + cp[1])});
+        const int *cp = &bptr[bucket[blk[f] + i]];
+        piv[i].push_back(NarrowTask{id, -1, cp[0], cp[1]});
         for (int c = 0; c < (s.m - s.k + cw - 1) / cw; ++c)
-          pan[i].push_back({NarrowTask{id, cw * c, (int)(a0 + cp[1 + c]), (int)(a0 + cp[2 + c])}, cw});
+          pan[i].push_back({NarrowTask{id, cw * c, cp[1 + c], cp[2 + c]}, cw});
         if (i % ng == 0) group0 = id;
         const bool last = i + 1 == nblk || (i + 1) % ng == 0;
         const int g0 = i / ng * ng * bs, g1 = std::min(k, g0 + ng * bs);     // the group's pivots
@@ -2211,7 +2266,7 @@ Plan *build_sym_plan(Handle &h, bool tensor_schur) {
     }
     P->level_slot.push_back(P->level_slot.back() + steps);
   }
-  return P;
+  return SS_OK;
 }
 
 Plan *build_plan(Handle &h, int small_m, bool tensor_schur) {
@@ -3466,8 +3521,11 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
   const int pi = (sizeof(T) == 8 ? 0 : 1) + (h.scale_sym ? 2 : 0);
   if (!h.plan[pi]) {
     // (the handle takes the plan when all of its device arrays are there)
-    std::unique_ptr<Plan> P(h.scale_sym ? build_sym_plan(h, sizeof(T) == 4)
-                                        : build_plan(h, small_limit<T>(), sizeof(T) == 4));
+    std::unique_ptr<Plan> P(h.scale_sym ? new Plan() : build_plan(h, small_limit<T>(), sizeof(T) == 4));
+    if (h.scale_sym) {
+      const int rc = build_sym_plan<T>(h, P.get());
+      if (rc) return rc;
+    }
     SS_CK(dupload(P->d_small, P->fronts_small));
     SS_CK(dupload(P->d_large, P->fronts_large));
     SS_CK(dupload(P->d_tasks, P->tasks));
@@ -3514,8 +3572,6 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
       SS_CK(dupload(P->d_imap, P->imap));
       for (int c = 0; c < 4; ++c) SS_CK(dupload(P->d_npiv[c], P->npiv[c]));
       for (int c = 0; c < 2; ++c) SS_CK(dupload(P->d_npan[c], P->npan[c]));
-      SS_CK(dupload(P->d_apos, P->apos));
-      SS_CK(dupload(P->d_aslot, P->aslot));
       SS_CK(cudaFuncSetAttribute(sym_pivot_kernel<T, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)pivot_smem<T>(64)));
       SS_CK(cudaFuncSetAttribute(sym_panel_kernel<T, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
