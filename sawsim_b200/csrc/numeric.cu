@@ -2694,8 +2694,8 @@ static int equilibrate(Handle &h, double w) {
   SS_CK(dalloc(rmax, n * sizeof(double)));
   SS_CK(dalloc(cmax, n * sizeof(unsigned long long)));
   std::vector<double> ones(n, 1.0);
-  SS_CK(cudaMemcpy(h.drow_scale.p, ones.data(), n * sizeof(double), cudaMemcpyHostToDevice));
-  SS_CK(cudaMemcpy(h.dcol_scale.p, ones.data(), n * sizeof(double), cudaMemcpyHostToDevice));
+  SS_CK(cudaMemcpyAsync(h.drow_scale.p, ones.data(), n * sizeof(double), cudaMemcpyHostToDevice, h.stream));
+  SS_CK(cudaMemcpyAsync(h.dcol_scale.p, ones.data(), n * sizeof(double), cudaMemcpyHostToDevice, h.stream));
   const cd *D = h.have_D && h.beta ? h.dDc.as<cd>() : nullptr;
   for (int it = 0; it < 3; ++it) {
     row_absmax_kernel<<<nb, 256, 0, h.stream>>>(n, h.dc_ptr.as<int64_t>(), h.dc_idx.as<int64_t>(), h.dKc.as<cd>(),
@@ -3685,7 +3685,7 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
     // frequencies still iterating in the Krylov loops (read by the solve kernels)
     SS_CK(dalloc(h.dmask, (size_t)B * sizeof(int)));
     std::vector<int> ones(B, 1);
-    SS_CK(cudaMemcpy(h.dmask.p, ones.data(), (size_t)B * sizeof(int), cudaMemcpyHostToDevice));
+    SS_CK(cudaMemcpyAsync(h.dmask.p, ones.data(), (size_t)B * sizeof(int), cudaMemcpyHostToDevice, h.stream));
   }
   DBuf &tcerr = h.wk[13];
   SS_CK(dalloc(tcerr, sizeof(int)));

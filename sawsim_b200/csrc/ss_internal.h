@@ -57,8 +57,11 @@ cudaError_t dalloc(DBuf &b, size_t bytes);
 template <class T>
 cudaError_t dupload(DBuf &b, const std::vector<T> &v) {
   cudaError_t e = dalloc(b, v.size() * sizeof(T) + 16);
-  if (e != cudaSuccess) return e;
-  return v.empty() ? cudaSuccess : cudaMemcpy(b.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
+  if (e != cudaSuccess || v.empty()) return e;
+  // A copy from pageable memory returns when its source is staged, which may be before it has
+  // arrived, and the handle's stream does not wait for the default one.
+  e = cudaMemcpy(b.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
+  return e != cudaSuccess ? e : cudaStreamSynchronize(cudaStreamLegacy);
 }
 
 // the same in the stream's order (the host vector may go once this returns)
