@@ -2606,8 +2606,11 @@ static int scale_values(Handle &h) {
 }
 
 // Symmetric equilibration at angular frequency w (sym_scale.cuh); `ok` tells whether
-// the scaled system is symmetric to kSymTol (entries are at most about 1).
-constexpr double kSymTol = 1e-13;
+// the scaled system is symmetric to kSymTol (entries are at most about 1).  The tolerance is
+// that of rounding: 40 cells and stacks are at 4.5e-16 or below, their electrode rows against
+// its columns at 1.9e-15.  A system that is symmetric to 1e-13 only would keep that as the
+// error of an adjoint taken from the primal solution, times its condition.
+constexpr double kSymTol = 4e-15;
 static int equilibrate_sym(Handle &h, double w, bool &ok) {
   const int64_t n = h.sym.n;
   const unsigned nb = (unsigned)((n + 255) / 256), wb = (unsigned)((n + 7) / 8);
