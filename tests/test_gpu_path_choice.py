@@ -1,6 +1,8 @@
 """Which path an engine takes follows its values: a system found unsymmetric keeps to the
 general path at other top frequencies too, and takes the symmetric one when its values
-become symmetric again.  The charges are those of a fresh engine, bit for bit."""
+become symmetric again.  The charges are those of a fresh engine: on the symmetric path bit for
+bit, on the general one, whose tuner may pick other tiles for another engine, to 1e-7 (the
+bar of the oracle comparisons)."""
 import numpy as np
 import pytest
 
@@ -35,10 +37,10 @@ def test_the_path_follows_the_values(built_lib):
         f.close()
     e = FrequencySolver.from_matrices(U, M, *c.bc)
     try:
-        assert np.array_equal(charges(e, False), fresh['U'])
+        assert np.max(np.abs(charges(e, False) - fresh['U']) / np.abs(fresh['U'])) < 1e-7
         e.update_matrices(K, M)
         assert np.array_equal(charges(e, True), fresh['K'])
         e.update_matrices(U, M)
-        assert np.array_equal(charges(e, False), fresh['U'])
+        assert np.max(np.abs(charges(e, False) - fresh['U']) / np.abs(fresh['U'])) < 1e-7
     finally:
         e.close()
