@@ -2017,7 +2017,10 @@ static void add_upper_tiles(std::vector<GemmTask> &v, int bm, int bn, int f, int
 // Pivot blocks are grouped kGroup pivots at a time: a block updates only the rows of its
 // group (the next blocks need them), the rest of the front gets the whole group at once.
 // The trailing block is then read and written once per group instead of once per block,
-// with a four times longer K loop behind each tile's epilogue.
+// with a four times longer K loop behind each tile's epilogue.  Groups of 64 (no groups), 128,
+// 256 and 512 pivots, milliseconds on the device: 64x256 ME1 (11 points) 74.8, 71.3, 70.3, 70.4;
+// 32x128 ME1 (51) 54.7, 53.2, 53.0, 53.0; 8x2x26 FP64 (33) 20.3, 19.2, 18.9, 19.0; 8x4x48 mixed
+// (16) 77.5, 65.9, 60.5, 63.1 (longer groups leave more of the update to the in-group tiles).
 constexpr int kGroup = 256;
 // FP64 updates of at most so many pivots take 32 x 32 tiles, longer ones 32 x 64: a short
 // product waits for its sources and operands, not for the tensor cores, so more and smaller
@@ -2239,7 +2242,8 @@ static int build_sym_plan(Handle &h, Plan *P) {
       P->pick.push_back(2);      // complex64: the tuner's choice
       if (!tensor_schur) continue;
       // packed operands and the TMA kernels' tiles; slots that are mostly padding in
-      // 128-row tiles stay on the SIMT kernel
+      // 128-row tiles stay on the SIMT kernel (the line at 1.5, 2.5 and 6 times the work:
+      // 8x4x48 at 16 points 61.5, 60.5, 60.5 ms, where the tuner has the last word)
       int64_t rows = 0;
       for (const Update &t : upd[i]) {
         if (padded > 2.5 * work) break;

@@ -15,6 +15,8 @@
 //     F11 and F12 when they are assembled, F22 in the epilogue of the Schur update, so
 //     F22 is written once and never zeroed, scattered into or copied.  The later blocks
 //     read the front itself, in place, through the identity map: the same kernels.
+// Pivots are searched inside a block only; points whose factors show that (run_sweep) are
+// solved again on the general path, which searches all of a front's pivot rows.
 // The maps are monotone, so upper entries come from upper entries.  A front's memory
 // holds, for every pivot block, L and U of F11 in pivot order, U12 right of it and L21
 // below it (its rows in front order): the row interchanges of a later block are not
@@ -34,9 +36,12 @@ namespace ss {
 // and the K loop its last half chunk when that is empty.
 //   32 x 32, for short products: four CTAs per SM, the first operands are asked for before the
 // sources' row maps, and the second source's entries with the first ones.
-//   32 x 64: 96 accumulator registers, three CTAs per SM.  64 x 64 tiles (two CTAs) wait
-// for C more and leave more of a diagonal tile unused: 40.2 against 33.7 ms for the updates
-// of the 64x256 ME1 cell at 11 points, 10.5 against 8.6 ms for the 8x2x26 Hex27 slab at 33.
+// Launches one at a time: 0.40 of the byte and operation bound on 16x64 ME0 (101 points, every
+// update short), 0.55 on 32x128 ME1 (51 points).
+//   32 x 64: 96 accumulator registers, three CTAs per SM; 0.75 of that bound on 32x128 ME1.
+// 64 x 64 tiles (two CTAs) wait for C more and leave more of a diagonal tile unused: 40.2
+// against 33.7 ms for the updates of the 64x256 ME1 cell at 11 points, 10.5 against 8.6 ms
+// for the 8x2x26 Hex27 slab at 33.
 template <int BN>
 constexpr int sym_schur_smem() { return 32 * (BN + 1) * (int)sizeof(cd); }
 template <int BN>
@@ -481,6 +486,8 @@ __device__ __forceinline__ int block_lu(cplx<T> *W, int ks, int k, T tiny, int *
   return npert;
 }
 
+// (In complex128 with KMAX = 64 the 168 registers of three CTAs per SM spill 228 bytes of
+// stores and 276 of loads per thread.)
 template <class T, int KMAX>
 __global__ void __launch_bounds__(2 * KMAX, KMAX == 64 ? 3 : KMAX == 48 ? 4 : KMAX == 32 ? 8 : 12)
     sym_pivot_kernel(FrontArgs<T> a, const NarrowTask *__restrict__ tasks, int nb, const uint16_t *__restrict__ apos,
@@ -762,7 +769,10 @@ __device__ __forceinline__ void panel_simt(const cf *A, int ks, cf *Y, int CS, i
 
 // Four warps for L21 and four for U12 of the same chunk.  (Four warps that solved one after
 // the other, with P F12 through global memory: 45.5 against 42.6 ms for the factorisation of
-// the 32x128 ME1 cell at 51 points, where complex128 keeps its rows in registers too.)
+// the 32x128 ME1 cell at 51 points, where complex128 keeps its rows in registers too.)  In
+// complex128 with 64 columns the 128 registers of two CTAs per SM spill 264 bytes of stores
+// and 292 of loads per thread.  Launches one at a time: 6.8 ms for the 64-column chunks of that
+// sweep and 6.6 for the 32-column ones, 3.4 and 2.6 times what their bytes or operations take.
 constexpr int kPanelThreadsSym = 256;
 // chunk width and padded sizes: the tile and F11 of one chunk leave room for at least two
 // CTAs per SM (complex128, 64 pivots: 104 KB at 32 columns; 64 would take 137)

@@ -539,8 +539,9 @@ namespace ss {
 // half of its fronts (separators of 13-25 pivots with 270-420 update rows): 8x4x48
 // goes from 1192 to 588 fronts, 14 to 10 levels and 306M to 206M front elements per
 // point.  At most kMergePivots pivots: beyond that the panel chain of the dense
-// diagonal block grows faster than the traffic saved (every chain of these slabs ends
-// below it).
+// diagonal block grows faster than the traffic saved.  The line at 0, 128, 256 and 512:
+// 8x2x26 FP64 (33 points) 20.4, 19.1, 18.9, 18.9 ms; 8x4x48 mixed (16) 65.1, 60.5, 60.5, 60.5;
+// four-layer 12x4x48 mixed (6) 55.8, 54.0, 54.0, 54.1 (few chains reach 256 there).
 constexpr int64_t kMergePivots = 256;
 static void merge_only_children(ND &nd, const std::vector<int64_t> &ap, const std::vector<int64_t> &aj,
                                 const std::vector<int64_t> &svp, int64_t nsv) {
