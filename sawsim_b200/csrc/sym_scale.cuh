@@ -118,16 +118,17 @@ __global__ void sym_cols_kernel(int64_t n, const double *__restrict__ t, const d
   if (R < n) cs[R] = t[R] * d[R];
 }
 
-// flag != 0 when some scaled entry pair differs by more than tol: |K'_ij - K'_ji| +
-// w2 |M'_ij - M'_ji| (+ wb |D'|), entries without a mirrored slot against zero
+// asym: the largest |K'_ij - K'_ji| + w2 |M'_ij - M'_ji| (+ wb |D'|) over the scaled entry
+// pairs, entries without a mirrored slot against zero, as the bits of a double (they order as
+// the non-negative numbers do; infinite where a difference is not a number)
 __global__ void __launch_bounds__(256) sym_check_kernel(int64_t n, const int64_t *__restrict__ rp,
                                                         const int64_t *__restrict__ ci, const cd *__restrict__ K,
                                                         const cd *__restrict__ M, const cd *__restrict__ D, double w2,
-                                                        double wb, double tol, int *__restrict__ flag) {
+                                                        double wb, unsigned long long *__restrict__ asym) {
   const int64_t R = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (R >= n) return;
-  bool bad = false;
+  double worst = 0.0;
   for (int64_t q = rp[R] + lane; q < rp[R + 1]; q += 32) {
     const int64_t C = ci[q];
     if (C == R) continue;
@@ -136,9 +137,11 @@ __global__ void __launch_bounds__(256) sym_check_kernel(int64_t n, const int64_t
     const cd z{0.0, 0.0};
     double e = sqrt(cabs2(K[q] - (p >= 0 ? K[p] : z))) + w2 * sqrt(cabs2(M[q] - (p >= 0 ? M[p] : z)));
     if (D) e += wb * sqrt(cabs2(D[q] - (p >= 0 ? D[p] : z)));
-    bad = bad || !(e <= tol);
+    worst = fmax(worst, e == e ? e : INFINITY);
   }
-  if (__any_sync(0xffffffffu, bad) && lane == 0) *flag = 1;
+  for (int o = 16; o > 0; o >>= 1) worst = fmax(worst, __shfl_xor_sync(0xffffffffu, worst, o));
+  const unsigned long long bits = (unsigned long long)__double_as_longlong(worst);
+  if (lane == 0 && bits > *asym) atomicMax(asym, bits);
 }
 
 }  // namespace ss
