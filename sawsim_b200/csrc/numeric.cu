@@ -1849,8 +1849,10 @@ __global__ void charge_row_kernel(int64_t n, int nb, const cd *__restrict__ kq, 
 
 // x += dx and per-frequency max |dx|, max |x| (for the refinement stopping test); grid (8, nb)
 __global__ void __cluster_dims__(kRedCtas, 1, 1) __launch_bounds__(kRedThreads)
-    axpy_norm_kernel(int64_t n, cd *__restrict__ x, const cd *__restrict__ dx, double *__restrict__ nrm) {
+    axpy_norm_kernel(int64_t n, cd *__restrict__ x, const cd *__restrict__ dx, double *__restrict__ nrm,
+                     const int *__restrict__ active = nullptr) {
   const int f = blockIdx.y;
+  if (active && !active[f]) return;
   cd mx{0.0, 0.0};
   SS_RED_LOOP(R, n) {
     const int64_t t = (int64_t)f * n + R;
@@ -2671,10 +2673,11 @@ static size_t sym_solve_elems(int k, int m) {
 // where the general solves go a little further), and no forced general
 // tile (SS_SCHUR_TILE, SS_SCHUR_TILE_C64: measurement and test overrides of the
 // general path; SS_SYMMETRIC=0 switches the symmetric path off).  A system that is not
-// symmetric, or whose symmetric factors failed every point of a sweep (run_sweep), keeps to
-// the general path until its values change.
-static bool sym_possible(const Handle &h, size_t eb) {
-  if (h.sym_off) return false;
+// symmetric, or whose symmetric factors failed most points of a call (run_sweep), keeps to the
+// general path until its values change: for calls of that use (charges, or fields: kUse*).
+constexpr int kUseCharges = 1, kUseFields = 2;
+static bool sym_possible(const Handle &h, size_t eb, int use) {
+  if (h.sym_off & use) return false;
   if (getenv("SS_SCHUR_TILE") || getenv("SS_SCHUR_TILE_C64")) return false;
   if (const char *e = getenv("SS_SYMMETRIC"))
     if (!atoi(e)) return false;
@@ -3508,7 +3511,8 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
   const int64_t n = S.n;
   double wmax = 0;
   for (int i = 0; i < n_f; ++i) wmax = std::max(wmax, std::fabs(omega[i]));
-  const bool try_sym = !opt.general && sym_possible(h, sizeof(cplx<T>));
+  const bool fields = disp || (ex && ex->per_chunk);     // the solutions themselves are asked for
+  const bool try_sym = !opt.general && sym_possible(h, sizeof(cplx<T>), fields ? kUseFields : kUseCharges);
   if (h.scale_w != wmax || h.scale_sym != try_sym) {
     h.scale_w = -1;      // an error on the way leaves no scaling that could be taken for a finished one
     bool sym = false;
@@ -3523,7 +3527,7 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
     // Not tried again at the next top frequency: the scaling and its check took 1.7 of the
     // 48.9 ms of a one-point solve of an unsymmetric 8x4x48 slab at a frequency of its own
     // (8x1x12: 0.4 of 5.5 ms).
-    if (try_sym && !sym) h.sym_off = true;
+    if (try_sym && !sym) h.sym_off = kUseCharges | kUseFields;
     h.scale_sym = sym;
   }
   // plans by precision and by symmetry of the scaled system
@@ -3774,6 +3778,64 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
     return SS_OK;
   };
   const unsigned vb = (unsigned)((n + 255) / 256);
+  auto residual = [&](int nb) {
+    spmv_kernel<<<dim3(spmv_rows(n), spmv_blocks(nb)), 256, 0, h.stream>>>(
+        n, nb, h.dc_ptr.as<int64_t>(), h.dc_idx.as<int64_t>(), nullptr, a.Kc, a.Mc, a.Dc, dom.as<double>(), h.beta,
+        b.as<cd>(), x.as<cd>(), r.as<cd>());
+  };
+  // A weak point's charge can still be good: the part of the solution that the factors miss is a
+  // nearly singular mode without charge (the 128x512 ME1 cell: fields wrong by their own size,
+  // charges by 7e-9).  With the adjoint mu = s x (below), Q + mu^T (b - A' x) is exact up to the
+  // product of two errors.  It is taken before and after one more refinement step; points whose
+  // two values agree to 1e-10 keep the second one (its correction goes to corr) and are no
+  // longer weak.
+  auto weak_charges = [&](int nb, std::vector<cd> &corr) -> int {
+    if (std::find(weak.begin(), weak.begin() + nb, 1) == weak.begin() + nb || h.scale_asym > kRoundTol) return SS_OK;
+    std::vector<cd> sc(nb), q[2], d[2];
+    std::vector<double> off(2 * nb);
+    charge_row_kernel<<<dim3(vb, nb), 256, 0, h.stream>>>(n, nb, h.dks.as<cd>() + n, h.dcol_scale.as<double>(),
+                                                        dx.as<cd>());
+    ratio_kernel<<<dim3(kRedCtas, nb), kRedThreads, 0, h.stream>>>(n, b.as<cd>(), dx.as<cd>(), dQ.as<cd>());
+    ratio_check_kernel<<<dim3(kRedCtas, nb), kRedThreads, 0, h.stream>>>(n, b.as<cd>(), dx.as<cd>(), dQ.as<cd>(),
+                                                                        nrm.as<double>());
+    SS_CK(cudaMemcpyAsync(sc.data(), dQ.p, nb * sizeof(cd), cudaMemcpyDeviceToHost, h.stream));
+    SS_CK(cudaMemcpyAsync(off.data(), nrm.p, 2 * nb * sizeof(double), cudaMemcpyDeviceToHost, h.stream));
+    std::vector<int> on(weak.begin(), weak.begin() + nb);
+    SS_CK(cudaMemcpyAsync(h.dmask.p, on.data(), nb * sizeof(int), cudaMemcpyHostToDevice, h.stream));
+    for (int i = 0; i < 2; ++i) {
+      if (i) {
+        const int rc = sw.solve_graphed(1, nb, r.as<cd>(), dx.as<cd>());
+        if (rc) return rc;
+        axpy_norm_kernel<<<dim3(kRedCtas, nb), kRedThreads, 0, h.stream>>>(n, x.as<cd>(), dx.as<cd>(), nrm.as<double>(),
+                                                                          h.dmask.as<int>());
+      }
+      residual(nb);
+      charge_kernel<<<dim3(kRedCtas, nb), kRedThreads, 0, h.stream>>>(
+          n, h.dks.as<cd>() + n, h.dcol_scale.as<double>(), x.as<cd>(), h.dQz.as<cd>(), V, dQ.as<cd>());
+      dotu_kernel<<<dim3(kRedCtas, nb), kRedThreads, 0, h.stream>>>(n, x.as<cd>(), r.as<cd>(), dQ.as<cd>() + B);
+      q[i].resize(nb);
+      d[i].resize(nb);
+      SS_CK(cudaMemcpyAsync(q[i].data(), dQ.p, nb * sizeof(cd), cudaMemcpyDeviceToHost, h.stream));
+      SS_CK(cudaMemcpyAsync(d[i].data(), dQ.as<cd>() + B, nb * sizeof(cd), cudaMemcpyDeviceToHost, h.stream));
+    }
+    std::fill(on.begin(), on.end(), 1);
+    SS_CK(cudaMemcpyAsync(h.dmask.p, on.data(), nb * sizeof(int), cudaMemcpyHostToDevice, h.stream));
+    SS_CK(cudaGetLastError());
+    SS_CK(cudaStreamSynchronize(h.stream));
+    for (int f = 0; f < nb; ++f) {
+      if (!weak[f]) continue;
+      ++hit[f];
+      const cd d1 = cmul(sc[f], d[1][f]), v = q[1][f] + d1, e = v - (q[0][f] + cmul(sc[f], d[0][f]));
+      if (off[2 * f] <= kRoundTol * off[2 * f + 1] && cabs2(e) <= 1e-20 * cabs2(v)) {
+        weak[f] = 0;
+        corr[f] = d1;
+      }
+      if (getenv("SS_DEBUG_IR"))
+        fprintf(stderr, "point %d: charge moves by %.2e, its correction is %.2e%s\n", f, std::sqrt(cabs2(e) / cabs2(v)),
+                std::sqrt(cabs2(d1) / cabs2(v)), weak[f] ? " (weak)" : "");
+    }
+    return SS_OK;
+  };
   auto t_start = std::chrono::steady_clock::now();
   cudaEvent_t eall0, eall1;
   cudaEventCreate(&eall0);
@@ -3831,9 +3893,7 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
               q[0] / q[nb], q[nb - 1] / q[2 * nb - 1]);
     }
     for (int it = 0; it < (use_krylov ? 0 : maxit); ++it) {
-      spmv_kernel<<<dim3(spmv_rows(n), spmv_blocks(nb)), 256, 0, h.stream>>>(
-          n, nb, h.dc_ptr.as<int64_t>(), h.dc_idx.as<int64_t>(), nullptr, a.Kc, a.Mc, a.Dc, dom.as<double>(), h.beta, b.as<cd>(),
-                                                          x.as<cd>(), r.as<cd>());
+      residual(nb);
       rc = sw.solve_graphed(1, nb, r.as<cd>(), dx.as<cd>());
       if (rc) return rc;
       axpy_norm_kernel<<<dim3(kRedCtas, nb), kRedThreads, 0, h.stream>>>(n, x.as<cd>(), dx.as<cd>(), nrm.as<double>());
@@ -3855,12 +3915,13 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
       }
       if (all) break;
     }
+    std::vector<cd> corr(nb, cd{0.0, 0.0});
     if (P.sym && sizeof(T) == 8 && !use_krylov) {
       rc = mark_weak(nb, hn.data(), r.as<cd>(), x.as<cd>());
+      if (!rc && !fields) rc = weak_charges(nb, corr);
       if (rc) return rc;
     }
     // adjoint of the charge functional: A'^T mu = c with c = cs * kq (Q = c^T x' + V Qz)
-    std::vector<cd> corr(nb, cd{0.0, 0.0});
     std::vector<char> aconv(nb, 1);
     if (need_adjoint) {
       charge_row_kernel<<<dim3(vb, nb), 256, 0, h.stream>>>(n, nb, h.dks.as<cd>() + n, h.dcol_scale.as<double>(),
@@ -3941,10 +4002,8 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
     SS_CK(cudaStreamSynchronize(h.stream));
     for (int f = 0; f < nb; ++f) {
       perturbed += hp[f];
-      if (correct) {
-        Qout[2 * (int64_t)(c0 + f)] += corr[f].x;
-        Qout[2 * (int64_t)(c0 + f) + 1] += corr[f].y;
-      }
+      Qout[2 * (int64_t)(c0 + f)] += corr[f].x;
+      Qout[2 * (int64_t)(c0 + f) + 1] += corr[f].y;
       const bool ok = !(sizeof(T) == 4 && !(conv[f] && aconv[f]));
       nfail += !ok;
       // singular: a non-finite charge, or (FP64 direct solve) statically
@@ -4044,7 +4103,9 @@ static int sweep_impl(Handle &h, int n_f, const double *omega, double V, double 
 // can grow on the first and not on the second.  Points that show it (sweep_impl: their
 // residuals, non-finite or singular results; without fp64_fallback also mixed points that did
 // not converge) are solved again on the general path in the same call.  A system that
-// needed it at every point of a sweep goes there directly until its values change.
+// needed it at most points of a call goes there directly until its values change.  The large
+// cells do too where fields are asked for: their nearly singular mode (128x512 ME1: a
+// condition of some 1e11) comes out wrong by up to its own size otherwise.
 int run_sweep(Handle &h, int n_f, const double *omega, double V, int precision, double *Q, int *status,
               int *iters, double *disp_out, const SweepExtra *ex) {
   SweepOpts opt;
@@ -4141,11 +4202,15 @@ int run_sweep(Handle &h, int n_f, const double *omega, double V, int precision, 
   if (std::find(weak.begin(), weak.end(), 1) != weak.end()) {
     double ms = 0;
     int points = 0;
+    // when most points need it all are solved there, and later calls go there directly: the
+    // same call then returns the same bits
+    const bool most = !(mixed && h.opt.fp64_fallback) && 2 * std::count(weak.begin(), weak.end(), 1) > n_f;
+    if (most) std::fill(weak.begin(), weak.end(), 1);
     rc = again(weak, mixed && !h.opt.fp64_fallback, true, ms, points);
     if (rc) return rc;
     h.st[39] = points;
     if (mixed && !h.opt.fp64_fallback) h.st[32] = (double)std::count(status, status + n_f, SS_ENOCONV);
-    h.sym_off = points == n_f;
+    if (most) h.sym_off |= disp_out || (ex && ex->per_chunk) ? kUseFields : kUseCharges;
   }
   h.st[17] += probe_ms;        // the probe is part of an AUTO sweep's device time
   h.st[15] += probe_launches;

@@ -69,7 +69,7 @@ extern "C" const char *ss_last_error(const ss_handle *hp) { return hp ? hp->h.er
 // what was kept for the old values: the scaling, the choice of path and SS_PREC_AUTO's
 static void new_values(Handle &h) {
   h.scale_w = -1;
-  h.sym_off = false;
+  h.sym_off = 0;
   h.auto_prec = -1;
 }
 

@@ -179,7 +179,7 @@ struct Handle {
   double scale_w = -1;                   // frequency the scaling was computed at
   bool scale_sym = false;                // the scaled system is symmetric (the symmetric scaling was kept)
   double scale_asym = 0;                 // largest difference of its mirrored entries
-  bool sym_off = false;                  // the symmetric path is not for these values (sym_possible)
+  int sym_off = 0;                       // uses for which the symmetric path is not for these values (sym_possible)
   // solver options (ss_set_option); kept until changed
   struct Options {
     int krylov_m = 30;                   // FGMRES restart length of the mixed sweep
